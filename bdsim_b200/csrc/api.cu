@@ -13,6 +13,7 @@
 
 #include "bdcu_internal.h"
 #include "integrator.cuh"
+#include "pair_layout.h"
 #include "plan.h"
 #include "team_layout.h"
 
@@ -23,6 +24,8 @@ cudaError_t occupancy_plain(int block, size_t smem, int* per_sm);
 cudaError_t occupancy_mixed(int block, size_t smem, int* per_sm);
 cudaError_t launch_mixed_team(int team_warps, int team_q, const RunArgs& a, int grid, size_t smem, cudaStream_t s);
 cudaError_t occupancy_mixed_team(int team_warps, int team_q, size_t smem, int* per_sm);
+cudaError_t launch_pair(int warps, const RunArgs& a, int grid, size_t smem, cudaStream_t s);
+cudaError_t occupancy_pair(int warps, size_t smem, int* per_sm);
 cudaError_t launch_forces(const DevChain* chains, int n_chains, int n_max, const double* arena, const double* R,
                           double t, int which, double* F, cudaStream_t s);
 cudaError_t launch_ran1(int n_chains, int32_t* rng, int n_per, double* out, cudaStream_t s);
@@ -318,8 +321,24 @@ Shape default_shape(const Bucket& b, int mixed, const std::vector<Shape>& shapes
     return first;
 }
 
-// Fill the launch fields of a bucket for a shape (block kernel) or for the
-// team kernel; 0 when the shape cannot run.
+// Warps per chain of the pair kernel that hold a chain of `beads`, the
+// bucket's default first.
+std::vector<Shape> pair_shapes(int id, int beads) {
+    std::vector<Shape> out;
+    auto add = [&](int T) {
+        if (32 * T < beads) return;
+        Shape s;
+        s.block = 32 * T;
+        out.push_back(s);
+    };
+    add(kDefaultPairWarps[id]);
+    for (int T : kPairWarps)
+        if (T != kDefaultPairWarps[id] && 32 * T <= 4 * kBucketBeads[id]) add(T);
+    return out;
+}
+
+// Fill the launch fields of a bucket for a shape (block or pair kernel) or for
+// the team kernel; 0 when the shape cannot run.
 int fill_launch(bdcu_ctx* ctx, int form, Bucket& b, const Shape* s) {
     const int mixed = form == BDCU_FORM_MIXED_FP32;
     int per_sm = 0;
@@ -342,6 +361,20 @@ int fill_launch(bdcu_ctx* ctx, int form, Bucket& b, const Shape* s) {
         b.v_cap = 0;
         b.d_in_smem = 0;
         b.scratch_stride = b.need_d ? team_scratch_doubles(b.n_max) : 1;
+        return BDCU_OK;
+    }
+    if (b.kernel == kKernelPair) {
+        const int T = s->block / 32;
+        b.block = s->block;
+        b.v_cap = b.d_in_smem = 0;
+        b.w_pairs = b.need_d ? pair_cached(b.n_max, T, ctx->max_smem) : 0;
+        b.smem = (size_t)pair_layout(b.n_max, T, b.w_pairs).total * sizeof(double);
+        if (b.smem > ctx->max_smem) return fail(ctx, BDCU_E_LIMIT, "chain too large for the shared-memory layout");
+        e = occupancy_pair(T, b.smem, &per_sm);
+        if (e != cudaSuccess) return cuda_fail(ctx, e, "occupancy_pair");
+        if (per_sm < 1) return fail(ctx, BDCU_E_LIMIT, "pair kernel shape cannot be resident");
+        b.grid = std::max(1, std::min(b.count, per_sm * ctx->sm_count));
+        b.scratch_stride = b.need_d ? pair_scratch_doubles(b.n_max) : 1;
         return BDCU_OK;
     }
     b.block = s->block;
@@ -392,7 +425,7 @@ int build_plan(bdcu_ctx* ctx, int form) {
     } else {
         for (int32_t c : ctx->sel) lists[bucket_of(ctx->chains_h[c], form)].push_back(c);
     }
-    if (ctx->single_launch) {
+    if (ctx->single_launch && mixed) {
         // one persistent launch for every team-kernel chain: the widest team
         // bucket present takes the others' chains (and runs its shape)
         int top = -1;
@@ -415,9 +448,9 @@ int build_plan(bdcu_ctx* ctx, int form) {
                          [&](int32_t x, int32_t y) { return ctx->chains_h[x].N > ctx->chains_h[y].N; });
         Bucket b;
         b.id = id;
-        b.kernel = id < kFirstBlockBucket ? BDCU_KERNEL_TEAM : BDCU_KERNEL_BLOCK;
-        b.team_warps = id < kFirstBlockBucket ? kDefaultTeamShape[id][0] : 0;
-        b.team_q = id < kFirstBlockBucket ? kDefaultTeamShape[id][1] : 0;
+        b.kernel = id >= kFirstBlockBucket ? BDCU_KERNEL_BLOCK : mixed ? BDCU_KERNEL_TEAM : kKernelPair;
+        b.team_warps = b.kernel == BDCU_KERNEL_TEAM ? kDefaultTeamShape[id][0] : 0;
+        b.team_q = b.kernel == BDCU_KERNEL_TEAM ? kDefaultTeamShape[id][1] : 0;
         b.count = (int)L.size();
         b.max_beads = ctx->chains_h[L.front()].N;
         b.min_beads = ctx->chains_h[L.back()].N;
@@ -436,6 +469,12 @@ int build_plan(bdcu_ctx* ctx, int form) {
             const Shape& t = ctx->tuned[mixed][id];
             const bool use = t.team_warps > 0 && team_shape_fits(t.team_warps, t.team_q, b.max_beads);
             if ((rc = fill_launch(ctx, form, b, use ? &t : nullptr))) return rc;
+            b.tuned = use ? 1 : 0;
+        } else if (b.kernel == kKernelPair) {
+            const Shape& t = ctx->tuned[mixed][id];
+            const bool use = t.block > 0 && t.block >= b.max_beads;
+            const Shape pick = use ? t : pair_shapes(id, b.max_beads).front();
+            if ((rc = fill_launch(ctx, form, b, &pick))) return rc;
             b.tuned = use ? 1 : 0;
         } else {
             const std::vector<Shape> shapes = block_shapes(ctx, b, form);
@@ -527,9 +566,12 @@ int launch_bucket(bdcu_ctx* ctx, int form, const Bucket& b, const State& st, int
     a.steps_done = st.steps_done;
     a.t_end = st.t_end;
     a.bounds_every = form == BDCU_FORM_MIXED_FP32 ? ctx->bounds_every : 1;
+    a.w_pairs = b.w_pairs;
     cudaError_t e;
     if (b.kernel == BDCU_KERNEL_TEAM)
         e = launch_mixed_team(b.team_warps, b.team_q, a, b.grid, b.smem, s);
+    else if (b.kernel == kKernelPair)
+        e = launch_pair(b.block / 32, a, b.grid, b.smem, s);
     else
         e = (form == BDCU_FORM_MIXED_FP32) ? launch_mixed(a, b.grid, b.block, b.smem, s)
                                            : launch_plain(a, b.grid, b.block, b.smem, s);
@@ -749,8 +791,8 @@ int bdcu_describe_plan(bdcu_ctx* ctx, int form, bdcu_bucket_info* out, int cap, 
     for (int i = 0; i < cap && i < (int)ctx->plan.size(); ++i) {
         const Bucket& b = ctx->plan[i];
         bdcu_bucket_info& o = out[i];
-        o.bucket = b.id;
-        o.kernel = b.kernel;
+        o.bucket = b.kernel == kKernelPair ? b.id + kFirstBlockBucket : b.id;
+        o.kernel = b.kernel == kKernelPair ? (int)BDCU_KERNEL_BLOCK : b.kernel;
         o.team_warps = b.team_warps;
         o.team_beads_per_thread = b.team_q;
         o.n_chains = b.count;
@@ -825,6 +867,8 @@ int bdcu_autotune(bdcu_ctx* ctx, int form, const double* R, const int32_t* rng, 
         std::vector<Shape> shapes;
         if (base.kernel == BDCU_KERNEL_BLOCK) {
             shapes = block_shapes(ctx, base, form);
+        } else if (base.kernel == kKernelPair) {
+            shapes = pair_shapes(base.id, base.max_beads);
         } else {
             // team shapes that hold any chain of the bucket, up to twice its width
             for (int i = 0; i < kNumTeamShapes; ++i) {

@@ -86,6 +86,7 @@ struct RunArgs {
     // steps (1: every step, the reference) and whenever a step's Chebyshev
     // check fails on the kept ones
     int32_t bounds_every;
+    int64_t w_pairs;        // pair kernel: cached pair weights (two doubles each) in shared memory
 };
 
 // Nanoseconds of the GPU's global timer.

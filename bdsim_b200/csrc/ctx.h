@@ -15,12 +15,14 @@ using bdcu::DevChain;
 
 namespace bdcu {
 
-// Buckets of a launch plan. Buckets 0..3 run the team kernel (FP32-mixed
-// form, no Cholesky method) with 1, 2, 4 and 8 warps per chain for N <= 64,
-// 128, 256 and 512; buckets 4..7 run one chain per block and split the rest by
-// bead count at 64, 128 and 256.
+// Buckets of a launch plan. Buckets 0..3 hold the chains of N <= 64, 128, 256
+// and 512 beads that do not use the Cholesky method: the team kernel in the
+// FP32-mixed form, the pair kernel (one chain per block, reported as block
+// buckets 4..7) in the plain form. Buckets 4..7 run one chain per block on the
+// general block kernel and split the rest by bead count at 64, 128 and 256.
 constexpr int kMaxBuckets = 8;
 constexpr int kFirstBlockBucket = 4;
+constexpr int kKernelPair = 2;  // Bucket::kernel of the pair kernel (BDCU_KERNEL_BLOCK outside)
 constexpr int kBucketBeads[kMaxBuckets] = {64, 128, 256, 512, 64, 128, 256, kMaxBeads};
 
 // A launch shape chosen by bdcu_autotune. Block kernel: threads per block,
@@ -44,6 +46,7 @@ struct Bucket {
     int need_chol = 0, need_d = 0, need_lz = 0;
     int64_t order_off = 0;  // first entry of this bucket's work list in order_d
     int block = 0, grid = 0, v_cap = 0, d_in_smem = 0, tuned = 0;
+    int64_t w_pairs = 0;  // pair kernel: cached pair weights
     size_t smem = 0;
     int64_t scratch_stride = 1;  // doubles per block (per warp)
 };

@@ -295,6 +295,32 @@ __device__ inline double ev_factor(const DevChain& c, double r, double phi_pair)
     }
 }
 
+// Distance beyond which the LJ and SDK factors are zero (0: everywhere).
+__device__ __forceinline__ double ev_outer_cutoff(const DevChain& c) {
+    switch (c.ev_type) {
+        case BDCU_EV_LJ: return dmax_(c.equil ? c.Rcutg : c.Rcutp, c.Rmin);
+        case BDCU_EV_SDK: return dmax_(dmax_(c.Rcutg, c.Rmin), c.equil ? 0.0 : c.RcutpSDK);
+        default: return 0.0;
+    }
+}
+
+// lj_factor / sdk_factor as ev_factor, at squared distance sq, with the 14th
+// and 8th powers of r as products of 1/r^2. phi: the pair's attractive
+// strength (null: zero).
+__device__ inline double ev_factor_short(const DevChain& c, double sq, const double* phi) {
+    const double r = sqrt(sq);
+    const bool sdk = c.ev_type == BDCU_EV_SDK;
+    if (r < c.Rmin) return sdk ? c.sdk_rmin_fac : c.lj_rmin_fac;
+    double fac = 0.0;
+    if (r <= (sdk || c.equil ? c.Rcutg : c.Rcutp)) {
+        const double i2 = 1.0 / sq, i4 = i2 * i2, i8 = i4 * i4;
+        fac = (sdk ? c.SDKa : c.LJa) * ((i8 * i4) * i2) - (sdk ? c.SDKb : c.LJb) * i8;
+    } else if (sdk && !c.equil && r <= c.RcutpSDK && phi) {
+        fac = 1.530633312 * *phi * sin(1.530633312 * sq + 1.213115524);
+    }
+    return fac;
+}
+
 // Flow::kappa (src/flow.cpp:5-26)
 __device__ inline void kappa_at(const DevChain& c, const double* arena, double t, double K[9]) {
     const int n = c.flow_n;

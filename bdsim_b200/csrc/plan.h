@@ -6,14 +6,18 @@
 #include <algorithm>
 
 #include "ctx.h"
+#include "pair_layout.h"
 #include "team_layout.h"
 
 namespace bdcu {
 
-// Bucket of a chain for `form` (bucket ids as in ctx.h).
-inline int bucket_of(const DevChain& c, int form) {
+// Bucket of a chain for `form` (bucket ids as in ctx.h). pair: whether the
+// plain form's pair kernel may be used (the static-scratch entry point keeps
+// the block kernel, whose scratch its limit is stated for).
+inline int bucket_of(const DevChain& c, int form, bool pair = true) {
     const bool chol = c.hstar > 0.0 && c.hi_method == BDCU_HI_CHOLESKY;
-    if (form == BDCU_FORM_MIXED_FP32 && !chol && c.N <= kTeamMaxN) {
+    static_assert(kPairMaxN == kTeamMaxN, "team and pair buckets share their bead ranges");
+    if ((form == BDCU_FORM_MIXED_FP32 || pair) && !chol && c.N <= kTeamMaxN) {
         const int T = team_warps_for(c.N);
         return T == 1 ? 0 : T == 2 ? 1 : T == 4 ? 2 : 3;
     }

@@ -141,7 +141,7 @@ extern "C" int bdcu_run_static(bdcu_ctx* ctx, int n_chains, const bdcu_phys* phy
     // buckets, as bdcu_run plans them (largest chains first within a bucket)
     const int mixed = (form == BDCU_FORM_MIXED_FP32);
     std::vector<std::vector<int32_t>> lists(kMaxBuckets);
-    for (int i = 0; i < n_chains; ++i) lists[bucket_of(recs[i], form)].push_back(i);
+    for (int i = 0; i < n_chains; ++i) lists[bucket_of(recs[i], form, false)].push_back(i);
     struct Launch {
         int id, team_warps, team_q, block, grid, v_cap, d_in_smem, n_max, need_d, need_lz, count;
         size_t smem, per_block;
