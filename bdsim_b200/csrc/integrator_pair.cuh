@@ -610,69 +610,6 @@ struct PairChain {
         return warm;
     }
 
-    // A warm Lanczos run (up to 8 steps) from the unit vector v with w = D v,
-    // its basis in shared memory. One reduction per step: the new vector u goes
-    // into the product unnormalised, and u.u, u.Du and the projections of Du on
-    // the basis are summed together, so that its norm (explicit, not by
-    // Pythagoras, whose cancellation would grow from step to step), alpha and
-    // the next vector follow at once. One projection pass per step keeps the
-    // basis orthogonal to about 1e-12 in 8 steps (1e-11 in 30, where the extreme
-    // eigenvalues still agree with the reference's scheme to 5e-15). Returns its
-    // steps; the tridiagonal is left in alpha and beta.
-    __device__ __forceinline__ int lanczos_warm(double (&v)[3], double (&w)[3]) {
-        const int m = n < kLanczosWarm ? n : kLanczosWarm;
-        double* V = area;
-        double u[3] = {v[0], v[1], v[2]};
-        int j = 0;
-#pragma unroll 1
-        for (;; ++j) {
-            if (j > 0) apply1(u, w);
-            double* r = next_red();
-            double c[8];  // (loads without a branch, so that they are all in flight together)
-            c[0] = fma(u[2], u[2], fma(u[1], u[1], u[0] * u[0]));
-            c[1] = fma(u[2], w[2], fma(u[1], w[1], u[0] * w[0]));
-#pragma unroll
-            for (int i = 0; i < kLanczosWarm - 2; ++i) {
-                const double* vi = V + max(min(i, j - 1), 0) * ldv + 3 * bc;
-                const double x = fma(w[2], vi[2], fma(w[1], vi[1], w[0] * vi[0]));
-                c[2 + i] = i < j && on ? x : 0.0;
-            }
-            warp_sum8(c, r);
-            __syncthreads();
-            const double t = total8(r), bsq = __shfl_sync(kFull, t, 0);
-            if (j > 0 && bsq < 1.0e-20) {
-                cnt[C_DX] -= 1;  // (the reference stops before this product)
-                break;
-            }
-            const double ib = rsqrt_refined(bsq), al = (__shfl_sync(kFull, t, 1) * ib) * ib;
-            if (tid == 0) {
-                alpha[j] = al;
-                if (j > 0) beta[j - 1] = bsq * ib;
-            }
-#pragma unroll
-            for (int d = 0; d < 3; ++d) v[d] = u[d] * ib;
-            if (own)
-#pragma unroll
-                for (int d = 0; d < 3; ++d) V[j * ldv + 3 * b + d] = v[d];
-            __syncwarp();  // (the lanes of a bead read it back)
-            if (j == m - 1) {
-                ++j;
-                break;
-            }
-#pragma unroll
-            for (int d = 0; d < 3; ++d) u[d] = fma(w[d], ib, -(al * v[d]));
-#pragma unroll
-            for (int i = 0; i < kLanczosWarm - 2; ++i)
-            {
-                const double g = __shfl_sync(kFull, t, 2 + i) * ib, c = i < j ? g : 0.0;
-                const double* vi = V + min(i, j) * ldv + 3 * bc;
-#pragma unroll
-                for (int d = 0; d < 3; ++d) u[d] = on ? fma(-c, vi[d], u[d]) : 0.0;
-            }
-        }
-        return j;
-    }
-
     // u -= sum_i (V_i.u) V_i over the first nv vectors of the cold basis, all
     // projections reduced together (one barrier).
     __device__ __forceinline__ void project(int nv, double (&u)[3]) {
@@ -702,18 +639,26 @@ struct PairChain {
         }
     }
 
-    // A cold run (30 steps, the first step of a call), its basis in global
-    // scratch: the three-term recurrence, followed by projections on the whole
-    // basis in two steps of every six (from 3N = 64; in every step below, where
-    // the Krylov space is soon exhausted). Two consecutive steps
-    // restore orthogonality, and between them it stays far below the square
-    // root of rounding that the tridiagonal's accuracy needs: over the chain
-    // lengths and potentials of the tests the extreme eigenvalues agree with the
-    // reference's scheme to 2e-14 and the basis is orthogonal to 1e-11.
-    // Projecting every step read the basis from L2 twice a step: 12.9 thousand
-    // cycles a step at N = 50, 2.7 of them the product.
-    __device__ __forceinline__ int lanczos_cold(double (&v)[3], double (&w)[3], bool have_w) {
-        const int m = n < kLanczosCold ? n : kLanczosCold;
+    // A Lanczos run from the unit vector v (with w = D v if have_w): 8 steps
+    // with the basis in shared memory (warm), or 30 with it in global scratch
+    // (cold, the first step of a call). One reduction per step: the new vector u
+    // goes into the product unnormalised, and u.u and u.Du are summed together,
+    // so that its norm (explicit: |Du|^2 - alpha^2 - beta^2 loses digits from
+    // step to step), alpha and the next vector follow at once.
+    // Orthogonality: the reference projects every vector on the whole basis. In 8
+    // steps the three-term recurrence alone gives the same extreme eigenvalues
+    // (to 5e-14) and start vector (to 5e-14). A cold run projects in two steps
+    // of every six (from 3N = 64; in every step below, where the Krylov space is
+    // soon exhausted): two consecutive steps restore orthogonality, and between
+    // them it stays far below the square root of rounding that the
+    // tridiagonal's accuracy needs. Over the chain lengths and potentials of the
+    // tests the eigenvalues agree with the reference's scheme to 2e-14, the
+    // basis is orthogonal to 1e-11. (Projecting in every step read the basis from
+    // L2 twice a step: 12.9 thousand cycles a step at N = 50, 2.7 of them the
+    // product; now 8.0.) Returns its steps; the tridiagonal is left in alpha and
+    // beta.
+    __device__ __forceinline__ int lanczos(double* V, bool cold, double (&v)[3], double (&w)[3], bool have_w) {
+        const int m = min(n, cold ? kLanczosCold : kLanczosWarm);
         const bool every = n < 64;
         double u[3] = {v[0], v[1], v[2]}, vp[3] = {0.0, 0.0, 0.0}, bprev = 1.0;
         bool due = false;
@@ -723,7 +668,7 @@ struct PairChain {
             double g2[2] = {fma(u[2], u[2], fma(u[1], u[1], u[0] * u[0])), fma(u[2], w[2], fma(u[1], w[1], u[0] * w[0]))};
             sums(g2);
             const double bsq = g2[0];
-            if (j > 0 && !(bsq >= 1.0e-20)) {
+            if (j > 0 && bsq < 1.0e-20) {
                 cnt[C_DX] -= 1;  // (the reference stops before this product)
                 return j;
             }
@@ -732,24 +677,25 @@ struct PairChain {
                 alpha[j] = al;
                 if (j > 0) beta[j - 1] = bt;
             }
-            // a beta far below its neighbours magnifies what orthogonality was lost
-            due = due ? bt < 0.1 * bprev : bt < 0.03 * fabs(al) || bt < 0.1 * bprev;
-            bprev = bt;
 #pragma unroll
             for (int d = 0; d < 3; ++d) v[d] = u[d] * ib;
             if (own)
 #pragma unroll
-                for (int d = 0; d < 3; ++d) Vg[j * ldv + 3 * b + d] = v[d];
-            __syncwarp();  // (the lanes of a bead read it back)
+                for (int d = 0; d < 3; ++d) V[j * ldv + 3 * b + d] = v[d];
             if (j == m - 1) return m;  // (the last beta is no entry of the tridiagonal)
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
                 u[d] = fma(w[d], ib, -(al * v[d]));
                 if (j > 0) u[d] = fma(-bt, vp[d], u[d]);
+                vp[d] = v[d];
             }
-            if (every || due || j % 6 >= 4) project(j + 1, u);
-#pragma unroll
-            for (int d = 0; d < 3; ++d) vp[d] = v[d];
+            if (cold) {
+                // a beta far below its neighbours magnifies what orthogonality was lost
+                due = due ? bt < 0.1 * bprev : bt < 0.03 * fabs(al) || bt < 0.1 * bprev;
+                bprev = bt;
+                __syncwarp();  // (the lanes of a bead read its basis entries back)
+                if (every || due || j % 6 >= 4) project(j + 1, u);
+            }
         }
     }
 
@@ -781,7 +727,7 @@ struct PairChain {
                 }
                 warp_multisect([&](double x) { return sturm_count8(ar, b2, k, x); }, wi == 0 ? 1 : k, lo, hi2);
                 r = 0.5 * (lo + hi2);
-                tridiag_vec_reg(ar, br, k, r, 1.0e-12, yr);
+                tridiag_vec_reg<2>(ar, br, k, r, yr);
                 if (wl == 0)
 #pragma unroll
                     for (int i = 0; i < kLanczosWarm; ++i)
@@ -835,16 +781,15 @@ struct PairChain {
             }
         }
         // (the warm basis is in shared memory, the cold one in global scratch)
-        bool cold = !can_warm;
-        int k = 0;
-        if (can_warm) {
-            k = lanczos_warm(v, w);
-            if (k < 4) {
-                start_vector(nullptr, false, v);
-                cold = true;
-            }
+        bool cold = !can_warm, have_w = true;
+        int k;
+        for (;;) {
+            k = lanczos(cold ? Vg : area, cold, v, w, have_w);
+            if (cold || k >= 4) break;
+            start_vector(nullptr, false, v);
+            cold = true;
+            have_w = false;
         }
-        if (cold) k = lanczos_cold(v, w, !can_warm);
         ritz_pair(cold ? Vg : area, k, ritz, rmin, rmax);
         cnt[cold ? C_LZCOLD : C_LZWARM] += 1;
         double s[3];

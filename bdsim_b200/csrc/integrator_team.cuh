@@ -158,20 +158,23 @@ __device__ __forceinline__ double rcp_newton(double x) {
 
 // Inverse iteration for a Ritz vector (src/hydrodynamics.cpp:106-136) with the
 // tridiagonal (k <= kLanczosWarm) in registers; every lane that calls it
-// computes the same y. One solve at a shift a relative `offset` below the
-// eigenvalue: it amplifies its eigenvector by 1 / offset over the others. (The
-// reference's two solves at 1e-7 leave 1e-14 of them: the plain form's one at
-// 1e-12 is as good; the mixed form, whose eigenvalue is good to 1e-6, keeps
-// 1e-7. The vector only seeds the next step's Lanczos.)
+// computes the same y. kPasses: the reference's two in the plain form (a
+// single solve closer to the eigenvalue leaves 1e-10 of the other vectors, two
+// at 1e-7 leave 1e-15); one in the mixed form, whose shift is within 1e-6
+// relative of the eigenvalue, so a single solve already amplifies its
+// eigenvector by ~1e5 over the others (the vector only seeds the next step's
+// Lanczos).
+template <int kPasses>
 __device__ __forceinline__ void tridiag_vec_reg(const double (&a)[kLanczosWarm], const double (&b)[kLanczosWarm],
-                                                int m, double lambda, double offset, double (&y)[kLanczosWarm]) {
+                                                int m, double lambda, double (&y)[kLanczosWarm]) {
     const double scale = dmax_(fabs(lambda), 1.0);
-    const double shift = lambda - offset * scale;
+    const double shift = lambda - 1.0e-7 * scale;
     const double y0 = rsqrt((double)m);
     double c[kLanczosWarm];
 #pragma unroll
     for (int i = 0; i < kLanczosWarm; ++i) y[i] = i < m ? y0 : 0.0;
-    {
+#pragma unroll 1
+    for (int it = 0; it < kPasses; ++it) {
         // pivots: the reference's tiny-pivot guard (1e-300) raised to 1e-30 so
         // that the reciprocal's single-precision seed stays in range (the
         // vector only seeds the next step's Lanczos)
@@ -888,7 +891,7 @@ struct TeamChain {
             halfwarp_multisect(ar, br, k, wl < 16 ? 1 : k, lo, hi2);
             const double r = 0.5 * (lo + hi2);
             double y[kLanczosWarm];
-            tridiag_vec_reg(ar, br, k, r, 1.0e-7, y);
+            tridiag_vec_reg<1>(ar, br, k, r, y);
             if ((wl & 15) == 0) {
                 double* dst = wl == 0 ? S.ymin : S.ymax;
 #pragma unroll
