@@ -350,7 +350,8 @@ int fill_launch(bdcu_ctx* ctx, int form, Bucket& b, const Shape* s) {
         }
         const int T = b.team_warps, Q = b.team_q;
         if (!team_shape_fits(T, Q, b.max_beads)) return fail(ctx, BDCU_E_ARG, "team shape does not hold the bucket");
-        b.smem = (size_t)team_smem(T, Q, b.n_max);
+        b.w_pairs = b.need_d ? team_weights(T, Q, b.n_max, ctx->max_smem) : 0;
+        b.smem = (size_t)team_smem(T, Q, b.n_max, b.w_pairs);
         if (b.smem > ctx->max_smem) return fail(ctx, BDCU_E_LIMIT, "team kernel shared memory exceeds the device limit");
         e = occupancy_mixed_team(T, Q, b.smem, &per_sm);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "occupancy_mixed_team");

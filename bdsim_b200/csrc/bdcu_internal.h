@@ -86,7 +86,8 @@ struct RunArgs {
     // steps (1: every step, the reference) and whenever a step's Chebyshev
     // check fails on the kept ones
     int32_t bounds_every;
-    int64_t w_pairs;        // pair kernel: cached pair weights (two doubles each) in shared memory
+    int64_t w_pairs;        // cached pair weights in shared memory, 16 bytes each: per block of the pair
+                            // kernel, per team of the team kernel
 };
 
 // Nanoseconds of the GPU's global timer.

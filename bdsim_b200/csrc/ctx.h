@@ -46,7 +46,7 @@ struct Bucket {
     int need_chol = 0, need_d = 0, need_lz = 0;
     int64_t order_off = 0;  // first entry of this bucket's work list in order_d
     int block = 0, grid = 0, v_cap = 0, d_in_smem = 0, tuned = 0;
-    int64_t w_pairs = 0;  // pair kernel: cached pair weights
+    int64_t w_pairs = 0;  // pair and team kernels: cached pair weights (per block, per team)
     size_t smem = 0;
     int64_t scratch_stride = 1;  // doubles per block (per warp)
 };

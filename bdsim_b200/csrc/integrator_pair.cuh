@@ -23,15 +23,6 @@
 
 namespace bdcu {
 
-// 1/sqrt(s) for s in [1e-12, 3e38]: the single-precision estimate y (relative
-// error below 2^-21) refined by one third-order step of the Newton-Halley
-// family, y (1 + e/2 + 3 e^2/8) with e = 1 - s y^2, whose error is O(e^3).
-__device__ __forceinline__ double rsqrt_refined(double s) {
-    const double y = (double)rsqrtf((float)s);
-    const double e = fma(-(s * y), y, 1.0);
-    return fma(y * e, fma(e, 0.375, 0.5), y);
-}
-
 // RPY weights of a pair at squared separation sq (src/hydrodynamics.cpp:36-43)
 // with h* folded into the constants. (The two branches meet continuously at
 // r = 2 sqrt(pi) h*.)
@@ -513,17 +504,6 @@ struct PairChain {
     // the generator's state at the start of its block: jumped there once per
     // chain, and from step to step by the same 3N draws for every thread (the
     // xorshift matrix power's columns in shared memory; 16807^3N mod 2^31 - 1).
-    __device__ __forceinline__ static uint32_t lehmer(uint32_t m, uint32_t x) {  // m x mod 2^31 - 1
-        const uint64_t p = (uint64_t)m * x;
-        uint32_t r = (uint32_t)(p & 0x7fffffffu) + (uint32_t)(p >> 31);
-        return r >= 0x7fffffffu ? r - 0x7fffffffu : r;
-    }
-    __device__ __forceinline__ static uint32_t jump(const uint32_t* cols, uint32_t x) {
-        uint32_t y = 0;
-#pragma unroll 8
-        for (int i = 0; i < 32; ++i) y ^= cols[i] & (0u - ((x >> i) & 1u));
-        return y;
-    }
     // State (ux, iy) of the chain's stream -> this thread's block start.
     __device__ __forceinline__ void noise_start(uint32_t& ux, int32_t& iy, int32_t& sd) {
         if (sd <= 0 || iy < 0) {
@@ -533,8 +513,8 @@ struct PairChain {
             sd = s + 1;
         }
         const int k0 = min(tid * ((n + TT - 1) / TT), n);
-        ux = jump(a.xs_pow + 32 * (int64_t)k0, ux);
-        iy = (int32_t)lehmer(a.a_pow[k0], (uint32_t)iy);
+        ux = xorshift_jump(a.xs_pow + 32 * (int64_t)k0, ux);
+        iy = (int32_t)lehmer_mul(a.a_pow[k0], (uint32_t)iy);
         if (tid < 32) jcols[tid] = a.xs_pow[32 * (int64_t)n + tid];
         __syncthreads();
     }
@@ -547,12 +527,12 @@ struct PairChain {
             ux ^= (ux << 13);
             ux ^= (ux >> 17);
             ux ^= (ux << 5);
-            iy = lehmer(16807u, iy);
+            iy = lehmer_mul(16807u, iy);
             const int32_t res = (int32_t)(((ux ^ iy) & 0x7fffffffu) | 1u);
             y[k] = (double)__fmul_rn(am, __int2float_rn(res));
         }
-        ux0 = jump(jcols, ux0);
-        iy0 = (int32_t)lehmer(a.a_pow[n], (uint32_t)iy0);
+        ux0 = xorshift_jump(jcols, ux0);
+        iy0 = (int32_t)lehmer_mul(a.a_pow[n], (uint32_t)iy0);
         __syncthreads();
 #pragma unroll
         for (int d = 0; d < 3; ++d) {

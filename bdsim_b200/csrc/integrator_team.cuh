@@ -146,6 +146,29 @@ static __device__ void halfwarp_multisect(const double (&a)[kLanczosWarm], const
     }
 }
 
+// m x mod 2^31 - 1, by folding the product's high part onto the low one.
+__device__ __forceinline__ uint32_t lehmer_mul(uint32_t m, uint32_t x) {
+    const uint64_t p = (uint64_t)m * x;
+    const uint32_t r = (uint32_t)(p & 0x7fffffffu) + (uint32_t)(p >> 31);
+    return r >= 0x7fffffffu ? r - 0x7fffffffu : r;
+}
+// The xorshift state x advanced by the matrix power whose columns are given.
+__device__ __forceinline__ uint32_t xorshift_jump(const uint32_t* cols, uint32_t x) {
+    uint32_t y = 0;
+#pragma unroll 8
+    for (int i = 0; i < 32; ++i) y ^= cols[i] & (0u - ((x >> i) & 1u));
+    return y;
+}
+
+// 1/sqrt(s) for s in [1e-12, 3e38]: the single-precision estimate y (relative
+// error below 2^-21) refined by one third-order step of the Newton-Halley
+// family, y (1 + e/2 + 3 e^2/8) with e = 1 - s y^2, whose error is O(e^3).
+__device__ __forceinline__ double rsqrt_refined(double s) {
+    const double y = (double)rsqrtf((float)s);
+    const double e = fma(-(s * y), y, 1.0);
+    return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+
 // 1/x for |x| in [1e-30, 1e30]: a single-precision seed refined by two
 // Newton-Raphson steps r <- r (2 - x r) (quadratic convergence: 2^-23 ->
 // 2^-46 -> below double rounding).
@@ -255,6 +278,7 @@ struct TeamChain {
     double* V;      // warm Lanczos basis in shared memory (kLanczosWarm x nv)
     float* sqx;     // Chebyshev node values, aliasing V (dead after the bounds)
     float* coef;    // Chebyshev coefficients, aliasing V
+    float* ct;      // cosine table, aliasing V
     double* Vg;     // cold basis in global scratch (kLanczosCold x nv)
     double* Lt;     // Cholesky factor in global scratch (n x n)
     int nv;
@@ -263,6 +287,9 @@ struct TeamChain {
     int team;       // team in the thread block (named barrier 1 + team)
     int N, n;
     bool hi;
+    float4* Wt;     // cached pair weights (omega1 of j, j+1, omega2 of j, j+1): row j/2, column bead
+    int jc;         // partner beads below jc have cached weights (even)
+    int par, xpar;  // parity of the reduction buffer and of the single products' input rows
     int32_t cnt[8];  // this call's counts for the chain (added to the 64-bit counters at the end)
     int status;
     // RPY constants (FP32). Bead coordinates are staged divided by `scale`
@@ -276,70 +303,65 @@ struct TeamChain {
     __device__ __forceinline__ int bead(int q) const { return tid + TT * q; }
     __device__ __forceinline__ void sync() const { team_sync<T>(team); }
 
-    // Sum over the team, the same bits in every thread: warp butterflies, then
-    // the warps' partial sums added in warp order.
-    __device__ double tsum(double v) const {
-        v = wsum(v);
-        if constexpr (T == 1) {
-            return v;
-        } else {
-            sync();
-            if (wl == 0) S.red[wi] = v;
-            sync();
-            double s = S.red[0];
-#pragma unroll
-            for (int w = 1; w < T; ++w) s += S.red[w];
-            return s;
-        }
+    // Sums over the team, the same bits in every thread: warp butterflies, then
+    // the warps' partial sums added in warp order. One barrier: consecutive
+    // calls alternate between two buffers.
+    __device__ __forceinline__ double* next_red() {
+        double* r = S.red[par];
+        par ^= 1;
+        return r;
     }
-
-    // Eight team sums at once (the batched projections of the warm Lanczos),
-    // the same bits in every thread. In each warp a transposed reduction:
-    // exchange halves of the vector with lane^16, ^8, ^4 (each lane keeps the
-    // half its lane bit selects), then a butterfly over lane^2, ^1, leaves sum
-    // u = 4*b4 + 2*b3 + b2 in the lanes whose bits 4, 3, 2 are b4, b3, b2;
-    // lanes 0, 4, ..., 28 publish the warp's eight sums in shared memory and
-    // the warps' partials are added in warp order.
-    __device__ void tsum8(double (&c)[kLanczosWarm]) const {
-        static_assert(kLanczosWarm == 8, "tsum8 reduces eight values");
-        const bool u16 = wl & 16, u8 = wl & 8, u4 = wl & 4;
-        double k4[4], k2[2];
+    template <int M>
+    __device__ __forceinline__ void sums(double (&v)[M]) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const double send = u16 ? c[u] : c[u + 4];
-            k4[u] = (u16 ? c[u + 4] : c[u]) + __shfl_xor_sync(kFull, send, 16);
-        }
+        for (int m = 0; m < M; ++m) v[m] = wsum(v[m]);
+        if constexpr (T > 1) {
+            double* r = next_red();
+            if (wl == 0)
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const double send = u8 ? k4[u] : k4[u + 2];
-            k2[u] = (u8 ? k4[u + 2] : k4[u]) + __shfl_xor_sync(kFull, send, 8);
-        }
-        double s = (u4 ? k2[1] : k2[0]) + __shfl_xor_sync(kFull, u4 ? k2[0] : k2[1], 4);
-        s += __shfl_xor_sync(kFull, s, 2);
-        s += __shfl_xor_sync(kFull, s, 1);
-        const int idx = (u16 ? 4 : 0) + (u8 ? 2 : 0) + (u4 ? 1 : 0);
-        if constexpr (T == 1) {
-            if ((wl & 3) == 0) S.red[idx] = s;
-            __syncwarp();
-#pragma unroll
-            for (int u = 0; u < kLanczosWarm; ++u) c[u] = S.red[u];
-            __syncwarp();
-        } else {
-            sync();
-            if ((wl & 3) == 0) S.red[kLanczosWarm * wi + idx] = s;
+                for (int m = 0; m < M; ++m) r[m * T + wi] = v[m];
             sync();
 #pragma unroll
-            for (int u = 0; u < kLanczosWarm; ++u) {
-                double v = S.red[u];
+            for (int m = 0; m < M; ++m) {
+                v[m] = r[m * T];
 #pragma unroll
-                for (int w = 1; w < T; ++w) v += S.red[kLanczosWarm * w + u];
-                c[u] = v;
+                for (int w = 1; w < T; ++w) v[m] += r[m * T + w];
             }
         }
     }
+    __device__ __forceinline__ double tsum(double v) {
+        double a1[1] = {v};
+        sums(a1);
+        return a1[0];
+    }
+
+    // Eight sums over the warp at once: halves of the vector exchanged with
+    // lanes ^16, ^8, ^4, then a butterfly over ^2, ^1; value u ends in lanes
+    // 4u..4u+3, which publish it for their warp at out[u * T + warp].
+    __device__ __forceinline__ void warp_sum8(const double (&c)[8], double* out) const {
+        const bool u16 = wl & 16, u8 = wl & 8, u4 = wl & 4;
+        double k4[4], k2[2];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            k4[u] = (u16 ? c[u + 4] : c[u]) + __shfl_xor_sync(kFull, u16 ? c[u] : c[u + 4], 16);
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+            k2[u] = (u8 ? k4[u + 2] : k4[u]) + __shfl_xor_sync(kFull, u8 ? k4[u] : k4[u + 2], 8);
+        double t = (u4 ? k2[1] : k2[0]) + __shfl_xor_sync(kFull, u4 ? k2[0] : k2[1], 4);
+        t += __shfl_xor_sync(kFull, t, 2);
+        t += __shfl_xor_sync(kFull, t, 1);
+        if ((wl & 3) == 0) out[(wl >> 2) * T + wi] = t;
+    }
+    // After a barrier: the total over the warps of published value u.
+    __device__ __forceinline__ double total(const double* r, int u) const {
+        double t = r[u * T];
+#pragma unroll
+        for (int w = 1; w < T; ++w) t += r[u * T + w];
+        return t;
+    }
 
     // OR of status bits over the team.
-    __device__ int tor(int v) const {
+    __device__ int tor(int v) {
         v = __reduce_or_sync(kFull, v);
         if constexpr (T == 1) {
             return v;
@@ -360,100 +382,172 @@ struct TeamChain {
     // pair geometry and weights are computed once for all K inputs (K = 3
     // for the products of a step that do not depend on one another).
     //
-    // The single products (K = 1, most of the step's passes) take the
-    // partner beads j two at a time in packed FP32x2 arithmetic (sm_100's
-    // FADD2 / FMUL2 / FFMA2: one issue slot for the pair; the FP32 pipe rate
-    // is that of scalar FFMA, measured 73 TFLOP/s on one B200 either way),
+    // The partner beads j are taken two at a time in packed FP32x2 arithmetic
+    // (sm_100's FADD2 / FMUL2 / FFMA2: one issue slot for the pair; the FP32 pipe
+    // rate is that of scalar FFMA, measured 73 TFLOP/s on one B200 either way),
     // from coordinates and inputs staged by component in shared memory, so
     // one 64-bit broadcast load brings (j, j+1) of a component. Each bead's
     // sum is kept as two interleaved partial sums (even and odd j), added at
     // the end. An odd N is padded with one zero input (whose contribution
     // om1 * 0 + om2 (d . 0) d is exactly zero).
+    // The pair weights of the first jc partner beads are computed once a step
+    // (build_weights) and kept in shared memory, 8 bytes per pair: a product
+    // then takes 13 packed operations per bead and two partners instead of about
+    // 35, and a chain of dependent operations half as long. The rest, where
+    // they do not fit (N above about 100), are evaluated in every product by the
+    // same operations, so a result does not depend on jc.
     template <int K>
-    __device__ void applyK(const float (&x)[K][Q][3], float (&acc)[K][Q][3]) {
+    __device__ __forceinline__ void applyK(const float (&x)[K][Q][3], float (&acc)[K][Q][3]) {
         static_assert(K >= 1 && K <= 3, "applyK stages at most three inputs");
         cnt[C_DX] += K;
+        // single products alternate between input rows 0 and 1, so that the
+        // barrier after staging also guards the rows' next use; the fused sets
+        // wait for the products before them
+        float(*xr)[3][32 * T * Q] = S.xk;
+        if (K == 1) {
+            xr += xpar;
+            xpar ^= 1;
+        } else {
+            sync();
+        }
 #pragma unroll
         for (int q = 0; q < Q; ++q)
             if (valid(q))
 #pragma unroll
                 for (int r = 0; r < K; ++r)
 #pragma unroll
-                    for (int d = 0; d < 3; ++d) S.xk[r][d][bead(q)] = x[r][q][d];
-        if ((N & 1) && tid < 3 * K) S.xk[tid / 3][tid % 3][N] = 0.f;
+                    for (int d = 0; d < 3; ++d) xr[r][d][bead(q)] = x[r][q][d];
+        if ((N & 1) && tid < 3 * K) xr[tid / 3][tid % 3][N] = 0.f;
         sync();
-        // In units of h*: with d = (R_j - R_b)/h*, s = |d|^2, rho = s^-1/2,
-        //   far  (s >= 4 pi): om1 = rho (K1 + K2 rho^2), om2 = rho^3 (K1 - K3 rho^2)
-        //   near (s <  4 pi): om1 = 1 - C3 s rho,         om2 = C7 rho
-        // and y_b += om1 x_j + om2 (d.x_j) d; both branches' weights are
-        // computed and each is selected once. The self
-        // pair (d = 0, s clamped to 1e-24) takes the near branch with om1 = 1
-        // exactly in FP32 and om2 d = 0: it contributes the identity block.
         bool one_slot = false;
         if constexpr (Q == 2) one_slot = __all_sync(kFull, !valid(1));
         const int nq = one_slot ? 1 : Q;
-        {
-            // every product (the Lanczos, Chebyshev, upsilon and corrector
-            // ones, and the fused sets of K = 2, 3): partner beads two at a
-            // time in packed FP32x2
-            float2 nb[Q][3], a[K][Q][3];
+        float2 nb[Q][3], a[K][Q][3];
+        own_coordinates(nb);
 #pragma unroll
-            for (int q = 0; q < Q; ++q)
+        for (int q = 0; q < Q; ++q)
 #pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    const float v = valid(q) ? -S.ps[d][bead(q)] : 0.f;
-                    nb[q][d] = make_float2(v, v);
-                    for (int r = 0; r < K; ++r) a[r][q][d] = make_float2(0.f, 0.f);
-                }
-            const float2 k1 = make_float2(K1, K1), k2 = make_float2(K2, K2), mk3 = make_float2(-K3, -K3);
-            const float2 mc3 = make_float2(-C3, -C3), c7 = make_float2(C7, C7), one = make_float2(1.f, 1.f);
-            const int n2 = (N + 1) & ~1;
-            // not unrolled: this loop is inlined at every product's call site
-#pragma unroll 1
-            for (int j = 0; j < n2; j += 2) {
-                float2 pj[3], xj[K][3];
+            for (int d = 0; d < 3; ++d)
 #pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    pj[d] = *reinterpret_cast<const float2*>(&S.ps[d][j]);
-                    for (int r = 0; r < K; ++r) xj[r][d] = *reinterpret_cast<const float2*>(&S.xk[r][d][j]);
-                }
+                for (int r = 0; r < K; ++r) a[r][q][d] = make_float2(0.f, 0.f);
+        auto products = [&](int q, const float2& dx, const float2& dy, const float2& dz, const float2& om1,
+                            const float2& om2, const float2 (&xj)[K][3]) {
 #pragma unroll
-                for (int q = 0; q < Q; ++q) {
-                    if (q < nq) {
-                        const float2 dx = __fadd2_rn(pj[0], nb[q][0]);
-                        const float2 dy = __fadd2_rn(pj[1], nb[q][1]);
-                        const float2 dz = __fadd2_rn(pj[2], nb[q][2]);
-                        float2 sq = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
-                        sq = make_float2(fmaxf(sq.x, 1e-24f), fmaxf(sq.y, 1e-24f));
-                        const float2 rho = make_float2(rsqrtf(sq.x), rsqrtf(sq.y));
-                        const float2 t = __fmul2_rn(rho, rho);
-                        const float2 u = __ffma2_rn(k2, t, k1), v = __ffma2_rn(mk3, t, k1);
-                        const float2 r = __fmul2_rn(sq, rho), rt = __fmul2_rn(rho, t);
-                        const bool fx = sq.x >= 12.566370614359172f, fy = sq.y >= 12.566370614359172f;
-                        // both branches' weights, then one select each (a far
-                        // weight of the clamped self pair may be infinite: it
-                        // is not selected)
-                        const float2 f1 = __fmul2_rn(rho, u), f2 = __fmul2_rn(rt, v);
-                        const float2 n1 = __ffma2_rn(mc3, r, one), n2 = __fmul2_rn(c7, rho);
-                        const float2 om1 = make_float2(fx ? f1.x : n1.x, fy ? f1.y : n1.y);
-                        const float2 om2 = make_float2(fx ? f2.x : n2.x, fy ? f2.y : n2.y);
-#pragma unroll
-                        for (int r = 0; r < K; ++r) {
-                            const float2 tt = __fmul2_rn(
-                                om2, __ffma2_rn(dz, xj[r][2], __ffma2_rn(dy, xj[r][1], __fmul2_rn(dx, xj[r][0]))));
-                            a[r][q][0] = __ffma2_rn(tt, dx, __ffma2_rn(om1, xj[r][0], a[r][q][0]));
-                            a[r][q][1] = __ffma2_rn(tt, dy, __ffma2_rn(om1, xj[r][1], a[r][q][1]));
-                            a[r][q][2] = __ffma2_rn(tt, dz, __ffma2_rn(om1, xj[r][2], a[r][q][2]));
-                        }
-                    }
-                }
+            for (int r = 0; r < K; ++r) {
+                const float2 tt =
+                    __fmul2_rn(om2, __ffma2_rn(dz, xj[r][2], __ffma2_rn(dy, xj[r][1], __fmul2_rn(dx, xj[r][0]))));
+                a[r][q][0] = __ffma2_rn(tt, dx, __ffma2_rn(om1, xj[r][0], a[r][q][0]));
+                a[r][q][1] = __ffma2_rn(tt, dy, __ffma2_rn(om1, xj[r][1], a[r][q][1]));
+                a[r][q][2] = __ffma2_rn(tt, dz, __ffma2_rn(om1, xj[r][2], a[r][q][2]));
             }
-            sync();
+        };
+        const int n2 = (N + 1) & ~1;
+        int j = 0;
+        const float4* w = Wt;
+#pragma unroll(K == 1 ? 2 : 1)
+        for (; j < jc; j += 2, w += N) {
+            float2 pj[3], xj[K][3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                pj[d] = *reinterpret_cast<const float2*>(&S.ps[d][j]);
+#pragma unroll
+                for (int r = 0; r < K; ++r) xj[r][d] = *reinterpret_cast<const float2*>(&xr[r][d][j]);
+            }
 #pragma unroll
             for (int q = 0; q < Q; ++q)
+                if (q < nq) {
+                    const float4 o = w[min(bead(q), N - 1)];
+                    products(q, __fadd2_rn(pj[0], nb[q][0]), __fadd2_rn(pj[1], nb[q][1]), __fadd2_rn(pj[2], nb[q][2]),
+                             make_float2(o.x, o.y), make_float2(o.z, o.w), xj);
+                }
+        }
+#pragma unroll 1
+        for (; j < n2; j += 2) {
+            float2 pj[3], xj[K][3];
 #pragma unroll
-                for (int d = 0; d < 3; ++d)
-                    for (int r = 0; r < K; ++r) acc[r][q][d] = valid(q) ? a[r][q][d].x + a[r][q][d].y : 0.f;
+            for (int d = 0; d < 3; ++d) {
+                pj[d] = *reinterpret_cast<const float2*>(&S.ps[d][j]);
+#pragma unroll
+                for (int r = 0; r < K; ++r) xj[r][d] = *reinterpret_cast<const float2*>(&xr[r][d][j]);
+            }
+#pragma unroll
+            for (int q = 0; q < Q; ++q)
+                if (q < nq) {
+                    const float2 dx = __fadd2_rn(pj[0], nb[q][0]), dy = __fadd2_rn(pj[1], nb[q][1]),
+                                 dz = __fadd2_rn(pj[2], nb[q][2]);
+                    float2 om1, om2;
+                    pair_weights2(dx, dy, dz, om1, om2);
+                    products(q, dx, dy, dz, om1, om2, xj);
+                }
+        }
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+#pragma unroll
+                for (int r = 0; r < K; ++r) acc[r][q][d] = valid(q) ? a[r][q][d].x + a[r][q][d].y : 0.f;
+    }
+
+    // Minus the coordinates of the thread's beads, both halves.
+    __device__ __forceinline__ void own_coordinates(float2 (&nb)[Q][3]) const {
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const float v = valid(q) ? -S.ps[d][bead(q)] : 0.f;
+                nb[q][d] = make_float2(v, v);
+            }
+    }
+
+    __device__ __forceinline__ static float rsqrt_approx(float x) {
+        float y;
+        asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+        return y;
+    }
+
+    // RPY weights of two pairs. In units of h*: with d = (R_j - R_b)/h*, s =
+    // |d|^2, rho = s^-1/2,
+    //   far  (s >= 4 pi): om1 = rho (K1 + K2 rho^2), om2 = rho^3 (K1 - K3 rho^2)
+    //   near (s <  4 pi): om1 = 1 - C3 s rho,         om2 = C7 rho
+    // and y_b += om1 x_j + om2 (d.x_j) d. The far weights are computed for all,
+    // the near ones in a branch that only neighbours along the chain and close
+    // contacts take. The self pair (d = 0, s clamped to 1e-24) is a near one
+    // with om1 = 1 exactly in FP32 and om2 d = 0: the identity block.
+    __device__ __forceinline__ void pair_weights2(const float2& dx, const float2& dy, const float2& dz, float2& om1,
+                                                  float2& om2) const {
+        const float2 k1 = make_float2(K1, K1), k2 = make_float2(K2, K2), mk3 = make_float2(-K3, -K3);
+        float2 sq = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+        sq = make_float2(fmaxf(sq.x, 1e-24f), fmaxf(sq.y, 1e-24f));
+        const float2 rho = make_float2(rsqrt_approx(sq.x), rsqrt_approx(sq.y));
+        const float2 t = __fmul2_rn(rho, rho);
+        om1 = __fmul2_rn(rho, __ffma2_rn(k2, t, k1));
+        om2 = __fmul2_rn(__fmul2_rn(rho, t), __ffma2_rn(mk3, t, k1));
+        const bool nx = sq.x < 12.566370614359172f, ny = sq.y < 12.566370614359172f;
+        if (nx || ny) {
+            const float2 n1 = __ffma2_rn(make_float2(-C3, -C3), __fmul2_rn(sq, rho), make_float2(1.f, 1.f));
+            const float2 n2 = __fmul2_rn(make_float2(C7, C7), rho);
+            if (nx) om1.x = n1.x, om2.x = n2.x;
+            if (ny) om1.y = n1.y, om2.y = n2.y;
+        }
+    }
+
+    // Weights of the thread's beads with partners below jc at the staged
+    // positions. Each thread reads back only its own columns (no barrier).
+    __device__ __forceinline__ void build_weights() {
+        float2 nb[Q][3];
+        own_coordinates(nb);
+#pragma unroll 1
+        for (int j = 0; j < jc; j += 2) {
+            float2 pj[3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) pj[d] = *reinterpret_cast<const float2*>(&S.ps[d][j]);
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                float2 om1, om2;
+                pair_weights2(__fadd2_rn(pj[0], nb[q][0]), __fadd2_rn(pj[1], nb[q][1]), __fadd2_rn(pj[2], nb[q][2]), om1,
+                              om2);
+                if (valid(q)) Wt[(j >> 1) * N + bead(q)] = make_float4(om1.x, om1.y, om2.x, om2.y);
+            }
         }
     }
 
@@ -493,7 +587,7 @@ struct TeamChain {
         apply32(x, y);
     }
 
-    __device__ double dotf(const float (&x)[Q][3], const float (&y)[Q][3]) const {
+    __device__ double dotf(const float (&x)[Q][3], const float (&y)[Q][3]) {
         double s = 0.0;
 #pragma unroll
         for (int q = 0; q < Q; ++q)
@@ -502,7 +596,7 @@ struct TeamChain {
         return tsum(s);
     }
 
-    __device__ double dot(const double (&x)[Q][3], const double (&y)[Q][3]) const {
+    __device__ double dot(const double (&x)[Q][3], const double (&y)[Q][3]) {
         double s = 0.0;
 #pragma unroll
         for (int q = 0; q < Q; ++q)
@@ -574,7 +668,6 @@ struct TeamChain {
         }
         // EV on the scaled coordinates: r = scale*|d|, force -fac(r) * scale * d
         const float zs = (float)(ch.zsbyds5 * scale), p5 = (float)(ch.pt5bydssq * (double)scale * scale);
-        const double* phi = (ch.ev_type == BDCU_EV_SDK && ch.phi_off >= 0) ? a.arena + ch.phi_off : nullptr;
         // excluded volume, FP32 pair sums over both bead slots at once: the
         // force on m from j is -fac(r) (R_j - R_m), |j - m| >= contour distance
         float fev[Q][3] = {};
@@ -599,20 +692,29 @@ struct TeamChain {
                 }
             }
         } else if (ch.ev_type != BDCU_EV_NONE) {
+            // LJ and SDK vanish beyond their outer cutoff: pairs outside it are
+            // passed over on the FP32 squared distance (a margin of 1e-5 covers
+            // its rounding; the cutoff itself is tested in FP64 on r). Each lane
+            // meets few partners inside, and the FP64 factor costs a hundred
+            // times the test.
+            const double* phi = (ch.ev_type == BDCU_EV_SDK && ch.phi_off >= 0) ? a.arena + ch.phi_off : nullptr;
+            const double cut = ev_outer_cutoff(ch) * (double)iscale, s2 = (double)scale * scale;
+            const float cut2 = (float)(cut * cut * 1.00001);
+            float4 pm[Q];
 #pragma unroll
-            for (int q = 0; q < Q; ++q) {
-                const int m = bead(q);
-                if (!valid(q)) continue;
-                const float4 pm = S.pos[m];
-                for (int j = 0; j < N; ++j) {
-                    const int dj = j > m ? j - m : m - j;
-                    if (dj < ch.cd || j == m) continue;
-                    const float4 pj = S.pos[j];
-                    const float dx = pj.x - pm.x, dy = pj.y - pm.y, dz = pj.z - pm.z;
+            for (int q = 0; q < Q; ++q) pm[q] = valid(q) ? S.pos[bead(q)] : make_float4(3e18f, 3e18f, 3e18f, 0.f);
+#pragma unroll 2
+            for (int j = 0; j < N; ++j) {
+                const float4 pj = S.pos[j];
+#pragma unroll
+                for (int q = 0; q < Q; ++q) {
+                    const int m = bead(q);
+                    const float dx = pj.x - pm[q].x, dy = pj.y - pm[q].y, dz = pj.z - pm[q].z;
                     const float sq = fmaxf(dx * dx + dy * dy + dz * dz, 1e-12f);
+                    const int dj = j > m ? j - m : m - j;
+                    if (!(sq <= cut2) || dj < ch.cd || j == m || m >= N) continue;
                     const int mu = j < m ? j : m, nu = j < m ? m : j;
-                    const float fac =
-                        (float)(ev_factor(ch, sqrt((double)sq) * scale, phi ? phi[mu * N + nu] : 0.0) * scale);
+                    const float fac = (float)(ev_factor_short(ch, (double)sq * s2, phi ? phi + (int64_t)mu * N + nu : nullptr) * scale);
                     fev[q][0] -= fac * dx;
                     fev[q][1] -= fac * dy;
                     fev[q][2] -= fac * dz;
@@ -646,54 +748,38 @@ struct TeamChain {
     }
 
     // ---- noise: the 3N draws of raw_noise (src/mobility.cpp:18-29) -------
-    // The team's threads draw contiguous blocks of the stream; thread u jumps
-    // to draw u*c with the tabulated powers, so the uniforms equal ran_1's,
-    // bit for bit.
-    __device__ void noise(uint32_t& ux0, int32_t& iy0, int32_t& seed, float (&X)[Q][3]) {
-        if (seed <= 0 || iy0 < 0) {
-            const int32_t s = seed < 0 ? -seed : seed;
-            iy0 = (888889999 ^ s) | 1;
-            ux0 = (uint32_t)(777755555 ^ s);
-            seed = s + 1;
+    // The team's threads draw contiguous blocks of c draws of the stream. Each
+    // keeps the generator's state at the start of its block: jumped there once
+    // per chain with the tabulated powers, and from step to step by the same 3N
+    // draws for every thread, so the uniforms equal ran_1's, bit for bit.
+    __device__ __forceinline__ void noise_start(uint32_t& ux, int32_t& iy, int32_t& sd) {
+        if (sd <= 0 || iy < 0) {
+            const int32_t s = sd < 0 ? -sd : sd;
+            iy = (888889999 ^ s) | 1;
+            ux = (uint32_t)(777755555 ^ s);
+            sd = s + 1;
         }
-        const int c = (n + TT - 1) / TT;
-        const int k0 = tid * c;
-        const int k1 = min(n, k0 + c);
-        uint32_t ux = 0;
-        int32_t iy = 0;
-        if (k0 < n) {
-            const uint32_t* cols = a.xs_pow + 32 * (int64_t)k0;
-#pragma unroll 8
-            for (int i = 0; i < 32; ++i) ux ^= cols[i] & (0u - ((ux0 >> i) & 1u));
-            iy = (int32_t)(((uint64_t)a.a_pow[k0] * (uint64_t)(uint32_t)iy0) % 2147483647ull);
-            const float am = __fdiv_rn(__int_as_float(0x3f7fffff), 2147483648.0f);
-            for (int k = k0; k < k1; ++k) {
-                ux ^= (ux << 13);
-                ux ^= (ux >> 17);
-                ux ^= (ux << 5);
-                const int32_t kk = iy / 127773;
-                iy = 16807 * (iy - kk * 127773) - 2836 * kk;
-                if (iy < 0) iy += 2147483647;
-                const uint32_t mixed = ux ^ (uint32_t)iy;
-                const int32_t res = (int32_t)((mixed & 0x7fffffffu) | 1u);
-                S.s0[k] = (double)__fmul_rn(am, __int2float_rn(res));
-            }
+        const int k0 = min(tid * ((n + TT - 1) / TT), n);
+        ux = xorshift_jump(a.xs_pow + 32 * (int64_t)k0, ux);
+        iy = (int32_t)lehmer_mul(a.a_pow[k0], (uint32_t)iy);
+        if (tid < 32) S.jcols[tid] = a.xs_pow[32 * (int64_t)n + tid];
+        sync();
+    }
+    __device__ void noise(uint32_t& ux0, int32_t& iy0, float (&X)[Q][3]) {
+        const int c = (n + TT - 1) / TT, k0 = tid * c, k1 = min(n, k0 + c);
+        const float am = __fdiv_rn(__int_as_float(0x3f7fffff), 2147483648.0f);
+        uint32_t ux = ux0, iy = (uint32_t)iy0;
+        for (int k = k0; k < k1; ++k) {
+            ux ^= (ux << 13);
+            ux ^= (ux >> 17);
+            ux ^= (ux << 5);
+            iy = lehmer_mul(16807u, iy);
+            const int32_t res = (int32_t)(((ux ^ iy) & 0x7fffffffu) | 1u);
+            S.s0[k] = (double)__fmul_rn(am, __int2float_rn(res));
         }
-        // the state after the last draw, from the thread that made it
-        const int last = (n - 1) / c;
-        if constexpr (T == 1) {
-            ux0 = __shfl_sync(kFull, ux, last);
-            iy0 = __shfl_sync(kFull, iy, last);
-            __syncwarp();
-        } else {
-            if (tid == last) {
-                S.bu = ux;
-                S.bi = iy;
-            }
-            sync();
-            ux0 = S.bu;
-            iy0 = S.bi;
-        }
+        ux0 = xorshift_jump(S.jcols, ux0);
+        iy0 = (int32_t)lehmer_mul(a.a_pow[n], (uint32_t)iy0);
+        sync();
 #pragma unroll
         for (int q = 0; q < Q; ++q)
 #pragma unroll
@@ -724,142 +810,133 @@ struct TeamChain {
                 for (int d = 0; d < 3; ++d) vec[3 * bead(q) + d] = x[q][d];
     }
 
-    // Lanczos start vector (src/hydrodynamics.cpp:152-155): the normalised
-    // warm-start cache, or the normalised default seed when cold or when the
-    // cache is zero.
-    __device__ void start_vector(bool warm, const double* cache, double (&v)[Q][3]) const {
-        double nv2 = 0.0;
+    // Lanczos start vector (src/hydrodynamics.cpp:152-155): the warm-start
+    // vector, normalised unless it is a unit vector to rounding (as every vector
+    // of an earlier step is: a run then does not depend on where it was cut),
+    // or the normalised default seed when cold or zero.
+    __device__ void start_vector(bool warm, const double* cache, double (&v)[Q][3]) {
         if (warm) {
             load(cache, v);
-            nv2 = sqrt(dot(v, v));
-        }
-        if (!(nv2 > 0.0)) {
-            load(a.seed_table, v);
-            nv2 = ch.seed_norm;
-        }
-        const double inv = 1.0 / nv2;
+            const double n2 = dot(v, v);
+            if (n2 > 0.0) {
+                if (fabs(n2 - 1.0) > 1.0e-13) {
+                    const double inv = 1.0 / sqrt(n2);
 #pragma unroll
-        for (int q = 0; q < Q; ++q)
+                    for (int q = 0; q < Q; ++q)
 #pragma unroll
-            for (int d = 0; d < 3; ++d) v[q][d] *= inv;
+                        for (int d = 0; d < 3; ++d) v[q][d] *= inv;
+                }
+                return;
+            }
+        }
+        load(S.seed, v);
     }
+
+    // w -= sum_i (V_i.w) V_i over the first nv vectors of the cold basis, all
+    // projections reduced together (one barrier).
+    __device__ __forceinline__ void project(int nv, double (&w)[Q][3]) {
+        double* r = S.proj;
+        sync();
+#pragma unroll 1
+        for (int u0 = 0; u0 < nv; u0 += 8) {
+            double c[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                double x[Q][3], t = 0.0;
+                load(Vg + (int64_t)min(u0 + i, nv - 1) * nv_stride(), x);
+#pragma unroll
+                for (int q = 0; q < Q; ++q)
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) t += w[q][d] * x[q][d];
+                c[i] = u0 + i < nv ? t : 0.0;
+            }
+            warp_sum8(c, r + u0 * T);
+        }
+        sync();
+#pragma unroll 1
+        for (int u = 0; u < nv; ++u) {
+            double x[Q][3];
+            load(Vg + (int64_t)u * nv_stride(), x);
+            const double c = total(r, u);
+#pragma unroll
+            for (int q = 0; q < Q; ++q)
+#pragma unroll
+                for (int d = 0; d < 3; ++d) w[q][d] -= c * x[q][d];
+        }
+    }
+    __device__ __forceinline__ int nv_stride() const { return nv; }
 
     // Returns the number of Lanczos steps; sets rmin/rmax and the Ritz vectors.
     // v0: the start vector; if have_dv0, dv0 = D v0 (computed by the caller
     // together with the step's other independent products).
+    // Warm runs (8 steps from the previous step's Ritz vectors) use the
+    // three-term recurrence without reorthogonalisation: in 8 FP64 steps the
+    // loss of orthogonality leaves the extreme Ritz values far inside the 2x /
+    // 2% padding of the bounds, and the Chebyshev fluctuation-dissipation check
+    // polices the result. Cold runs (30 steps, the first step of a call) project
+    // on the whole basis in two steps of every six (below 3N = 64 in every
+    // step), which keeps it orthogonal to about 1e-11; the reference's modified
+    // Gram-Schmidt took up to 30 reductions in turn per step. One reduction per
+    // step: the new vector u goes into the product unnormalised, and u.u and u.Du
+    // are summed together.
     __device__ int lanczos(int m, bool warm, const double (&v0)[Q][3], const double (&dv0)[Q][3], bool have_dv0,
                            double (&vmin)[Q][3], double (&vmax)[Q][3], double& rmin, double& rmax) {
         if (n < m) m = n;
-        double v[Q][3], w[Q][3], vp[Q][3];
+        const bool cold = !(m <= kLanczosWarm), every = n < 64;
+        double u[Q][3], w[Q][3], vp[Q][3];
 #pragma unroll
         for (int q = 0; q < Q; ++q)
 #pragma unroll
-            for (int d = 0; d < 3; ++d) v[q][d] = v0[q][d];
-#pragma unroll
-        for (int q = 0; q < Q; ++q)
-#pragma unroll
-            for (int d = 0; d < 3; ++d) vp[q][d] = 0.0;
-        int k = 0;
-        double b = 0.0;
-        if (m <= kLanczosWarm) {
-            // warm runs (8 steps from the previous step's Ritz vectors): the
-            // three-term recurrence without reorthogonalisation. In 8 FP64
-            // steps the loss of orthogonality (of order eps over the accuracy
-            // of the converged Ritz values) leaves the extreme Ritz values far
-            // inside the 2x / 2% padding of the bounds, and the Chebyshev
-            // fluctuation-dissipation check polices the result. One batched
-            // team sum per step gives alpha = v.w and |w|^2, so beta^2 =
-            // |w|^2 - alpha^2 (Pythagoras, |v| = 1); when that cancels by more
-            // than 99% beta comes from an explicit norm. The last step's beta
-            // is not needed (it is not an entry of T).
-            for (int j = 0; j < m; ++j) {
-                store(basis(j, m), v);
-                if (j == 0 && have_dv0) {
-#pragma unroll
-                    for (int q = 0; q < Q; ++q)
-#pragma unroll
-                        for (int d = 0; d < 3; ++d) w[q][d] = dv0[q][d];
-                } else {
-                    apply(v, w);
-                }
-                if (j > 0)
-#pragma unroll
-                    for (int q = 0; q < Q; ++q)
-#pragma unroll
-                        for (int d = 0; d < 3; ++d) w[q][d] -= b * vp[q][d];
-                double c[kLanczosWarm];
-#pragma unroll
-                for (int u = 0; u < kLanczosWarm; ++u) c[u] = 0.0;
-#pragma unroll
-                for (int q = 0; q < Q; ++q)
-#pragma unroll
-                    for (int d = 0; d < 3; ++d) {
-                        c[0] += v[q][d] * w[q][d];
-                        c[1] += w[q][d] * w[q][d];
-                    }
-                tsum8(c);
-                const double al = c[0];
-#pragma unroll
-                for (int q = 0; q < Q; ++q)
-#pragma unroll
-                    for (int d = 0; d < 3; ++d) w[q][d] -= al * v[q][d];
-                if (tid == 0) S.alpha[k] = al;
-                ++k;
-                if (j == m - 1) break;
-                double bsq = c[1] - al * al;
-                if (!(bsq >= 0.01 * c[1])) bsq = dot(w, w);
-                b = sqrt(bsq);
-                if (b < 1.0e-10) break;
-                const double ib = 1.0 / b;
-#pragma unroll
-                for (int q = 0; q < Q; ++q)
-#pragma unroll
-                    for (int d = 0; d < 3; ++d) {
-                        vp[q][d] = v[q][d];
-                        v[q][d] = w[q][d] * ib;
-                    }
-                if (tid == 0) S.beta[j] = b;
+            for (int d = 0; d < 3; ++d) {
+                u[q][d] = v0[q][d];
+                w[q][d] = dv0[q][d];
+                vp[q][d] = 0.0;
             }
-        } else {
-            // cold runs (first step of a call): the reference's modified Gram-Schmidt
-            for (int j = 0; j < m; ++j) {
-                store(basis(j, m), v);
-                if (j == 0 && have_dv0) {
+        int k = 0;
+        double bprev = 1.0;
+        bool due = false;
+#pragma unroll 1
+        for (int j = 0;; ++j) {
+            if (j > 0 || !have_dv0) apply(u, w);
+            double g[2] = {0.0, 0.0};
 #pragma unroll
-                    for (int q = 0; q < Q; ++q)
+            for (int q = 0; q < Q; ++q)
 #pragma unroll
-                        for (int d = 0; d < 3; ++d) w[q][d] = dv0[q][d];
-                } else {
-                    apply(v, w);
+                for (int d = 0; d < 3; ++d) {
+                    g[0] += u[q][d] * u[q][d];
+                    g[1] += u[q][d] * w[q][d];
                 }
-                const double al = dot(v, w);
-                if (tid == 0) S.alpha[k] = al;
-                ++k;
+            sums(g);
+            if (j > 0 && g[0] < 1.0e-20) {
+                cnt[C_DX] -= 1;  // (the reference stops before this product)
+                break;
+            }
+            const double ib = rsqrt_refined(g[0]), bt = g[0] * ib, al = (g[1] * ib) * ib;
+            if (tid == 0) {
+                S.alpha[j] = al;
+                if (j > 0) S.beta[j - 1] = bt;
+            }
+            ++k;
+            double v[Q][3];
 #pragma unroll
-                for (int q = 0; q < Q; ++q)
+            for (int q = 0; q < Q; ++q)
 #pragma unroll
-                    for (int d = 0; d < 3; ++d) w[q][d] -= al * v[q][d] + b * vp[q][d];
-                sync();
-                for (int u = 0; u <= j; ++u) {
-                    double uu[Q][3];
-                    load(basis(u, m), uu);
-                    const double dd = dot(w, uu);
+                for (int d = 0; d < 3; ++d) v[q][d] = u[q][d] * ib;
+            store(basis(j, m), v);
+            if (j == m - 1) break;  // (the last beta is no entry of the tridiagonal)
 #pragma unroll
-                    for (int q = 0; q < Q; ++q)
+            for (int q = 0; q < Q; ++q)
 #pragma unroll
-                        for (int d = 0; d < 3; ++d) w[q][d] -= dd * uu[q][d];
+                for (int d = 0; d < 3; ++d) {
+                    u[q][d] = w[q][d] * ib - al * v[q][d];
+                    if (j > 0) u[q][d] -= bt * vp[q][d];
+                    vp[q][d] = v[q][d];
                 }
-                b = sqrt(dot(w, w));
-                if (b < 1.0e-10) break;
-                const double ib = 1.0 / b;
-#pragma unroll
-                for (int q = 0; q < Q; ++q)
-#pragma unroll
-                    for (int d = 0; d < 3; ++d) {
-                        vp[q][d] = v[q][d];
-                        v[q][d] = w[q][d] * ib;
-                    }
-                if (tid == 0) S.beta[j] = b;
+            if (cold) {
+                // a beta far below its neighbours magnifies what orthogonality was lost
+                due = due ? bt < 0.1 * bprev : bt < 0.03 * fabs(al) || bt < 0.1 * bprev;
+                bprev = bt;
+                if (every || due || j % 6 >= 4) project(j + 1, u);
             }
         }
         sync();
@@ -946,19 +1023,18 @@ struct TeamChain {
         return k;
     }
 
-    // spectral_bounds (src/hydrodynamics.cpp:224-264): the warm-start vector
-    // lives in the chain's cache slice.
+    // spectral_bounds (src/hydrodynamics.cpp:224-264). v0: the start vector,
+    // replaced by the next step's.
     // The step's three mutually independent products against D(R) run in
     // one pass first: D v0 (the Lanczos start vector), D X0 (the noise, for
     // the Chebyshev series) and D A (A = Fs + Fe, the predictor's force).
     // fuse: also form DX0 = D X0 and DA = D A in the start vector's pass;
     // otherwise the caller has them and the Lanczos forms D v0 itself.
-    __device__ void bounds(double* cache, int& cache_valid, double& lmin, double& lmax, const float (&X0)[Q][3],
+    __device__ void bounds(double (&v0)[Q][3], int& cache_valid, double& lmin, double& lmax, const float (&X0)[Q][3],
                            const float (&A)[Q][3], float (&DX0)[Q][3], float (&DA)[Q][3], bool fuse = true) {
         double vmin[Q][3], vmax[Q][3], rmin, rmax;
         const bool can_warm = cache_valid != 0;
-        double v0[Q][3], dv0[Q][3];
-        start_vector(can_warm, cache, v0);
+        double dv0[Q][3];
         if (fuse) {
             float x3[3][Q][3], y3[3][Q][3];
 #pragma unroll
@@ -982,31 +1058,25 @@ struct TeamChain {
         const int steps =
             lanczos(can_warm ? kLanczosWarm : kLanczosCold, can_warm, v0, dv0, fuse, vmin, vmax, rmin, rmax);
         if (can_warm && steps < 4) {
-            start_vector(false, cache, v0);
+            start_vector(false, nullptr, v0);
             lanczos(kLanczosCold, false, v0, dv0, false, vmin, vmax, rmin, rmax);
             cnt[C_LZCOLD] += 1;
         } else {
             cnt[can_warm ? C_LZWARM : C_LZCOLD] += 1;
         }
-        double s[Q][3], u[Q][3];
-        load(a.seed_table, u);
-        const double iun = 1.0 / ch.seed_norm;
+        double sd[Q][3];
+        load(S.seed, sd);
 #pragma unroll
         for (int q = 0; q < Q; ++q)
 #pragma unroll
-            for (int d = 0; d < 3; ++d) s[q][d] = vmin[q][d] + vmax[q][d] + 0.01 * u[q][d] * iun;
-        const double sn = sqrt(dot(s, s));
-        if (sn > 0.0 && isfinite(sn)) {
-            const double is = 1.0 / sn;
+            for (int d = 0; d < 3; ++d) v0[q][d] = vmin[q][d] + vmax[q][d] + 0.01 * sd[q][d];
+        const double s2 = dot(v0, v0);
+        cache_valid = (s2 > 0.0 && isfinite(s2)) ? 1 : 0;
+        const double is = rsqrt_refined(s2);
 #pragma unroll
-            for (int q = 0; q < Q; ++q)
+        for (int q = 0; q < Q; ++q)
 #pragma unroll
-                for (int d = 0; d < 3; ++d) s[q][d] *= is;
-            store(cache, s);
-            cache_valid = 1;
-        } else {
-            cache_valid = 0;
-        }
+            for (int d = 0; d < 3; ++d) v0[q][d] = cache_valid ? v0[q][d] * is : sd[q][d];
         lmin = 0.5 * rmin;
         lmax = 1.02 * rmax;
         if (lmin < 1.0e-12) lmin = 1.0e-12;
@@ -1028,17 +1098,27 @@ struct TeamChain {
         const float db = (float)(-(lmax + lmin) / (lmax - lmin));
         double fd = 0.0;
         for (;;) {
-            const float inv = 1.f / (float)(L + 1);
+            // every cosine of the coefficient sums is cos(pi m / 2P), P = L + 1,
+            // with integer m: one table of P + 1 values
+            const int P = L + 1;
             const float ida = 1.f / da;
-            for (int k = tid; k <= L; k += TT) {
-                const float xk = (cospif(((float)k + 0.5f) * inv) - db) * ida;
-                sqx[k] = sqrtf(xk);
+            for (int m = tid; m <= P; m += TT) ct[m] = cospif((float)m / (float)(2 * P));
+            sync();
+            for (int k = tid; k < P; k += TT) {
+                const int m = 2 * k + 1;
+                sqx[k] = sqrtf(((m <= P ? ct[m] : -ct[2 * P - m]) - db) * ida);
             }
             sync();
-            for (int j = tid; j <= L; j += TT) {
+            for (int j = tid; j < P; j += TT) {
                 float s = 0.f;
-                for (int k = 0; k <= L; ++k) s += sqx[k] * cospif((float)j * ((float)k + 0.5f) * inv);
-                s *= 2.f * inv;
+                int m = j;  // j (2k + 1) modulo 4P
+                for (int k = 0; k < P; ++k) {
+                    const int h = m > 2 * P ? 4 * P - m : m;
+                    s += sqx[k] * (h <= P ? ct[h] : -ct[2 * P - h]);
+                    m += 2 * j;
+                    if (m >= 4 * P) m -= 4 * P;
+                }
+                s *= 2.f / (float)P;
                 if (j == 0) s *= 0.5f;
                 coef[j] = s;
             }
@@ -1159,7 +1239,7 @@ __global__ void __launch_bounds__(TeamCfg<T, Q>::kCtaThreads, TeamCfg<T, Q>::kMi
     constexpr int TT = TeamCfg<T, Q>::kThreads;
     const int team = threadIdx.x / TT;
     const int tid = threadIdx.x % TT;
-    const int64_t stride = team_area_stride<T, Q>(a.n_max);
+    const int64_t stride = team_area_stride<T, Q>(a.n_max, a.w_pairs);
     TeamShared<T, Q>& S = *reinterpret_cast<TeamShared<T, Q>*>(wsm + stride * team);
     double* Vs = reinterpret_cast<double*>(wsm + stride * team + (sizeof(TeamShared<T, Q>) + 15) / 16 * 16);
     const int64_t gw = (int64_t)blockIdx.x * TeamCfg<T, Q>::kTeamsPerCta + team;
@@ -1193,6 +1273,9 @@ __global__ void __launch_bounds__(TeamCfg<T, Q>::kCtaThreads, TeamCfg<T, Q>::kMi
         W.V = Vs;
         W.sqx = reinterpret_cast<float*>(Vs);
         W.coef = reinterpret_cast<float*>(Vs) + kCoefCap;
+        W.ct = reinterpret_cast<float*>(Vs) + 2 * kCoefCap;
+        W.Wt = reinterpret_cast<float4*>(reinterpret_cast<unsigned char*>(&S) + team_weight_offset<T, Q>(a.n_max));
+        W.par = W.xpar = 0;
         W.Vg = scr;
         W.Lt = scr + (int64_t)kLanczosCold * nvr;
         W.nv = nvr;
@@ -1202,6 +1285,7 @@ __global__ void __launch_bounds__(TeamCfg<T, Q>::kCtaThreads, TeamCfg<T, Q>::kMi
         W.team = team;
         W.N = ch.N;
         W.n = 3 * ch.N;
+        W.jc = 2 * (int)min((int64_t)(ch.N + 1) / 2, a.w_pairs / ch.N);
         W.hi = ch.hstar > 0.0;
         W.status = status;
         for (int k = 0; k < 8; ++k) W.cnt[k] = 0;
@@ -1221,14 +1305,28 @@ __global__ void __launch_bounds__(TeamCfg<T, Q>::kCtaThreads, TeamCfg<T, Q>::kMi
         double* gcache = a.cache + 3 * ch.bead_off;
         int cache_valid = (a.cache_mode == BDCU_CACHE_PERSIST) ? a.cache_valid[c] : 0;
         uint32_t ux = (uint32_t)a.rng[3 * c];
-        int32_t iy = a.rng[3 * c + 1], seed = a.rng[3 * c + 2];
+        int32_t iy = a.rng[3 * c + 1], sd = a.rng[3 * c + 2];
+        W.noise_start(ux, iy, sd);
+        bool drew = false, used_cache = false;
+        double v0[Q][3];  // the Lanczos start vector, kept from step to step
+        if (W.hi) {
+            double s0[Q][3];
+            W.load(a.seed_table, s0);
+            const double iun = 1.0 / ch.seed_norm;
+#pragma unroll
+            for (int q = 0; q < Q; ++q)
+#pragma unroll
+                for (int d = 0; d < 3; ++d) s0[q][d] *= iun;
+            W.store(S.seed, s0);  // (each thread reads back only its own)
+            W.start_vector(cache_valid != 0, gcache, v0);
+        }
         double R[Q][3];
         W.load(gR, R);
         const int nsteps = a.n_steps[c];
         double t = a.t_start[c];
         const double dt = ch.dt;
         const double sqrt2inv = 1.0 / sqrt(2.0);
-        const double sqrt_dt = sqrt(dt);
+        const double sqrt_dt = sqrt(dt), inv_n = 1.0 / N;
         // spectral bounds kept between refreshes (a launch starts with a refresh)
         const int bounds_every = a.bounds_every > 1 ? a.bounds_every : 1;
         int since_bounds = bounds_every;
@@ -1240,12 +1338,15 @@ __global__ void __launch_bounds__(TeamCfg<T, Q>::kCtaThreads, TeamCfg<T, Q>::kMi
             // recenter (src/integrator.cpp:88-93)
             if (ch.update_com) {
                 double com[3];
-                for (int d = 0; d < 3; ++d) {
-                    double s = 0.0;
 #pragma unroll
-                    for (int q = 0; q < Q; ++q) s += R[q][d];
-                    com[d] = (1.0 / N) * W.tsum(s);
+                for (int d = 0; d < 3; ++d) {
+                    com[d] = 0.0;
+#pragma unroll
+                    for (int q = 0; q < Q; ++q) com[d] += R[q][d];
                 }
+                W.sums(com);
+#pragma unroll
+                for (int d = 0; d < 3; ++d) com[d] *= inv_n;
 #pragma unroll
                 for (int q = 0; q < Q; ++q)
                     if (W.valid(q))
@@ -1255,7 +1356,9 @@ __global__ void __launch_bounds__(TeamCfg<T, Q>::kCtaThreads, TeamCfg<T, Q>::kMi
             float Fs[Q][3], Fe[Q][3];
             W.forces(R, t, Fs, Fe, true);
             float X0[Q][3], dW[Q][3], A[Q][3], DF[Q][3];
-            W.noise(ux, iy, seed, X0);
+            W.noise(ux, iy, X0);
+            drew = true;
+            if (W.hi) W.build_weights();
             // brownian_step (src/mobility.cpp:58-88)
             if (!W.hi) {
 #pragma unroll
@@ -1270,7 +1373,8 @@ __global__ void __launch_bounds__(TeamCfg<T, Q>::kCtaThreads, TeamCfg<T, Q>::kMi
                     for (int d = 0; d < 3; ++d) A[q][d] = Fs[q][d] + Fe[q][d];
                 double fd;
                 if (since_bounds >= bounds_every) {
-                    W.bounds(gcache, cache_valid, lmin, lmax, X0, A, DX0, DF);
+                    W.bounds(v0, cache_valid, lmin, lmax, X0, A, DX0, DF);
+                    used_cache = true;
                     since_bounds = 0;
                     fd = W.chebyshev(X0, DX0, lmin, lmax, bx);
                 } else {
@@ -1293,7 +1397,8 @@ __global__ void __launch_bounds__(TeamCfg<T, Q>::kCtaThreads, TeamCfg<T, Q>::kMi
                         }
                     fd = W.chebyshev(X0, DX0, lmin, lmax, bx, false);
                     if (!(fd <= ch.fd_tol)) {  // the kept bounds no longer hold: refresh and redo
-                        W.bounds(gcache, cache_valid, lmin, lmax, X0, A, DX0, DF, false);
+                        W.bounds(v0, cache_valid, lmin, lmax, X0, A, DX0, DF, false);
+                        used_cache = true;
                         since_bounds = 0;
                         fd = W.chebyshev(X0, DX0, lmin, lmax, bx);
                     }
@@ -1562,11 +1667,14 @@ __global__ void __launch_bounds__(TeamCfg<T, Q>::kCtaThreads, TeamCfg<T, Q>::kMi
             W.cnt[C_STEPS] += 1;
             t += dt;
         }
+        if (used_cache && cache_valid) W.store(gcache, v0);
         if (!(W.status & BDCU_ST_FATAL_MASK)) W.store(gR, R);
         if (tid == 0) {
-            a.rng[3 * c] = (int32_t)ux;
-            a.rng[3 * c + 1] = iy;
-            a.rng[3 * c + 2] = seed;
+            if (drew) {  // (lazy seeding belongs to the first draw)
+                a.rng[3 * c] = (int32_t)ux;
+                a.rng[3 * c + 1] = iy;
+                a.rng[3 * c + 2] = sd;
+            }
             a.cache_valid[c] = cache_valid;
             a.status[c] = W.status;
             int64_t* cc = reinterpret_cast<int64_t*>(a.counters + c);

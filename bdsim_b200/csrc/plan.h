@@ -37,11 +37,18 @@ inline int bucket_of(const DevChain& c, int form, bool pair = true) {
                          : FALLBACK
 
 // Shared memory of a team-kernel block of shape (T, Q) for chains of up to
-// n_max/3 beads (-1: no such shape).
-inline int64_t team_smem(int T, int Q, int n_max) {
-#define BDCU_SMEM(t, q) team_smem_bytes<t, q>(n_max)
+// n_max/3 beads with w_pairs cached weights per team (-1: no such shape).
+inline int64_t team_smem(int T, int Q, int n_max, int64_t w_pairs) {
+#define BDCU_SMEM(t, q) (team_smem_bytes<t, q>(n_max, w_pairs))
     return BDCU_TEAM_SHAPE_SWITCH(T, Q, BDCU_SMEM, (int64_t)-1);
 #undef BDCU_SMEM
+}
+
+// Cached weights per team of shape (T, Q).
+inline int64_t team_weights(int T, int Q, int n_max, size_t max_smem) {
+#define BDCU_WTS(t, q) (team_cached<t, q>(n_max, max_smem))
+    return BDCU_TEAM_SHAPE_SWITCH(T, Q, BDCU_WTS, (int64_t)0);
+#undef BDCU_WTS
 }
 
 inline int teams_per_cta(int T, int Q) {

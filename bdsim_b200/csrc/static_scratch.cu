@@ -145,7 +145,7 @@ extern "C" int bdcu_run_static(bdcu_ctx* ctx, int n_chains, const bdcu_phys* phy
     struct Launch {
         int id, team_warps, team_q, block, grid, v_cap, d_in_smem, n_max, need_d, need_lz, count;
         size_t smem, per_block;
-        int64_t stride, order_off;
+        int64_t stride, order_off, w_pairs;
     };
     std::vector<Launch> launches;
     std::vector<int32_t> order;
@@ -172,7 +172,8 @@ extern "C" int bdcu_run_static(bdcu_ctx* ctx, int n_chains, const bdcu_phys* phy
             any_team = true;
             l.team_warps = kDefaultTeamShape[id][0];
             l.team_q = kDefaultTeamShape[id][1];
-            l.smem = (size_t)team_smem(l.team_warps, l.team_q, l.n_max);
+            l.w_pairs = l.need_d ? team_weights(l.team_warps, l.team_q, l.n_max, ctx->max_smem) : 0;
+            l.smem = (size_t)team_smem(l.team_warps, l.team_q, l.n_max, l.w_pairs);
             if (l.smem > ctx->max_smem) return fail(ctx, BDCU_E_LIMIT, "bdcu_run_static: team kernel shared memory too large");
             e = occupancy_mixed_team(l.team_warps, l.team_q, l.smem, &per_sm);
             l.stride = l.need_d ? team_scratch_doubles(l.n_max) : 1;
@@ -288,6 +289,7 @@ extern "C" int bdcu_run_static(bdcu_ctx* ctx, int n_chains, const bdcu_phys* phy
         a.need_chol = l.need_d;
         a.need_d = l.need_d;
         a.need_lz = l.need_lz;
+        a.w_pairs = l.w_pairs;
         a.work_counter = reinterpret_cast<int32_t*>(b + o_cnt) + l.id;
         a.scratch = reinterpret_cast<double*>(b + o_scr);
         a.scratch_stride = l.stride;

@@ -33,9 +33,9 @@ struct TeamCfg {
 };
 
 // Per-team shared memory (fixed part). The warm Lanczos basis
-// (kLanczosWarm x nv doubles) follows it; the Chebyshev node and coefficient
-// tables (2 x kCoefCap floats) share that area, as the basis is dead once the
-// spectral bounds are known.
+// (kLanczosWarm x nv doubles) follows it; the Chebyshev cosine, node and
+// coefficient tables (3 x kCoefCap floats) share that area, as the basis is dead
+// once the spectral bounds are known. Cached pair weights come last.
 template <int T, int Q>
 struct TeamShared {
     float4 pos[32 * T * Q];   // FP32 bead coordinates of the tensor's configuration
@@ -48,26 +48,41 @@ struct TeamShared {
     double s3[32 * T * Q > 64 ? 32 * T * Q : 64];
     double s4[32 * T * Q > 64 ? 32 * T * Q : 64];
     double alpha[32], beta[32], ymin[32], ymax[32];
-    double red[8 * T];    // per-warp partial sums (up to 8 reduced together)
+    double red[2][3 * T]; // per-warp partial sums, two buffers used in turn
+    double proj[32 * T];  // per-warp partial projections of a cold Lanczos step
+    double seed[96 * T * Q];  // normalised default Lanczos seed
     double tot[6 * T];    // per-warp scan totals (2 bead slots x 3 components)
     double rr[2];         // extreme Ritz values
-    uint32_t bu;          // RNG state handed from the last drawing thread
-    int32_t bi;
+    uint32_t jcols[32];   // columns of the xorshift matrix power 3N
     int32_t item;         // claimed chain
     int32_t flag[T];      // per-warp status bits
     DevChain ch;
 };
 
 template <int T, int Q>
-__host__ __device__ inline int64_t team_area_stride(int n_max) {
+__host__ __device__ inline int64_t team_weight_offset(int n_max) {
     const int64_t nv = round_up8(n_max);
     int64_t area = (int64_t)kLanczosWarm * nv * 8;
-    if (area < (int64_t)2 * kCoefCap * 4) area = (int64_t)2 * kCoefCap * 4;
-    return (int64_t)((sizeof(TeamShared<T, Q>) + 15) / 16 * 16) + area;
+    if (area < (int64_t)3 * kCoefCap * 4) area = (int64_t)3 * kCoefCap * 4;
+    return ((int64_t)((sizeof(TeamShared<T, Q>) + 15) / 16 * 16) + area + 15) / 16 * 16;
 }
 template <int T, int Q>
-__host__ __device__ inline int64_t team_smem_bytes(int n_max) {
-    return team_area_stride<T, Q>(n_max) * TeamCfg<T, Q>::kTeamsPerCta;
+__host__ __device__ inline int64_t team_area_stride(int n_max, int64_t w_pairs) {
+    return team_weight_offset<T, Q>(n_max) + 16 * w_pairs;
+}
+template <int T, int Q>
+__host__ __device__ inline int64_t team_smem_bytes(int n_max, int64_t w_pairs) {
+    return team_area_stride<T, Q>(n_max, w_pairs) * TeamCfg<T, Q>::kTeamsPerCta;
+}
+// Cached weights per team (16 bytes: a bead with two partners): all of the
+// largest chain's when they fit the team's share of an SM's shared memory at the
+// blocks per SM the registers are sized for, else as many as fit.
+template <int T, int Q>
+inline int64_t team_cached(int n_max, size_t max_smem) {
+    const int64_t share = ((int64_t)max_smem + 1024) / TeamCfg<T, Q>::kMinBlocks - 1024;
+    const int64_t room = (share / TeamCfg<T, Q>::kTeamsPerCta - team_weight_offset<T, Q>(n_max)) / 16;
+    const int64_t N = n_max / 3, all = (N + 1) / 2 * N;
+    return room <= 0 ? 0 : room < all ? room : all;
 }
 
 // Per-team global scratch (doubles): cold Lanczos basis, Cholesky factor.
