@@ -276,11 +276,9 @@ void free_staging(Staging& st) {
 // ------------------------------------------------------------ launch plans
 
 // Launch shapes of the block kernel for a bucket, the heuristic's choice first:
-// widest block, dense D in shared memory when it fits (plain form), then as
-// many Lanczos vectors in shared memory as fit.
+// widest block, as many Lanczos vectors in shared memory as fit.
 std::vector<Shape> block_shapes(const bdcu_ctx* ctx, const Bucket& b, int form) {
     const int mixed = form == BDCU_FORM_MIXED_FP32;
-    const std::vector<int> d_opts = (!mixed && b.need_d) ? std::vector<int>{1, 0} : std::vector<int>{0};
     const std::vector<int> v_opts = b.need_lz ? std::vector<int>{kLanczosCold, kLanczosWarm, 0} : std::vector<int>{0};
     const int wide = widest_block(b.n_max);
     std::vector<int> blocks{wide};
@@ -288,37 +286,15 @@ std::vector<Shape> block_shapes(const bdcu_ctx* ctx, const Bucket& b, int form) 
         if (x < wide) blocks.push_back(x);
     std::vector<Shape> out;
     for (int blk : blocks)
-        for (int d : d_opts)
-            for (int v : v_opts) {
-                if ((size_t)smem_layout(b.n_max, d, v, mixed).total * sizeof(double) > ctx->max_smem) continue;
-                Shape s;
-                s.block = blk;
-                s.v_cap = v;
-                s.d_in_smem = d;
-                out.push_back(s);
-            }
+        for (int v : v_opts) {
+            if ((size_t)smem_layout(b.n_max, 0, v, mixed).total * sizeof(double) > ctx->max_smem) continue;
+            Shape s;
+            s.block = blk;
+            s.v_cap = v;
+            s.d_in_smem = 0;
+            out.push_back(s);
+        }
     return out;
-}
-
-// The heuristic's shape (when none is tuned): the widest block, with D in
-// shared memory unless keeping D in global memory lets more blocks share an
-// SM. D in global stays L2-resident: a D that fits shared memory is at most
-// ~195 KB, ~87 MB over three blocks on each of 148 SMs. Measured at
-// 4096 x N=50 (plain form): D in global with three blocks per SM runs 1.7x
-// the D-in-shared shape's one block per SM.
-Shape default_shape(const Bucket& b, int mixed, const std::vector<Shape>& shapes) {
-    const Shape& first = shapes.front();
-    if (mixed || !first.d_in_smem) return first;
-    for (const Shape& s : shapes) {
-        if (s.block != first.block || s.d_in_smem) continue;
-        int per_d = 0, per_g = 0;
-        const size_t sm_d = (size_t)smem_layout(b.n_max, 1, first.v_cap, 0).total * sizeof(double);
-        const size_t sm_g = (size_t)smem_layout(b.n_max, 0, s.v_cap, 0).total * sizeof(double);
-        if (occupancy_plain(first.block, sm_d, &per_d) != cudaSuccess) return first;
-        if (occupancy_plain(s.block, sm_g, &per_g) != cudaSuccess) return first;
-        return per_g > per_d ? s : first;
-    }
-    return first;
 }
 
 // Warps per chain of the pair kernel that hold a chain of `beads`, the
@@ -368,14 +344,15 @@ int fill_launch(bdcu_ctx* ctx, int form, Bucket& b, const Shape* s) {
         const int T = s->block / 32;
         b.block = s->block;
         b.v_cap = b.d_in_smem = 0;
-        b.w_pairs = b.need_d ? pair_cached(b.n_max, T, ctx->max_smem) : 0;
+        b.w_pairs = b.need_lz ? pair_cached(b.n_max, T, ctx->max_smem) : 0;
+        if (b.chol_beads > 0) b.w_pairs = std::max(b.w_pairs, (pair_factor_doubles(b.chol_beads) + 1) / 2);
         b.smem = (size_t)pair_layout(b.n_max, T, b.w_pairs).total * sizeof(double);
         if (b.smem > ctx->max_smem) return fail(ctx, BDCU_E_LIMIT, "chain too large for the shared-memory layout");
         e = occupancy_pair(T, b.smem, &per_sm);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "occupancy_pair");
         if (per_sm < 1) return fail(ctx, BDCU_E_LIMIT, "pair kernel shape cannot be resident");
         b.grid = std::max(1, std::min(b.count, per_sm * ctx->sm_count));
-        b.scratch_stride = b.need_d ? pair_scratch_doubles(b.n_max) : 1;
+        b.scratch_stride = b.need_lz ? pair_scratch_doubles(b.n_max) : 1;
         return BDCU_OK;
     }
     b.block = s->block;
@@ -387,7 +364,7 @@ int fill_launch(bdcu_ctx* ctx, int form, Bucket& b, const Shape* s) {
     if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
     if (per_sm < 1) return fail(ctx, BDCU_E_LIMIT, "block kernel shape cannot be resident");
     b.grid = std::max(1, std::min(b.count, per_sm * ctx->sm_count));
-    const ScratchLayout scl = scratch_layout(b.n_max, b.d_in_smem, b.v_cap, b.need_chol, mixed, b.need_d, b.need_lz);
+    const ScratchLayout scl = scratch_layout(b.n_max, 0, b.v_cap, b.need_chol, mixed, 0, b.need_lz);
     b.scratch_stride = std::max<int64_t>(scl.total, 1);
     return BDCU_OK;
 }
@@ -462,6 +439,7 @@ int build_plan(bdcu_ctx* ctx, int form) {
                 b.need_d = 1;
                 b.need_chol = 1;  // Cholesky method, or the Chebyshev fallback
                 if (ch.hi_method == BDCU_HI_CHEBYSHEV) b.need_lz = 1;
+                if (ch.hi_method == BDCU_HI_CHOLESKY) b.chol_beads = std::max(b.chol_beads, (int)ch.N);
             }
         }
         b.order_off = (int64_t)ctx->order_h.size();
@@ -480,7 +458,7 @@ int build_plan(bdcu_ctx* ctx, int form) {
         } else {
             const std::vector<Shape> shapes = block_shapes(ctx, b, form);
             if (shapes.empty()) return fail(ctx, BDCU_E_LIMIT, "chain too large for the shared-memory layout");
-            Shape pick = default_shape(b, mixed, shapes);
+            Shape pick = shapes.front();
             const Shape& t = ctx->tuned[mixed][id];
             if (t.block > 0) {
                 // the tuned shape, or the nearest one that still fits this bucket
@@ -554,7 +532,7 @@ int launch_bucket(bdcu_ctx* ctx, int form, const Bucket& b, const State& st, int
     a.d_in_smem = b.d_in_smem;
     a.v_cap = b.v_cap;
     a.need_chol = b.need_chol;
-    a.need_d = b.need_d;
+    a.need_d = 0;  // (no dense D)
     a.need_lz = b.need_lz;
     a.work_counter = ctx->work_d + b.id;
     a.order = ctx->order_d + b.order_off;

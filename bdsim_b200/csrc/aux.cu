@@ -6,6 +6,44 @@
 
 namespace bdcu {
 
+// Excluded-volume force on bead b from partners part, part + S, ...
+// (ExcludedVolume::force, src/excluded_volume.cpp:60-89): the force from j is
+// -fac (R_j - R_b). The Gaussian factor is formed without a branch; LJ and SDK
+// pairs beyond the outer cutoff are passed over on the squared distance.
+static __device__ __forceinline__ void ev_share(const DevChain& c, const double* arena, const double* R, int b, int part,
+                                                int S, double (&f)[3]) {
+    if (c.ev_type == BDCU_EV_NONE) return;
+    const int N = c.N, cd = c.cd > 1 ? c.cd : 1;
+    const double qx = R[3 * b], qy = R[3 * b + 1], qz = R[3 * b + 2];
+    if (c.ev_type == BDCU_EV_GAUSS) {
+        const double zs = c.zsbyds5, p5 = c.pt5bydssq;
+#pragma unroll 4
+        for (int j = part; j < N; j += S) {
+            const double dx = R[3 * j] - qx, dy = R[3 * j + 1] - qy, dz = R[3 * j + 2] - qz;
+            const double sq = fmax(fma(dz, dz, fma(dy, dy, dx * dx)), 1.0e-12);
+            const int dj = j > b ? j - b : b - j;
+            const double fac = (dj >= cd ? zs : 0.0) * exp(-(sq * p5));
+            f[0] = fma(-fac, dx, f[0]);
+            f[1] = fma(-fac, dy, f[1]);
+            f[2] = fma(-fac, dz, f[2]);
+        }
+        return;
+    }
+    const double cut = ev_outer_cutoff(c), cut2 = cut * cut * (1.0 + 1e-9);
+    const double* phi = (c.ev_type == BDCU_EV_SDK && c.phi_off >= 0) ? arena + c.phi_off : nullptr;
+    for (int j = part; j < N; j += S) {
+        const double dx = R[3 * j] - qx, dy = R[3 * j + 1] - qy, dz = R[3 * j + 2] - qz;
+        const double sq = fmax(fma(dz, dz, fma(dy, dy, dx * dx)), 1.0e-12);
+        const int dj = j > b ? j - b : b - j;
+        if (dj < cd || sq > cut2) continue;
+        const int mu = j < b ? j : b, nu = j < b ? b : j;
+        const double fac = ev_factor_short(c, sq, phi ? phi + (int64_t)mu * N + nu : nullptr);
+        f[0] = fma(-fac, dx, f[0]);
+        f[1] = fma(-fac, dy, f[1]);
+        f[2] = fma(-fac, dz, f[2]);
+    }
+}
+
 // One chain per block. `which` selects force components (BDCU_F_*); present
 // terms are combined as (spring + (EV + bending)) + external.
 __global__ void __launch_bounds__(256) forces_kernel(const RunArgs a, const double* __restrict__ Rg, double t,
@@ -53,9 +91,20 @@ __global__ void __launch_bounds__(256) forces_kernel(const RunArgs a, const doub
         }
         __syncthreads();
         double* gF = Fg + 3 * chs.bead_off;
-        for (int m = threadIdx.x; m < N; m += blockDim.x) {
+        // excluded volume: S adjacent lanes per bead, each a share of the
+        // partners, the shares added by shuffles (with one thread per bead a
+        // 50-bead chain kept 50 of a block's 128 threads busy)
+        int S = 1;
+        while (S < 32 && 2 * S * N <= (int)blockDim.x) S *= 2;
+        for (int m0 = 0; m0 < N; m0 += blockDim.x / S) {
+            const int m = m0 + threadIdx.x / S, part = threadIdx.x % S;
             double fe[3] = {0.0, 0.0, 0.0}, fb[3] = {0.0, 0.0, 0.0}, fx[3] = {0.0, 0.0, 0.0};
-            if (which & BDCU_F_EV) B.ev_on_bead(R, m, fe);
+            if (which & BDCU_F_EV) {
+                if (m < N) ev_share(chs, a.arena, R, m, part, S, fe);
+                for (int o = 1; o < S; o <<= 1)
+                    for (int d = 0; d < 3; ++d) fe[d] += __shfl_xor_sync(0xffffffffu, fe[d], o);
+            }
+            if (m >= N || part != 0) continue;
             if (bend) bending_on_bead(chs, m, u, cs, len, fb);
             if ((which & BDCU_F_EXTERNAL) && chs.ext_n > 0) external_on_bead(chs, a.arena, m, t, fx);
             for (int d = 0; d < 3; ++d) {

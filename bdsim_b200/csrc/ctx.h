@@ -18,7 +18,7 @@ namespace bdcu {
 // Buckets of a launch plan. Buckets 0..3 hold the chains of N <= 64, 128, 256
 // and 512 beads that do not use the Cholesky method: the team kernel in the
 // FP32-mixed form, the pair kernel (one chain per block, reported as block
-// buckets 4..7) in the plain form. Buckets 4..7 run one chain per block on the
+// buckets 4..7) in the plain form, which takes Cholesky chains of N <= 64 too. Buckets 4..7 run one chain per block on the
 // general block kernel and split the rest by bead count at 64, 128 and 256.
 constexpr int kMaxBuckets = 8;
 constexpr int kFirstBlockBucket = 4;
@@ -44,6 +44,7 @@ struct Bucket {
     int count = 0, min_beads = 0, max_beads = 0;
     int n_max = 0;  // 3 * max_beads
     int need_chol = 0, need_d = 0, need_lz = 0;
+    int chol_beads = 0;  // largest chain of the Cholesky method
     int64_t order_off = 0;  // first entry of this bucket's work list in order_d
     int block = 0, grid = 0, v_cap = 0, d_in_smem = 0, tuned = 0;
     int64_t w_pairs = 0;  // pair and team kernels: cached pair weights (per block, per team)

@@ -447,4 +447,45 @@ __device__ __forceinline__ void rpy_weights(double hstar, double sq, double& om1
     }
 }
 
+// 1/sqrt(s) for s in [1e-30, 3e38]: the single-precision estimate y (relative
+// error below 2^-21) refined by one third-order step of the Newton-Halley
+// family, y (1 + e/2 + 3 e^2/8) with e = 1 - s y^2, whose error is O(e^3).
+__device__ __forceinline__ double rsqrt_refined(double s) {
+    const double y = (double)rsqrtf((float)s);
+    const double e = fma(-(s * y), y, 1.0);
+    return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+
+// RPY weights of a pair at squared separation sq (src/hydrodynamics.cpp:36-43)
+// with h* folded into the constants. (The two branches meet continuously at
+// r = 2 sqrt(pi) h*.)
+struct RpyConst {
+    double A1, A3, B3, c3, c7, far2;
+    __device__ void set(double h) {
+        const double rpi = 1.7724538509055160, tpi = 6.283185307179586, k = 0.75 * rpi;
+        A1 = k * h;
+        A3 = k * (tpi / 3.0) * h * h * h;
+        B3 = k * tpi * h * h * h;
+        c3 = 0.75 / rpi * 0.375 / h;
+        c7 = 0.09375 / rpi / h;
+        far2 = (2.0 * rpi * h) * (2.0 * rpi * h);
+    }
+    // Far pairs (all but neighbours along the chain and close contacts).
+    __device__ __forceinline__ void far_weights(double sq, double& om1, double& om2) const {
+        const double rho = rsqrt_refined(sq), t = rho * rho;
+        om1 = rho * fma(A3, t, A1);
+        om2 = (rho * t) * fma(-B3, t, A1);
+    }
+    // Any pair, and a bead with itself (omega1 = 1 along the diagonal block).
+    __device__ __forceinline__ void weights(double sq, bool self, double& om1, double& om2) const {
+        far_weights(sq, om1, om2);
+        if (!(sq >= far2)) {
+            sq = fmax(sq, 1.0e-12);
+            const double rho = rsqrt_refined(sq);
+            om1 = self ? 1.0 : fma(-c3, sq * rho, 1.0);
+            om2 = self ? 0.0 : c7 * rho;
+        }
+    }
+};
+
 }  // namespace bdcu

@@ -2,12 +2,12 @@
 // kernel: one chain per thread block, chains claimed from a device work queue,
 // chain state resident in shared memory for all steps of a call.
 //
-// FORM == BDCU_FORM_PLAIN_FP64: the reference algorithm in FP64. The dense RPY
-//   tensor D lives in shared memory (global scratch when 3N is too large);
-//   D.x is a row-sequential sum per thread, EV forces are accumulated per bead
-//   in the reference's pair order, Cholesky is right-looking with the
-//   reference's per-element subtraction order. Only block dot products
-//   (Lanczos, FD check) use a tree order.
+// FORM == BDCU_FORM_PLAIN_FP64: the reference algorithm in FP64. D.x is
+//   evaluated pair by pair from the positions, EV forces are accumulated per
+//   bead in the reference's pair order, Cholesky is right-looking (blocked from
+//   3N = 300, trailing updates on the FP64 tensor cores). It runs the chains the
+//   pair kernel does not take: the Cholesky method above N = 64, any chain above
+//   N = 512, and every chain of the static-scratch entry point.
 // FORM == BDCU_FORM_MIXED_FP32: D.x recomputed pairwise in FP32 from
 //   shared-memory bead coordinates (no stored D), FP32 excluded volume; FP64
 //   positions, connector solve, Lanczos bounds and Cholesky.
@@ -128,30 +128,6 @@ static __device__ double block_dot(const double* a, const double* b, int n, doub
     return red[0] + red[1];
 }
 
-// y_r = D x_r for K vectors in one read of D: one row per thread, each
-// product summed over j in order exactly as matvec does
-// (src/linalg.cpp:81-89), so every y_r equals its own single product bit for
-// bit. The plain form reads D (L2-resident) once for the step's K mutually
-// independent products instead of K times.
-template <int K>
-__device__ __forceinline__ void matvec_dense_k(const double* __restrict__ D, int ld, const double* const (&x)[K],
-                                               double* const (&y)[K], int n) {
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        double s[K];
-#pragma unroll
-        for (int r = 0; r < K; ++r) s[r] = 0.0;
-        const double* col = D + i;
-#pragma unroll 8
-        for (int j = 0; j < n; ++j) {
-            const double d = col[(int64_t)j * ld];
-#pragma unroll
-            for (int r = 0; r < K; ++r) s[r] += d * x[r][j];
-        }
-#pragma unroll
-        for (int r = 0; r < K; ++r) y[r][i] = s[r];
-    }
-}
-
 // Drop the L2 lines of [p, p + doubles) without writing them back: the dense
 // D (and a factor) are rebuilt every step, so after a step's last read the
 // data is dead. p must start a 128-byte line and the range must end at the
@@ -163,20 +139,6 @@ __device__ __forceinline__ void discard_l2(const double* p, int64_t doubles) {
     const char* base = reinterpret_cast<const char*>(p);
     for (int64_t l = threadIdx.x; l < lines; l += blockDim.x)
         asm volatile("discard.global.L2 [%0], 128;" ::"l"(base + 128 * l) : "memory");
-}
-
-// y = D x, one row per thread, summed over j in order (matvec,
-// src/linalg.cpp:81-89). D is exactly symmetric (rpy_diffusion_matrix writes
-// both halves from one value), so row i is read as column i for coalescing.
-__device__ __forceinline__ void matvec_dense(const double* __restrict__ D, int ld, const double* __restrict__ x,
-                                             double* __restrict__ y, int n) {
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        double s = 0.0;
-        const double* col = D + i;
-#pragma unroll 16  // (16 loads of D in flight per row: +4.5% on the plain form over 8; 32 was slower)
-        for (int j = 0; j < n; ++j) s += col[(int64_t)j * ld] * x[j];
-        y[i] = s;
-    }
 }
 
 // sturm_count (src/hydrodynamics.cpp:91-104)
@@ -280,8 +242,6 @@ struct Block {
     double* slot[kSlots];
     double* Vs;        // shared Lanczos basis (v_cap vectors)
     double* Vg;        // global Lanczos basis (kLanczosCold vectors)
-    double* D;         // plain: dense D (shared or global)
-    int ldd;
     double* Lt;        // transposed Cholesky factor, global scratch (leading dimension ldl)
     int ldl;           // chol_ld(n)
     double* stage;     // blocked Cholesky tile staging (vector slots kCholFirstSlot..)
@@ -309,14 +269,16 @@ struct Block {
         }
         count(C_DX, 1);
         if constexpr (!kMixed) {
-            matvec_dense(D, ldd, x, y, n);
+            const double* const xs[1] = {x};
+            double* const ys[1] = {y};
+            apply_D_pairs<1>(xs, ys);
         } else {
             apply_D_pairwise(x, y);
         }
     }
 
-    // K products against D at once (K = 1..4): the plain form reads D once,
-    // the mixed form runs its matrix-free products one after another. Caller
+    // K products against D at once (K = 1..4): the plain form evaluates the pair
+    // weights once, the mixed form runs its products one after another. Caller
     // syncs before and after, as for apply_D.
     template <int K>
     __device__ void apply_D_multi(const double* const (&x)[K], double* const (&y)[K]) {
@@ -328,7 +290,7 @@ struct Block {
         }
         if constexpr (!kMixed) {
             count(C_DX, K);
-            matvec_dense_k<K>(D, ldd, x, y, n);
+            apply_D_pairs<K>(x, y);
         } else {
 #pragma unroll
             for (int r = 0; r < K; ++r) {
@@ -347,6 +309,52 @@ struct Block {
                       apply_D_multi<3>(xs, ys); break; }
             default: { const double* const xs[4] = {x[0], x[1], x[2], x[3]};
                        double* const ys[4] = {y[0], y[1], y[2], y[3]}; apply_D_multi<4>(xs, ys); break; }
+        }
+    }
+
+    // Matrix-free FP64 D.x for K vectors: y_b = sum_j omega1 x_j + omega2 (d.x_j) d
+    // with d = R_j - R_b at the step's positions (slot 0), two adjacent lanes
+    // per bead up to N = 256 (the split depends on N alone, so that a result
+    // does not depend on the launch shape). Bound by the FP64 pipe: about 28
+    // operations per pair and 13 more per further vector. A dense D took 72
+    // bytes of HBM or L2 per pair and product (N = 500: 18 MB a chain).
+    template <int K>
+    __device__ void apply_D_pairs(const double* const (&x)[K], double* const (&y)[K]) {
+        RpyConst rpy;
+        rpy.set(ch.hstar);
+        const double* R = slot[0];
+        const int S = N <= 256 ? 2 : 1, per = blockDim.x / S;
+        for (int b0 = 0; b0 < N; b0 += per) {
+            const int b = b0 + threadIdx.x / S, part = threadIdx.x % S;
+            double acc[K][3];
+#pragma unroll
+            for (int r = 0; r < K; ++r)
+#pragma unroll
+                for (int d = 0; d < 3; ++d) acc[r][d] = 0.0;
+            if (b < N) {
+                const double q0 = R[3 * b], q1 = R[3 * b + 1], q2 = R[3 * b + 2];
+#pragma unroll 2
+                for (int j = part; j < N; j += S) {
+                    const double d0 = R[3 * j] - q0, d1 = R[3 * j + 1] - q1, d2 = R[3 * j + 2] - q2;
+                    double om1, om2;
+                    rpy.weights(fma(d2, d2, fma(d1, d1, d0 * d0)), j == b, om1, om2);
+#pragma unroll
+                    for (int r = 0; r < K; ++r) {
+                        const double x0 = x[r][3 * j], x1 = x[r][3 * j + 1], x2 = x[r][3 * j + 2];
+                        const double t = om2 * fma(d2, x2, fma(d1, x1, d0 * x0));
+                        acc[r][0] = fma(t, d0, fma(om1, x0, acc[r][0]));
+                        acc[r][1] = fma(t, d1, fma(om1, x1, acc[r][1]));
+                        acc[r][2] = fma(t, d2, fma(om1, x2, acc[r][2]));
+                    }
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < K; ++r)
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    if (S == 2) acc[r][d] += __shfl_xor_sync(0xffffffffu, acc[r][d], 1);
+                    if (b < N && part == 0) y[r][3 * b + d] = acc[r][d];
+                }
         }
     }
 
@@ -425,16 +433,13 @@ struct Block {
     // ---- Cholesky (cholesky_lower, src/linalg.cpp:91-107) ---------------
     // Right-looking on Lt = L^T (Lt[k*ldl + i] = L(i,k)). Element (i,j) receives
     // M(i,j) - L(i,0)L(j,0) - L(i,1)L(j,1) - ... in k order, then / L(j,j):
-    // the reference's rounding sequence. Returns false on a pivot <= 0.
-    // src: dense D at (Dp, ld) or, if src_in_lt, Lt already holds D's lower part.
+    // the reference's order (the blocked form's trailing products in the tensor
+    // cores' own). Returns false on a pivot <= 0.
+    // Lt holds D's lower part (build_rpy).
     // From 3N = kBlockedCholMin the factorisation is blocked (cholesky_blocked);
     // vector slots kCholFirstSlot.. must then be free (the callers' are).
-    __device__ bool cholesky(const double* Dp, int ld, bool src_in_lt) {
+    __device__ bool cholesky() {
         double* L = Lt;
-        if (!src_in_lt) {
-            for (int j = threadIdx.x >> 5; j < n; j += blockDim.x >> 5)
-                for (int i = j + (threadIdx.x & 31); i < n; i += 32) L[(int64_t)j * ldl + i] = Dp[(int64_t)i * ld + j];
-        }
         __syncthreads();
         const int nb = chol_panel_width();
         if (nb > 0) return cholesky_blocked(nb);
@@ -484,10 +489,8 @@ struct Block {
     //     C(i,j) -= sum_{k in [kb,ke)} L(i,k) L(j,k), tile by tile, with the
     //     tile's panel rows staged in shared memory.
     // Every element still receives its products in k order before its
-    // division, so the plain form keeps the reference's rounding sequence
-    // (trailing updates one rounded product and one rounded subtraction per
-    // k); the mixed form's trailing updates run on the FP64 tensor cores
-    // (mma.m8n8k4, products accumulated in the tensor core's own order).
+    // division; the trailing updates run on the FP64 tensor cores (mma.m8n8k4,
+    // products accumulated in the tensor core's own order).
     __device__ bool cholesky_blocked(int nb) {
         for (int kb = 0; kb < n; kb += nb) {
             const int ke = kb + nb < n ? kb + nb : n;
@@ -509,28 +512,21 @@ struct Block {
     __device__ void chol_update(int k0, int k1, int r0, int c0, int c1) {
         double* L = Lt;
         const int kk = k1 - k0, kk4 = (kk + 3) & ~3;  // staged rows k >= kk are zero
-        if constexpr (kMixed)
-            if ((int64_t)kStageBufs * kk4 * kCholTileStride + 8 <= stage_cap && (r0 & 7) == 0 && (c0 & 7) == 0) {
-                chol_update_bulk(k0, k1, r0, c0, c1);
-                return;
-            }
-        if constexpr (!kMixed)
-            if (blockDim.x == 512 && (int64_t)3 * kk4 * kCholTile <= stage_cap) {
-                chol_update_pairs(k0, k1, r0, c0, c1);
-                return;
-            }
+        if ((int64_t)kStageBufs * kk4 * kCholTileStride + 8 <= stage_cap && (r0 & 7) == 0 && (c0 & 7) == 0) {
+            chol_update_bulk(k0, k1, r0, c0, c1);
+            return;
+        }
         double* As = stage;                                   // As[k*TS + r] = L(i0 + r, k0 + k)
         double* Bs = stage + (int64_t)kk4 * kCholTileStride;  // Bs[k*TS + c] = L(j0 + c, k0 + k)
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
         const int nti = (n - r0 + kCholTile - 1) / kCholTile, ntj = (c1 - c0 + kCholTile - 1) / kCholTile;
         // Staging loads are issued kStageBatch at a time before their shared
         // stores, so one memory latency covers a batch instead of each element.
-        // The tiles go row by row; the mixed form stages As once per tile-row
-        // (a_i0) and Bs only when its column block changes (b_j0), and a
-        // diagonal tile (i0 == j0) multiplies As by itself (its B rows beyond c1
-        // differ from the zeros Bs would hold, but they only reach C columns >=
-        // c1, which are not stored). The plain form restages both for every
-        // tile: the reuse measured 2.5% slower there (5% faster in the mixed form).
+        // The tiles go row by row; As is staged once per tile-row (a_i0) and Bs
+        // only when its column block changes (b_j0), and a diagonal tile (i0 ==
+        // j0) multiplies As by itself (its B rows beyond c1 differ from the zeros
+        // Bs would hold, but they only reach C columns >= c1, which are not
+        // stored).
         constexpr int kStageBatch = 8;
         const int tot = kk4 * kCholTile, nt = nti * ntj;
         auto next_tile = [&](int t) {  // first tile >= t not wholly above the diagonal
@@ -540,7 +536,7 @@ struct Block {
         int a_i0 = -1, b_j0 = -1;
         for (int t = next_tile(0); t < nt; t = next_tile(t + 1)) {
             const int i0 = r0 + (t / ntj) * kCholTile, j0 = c0 + (t % ntj) * kCholTile;
-            const bool diag = kMixed && i0 == j0, stA = !kMixed || i0 != a_i0, stB = !kMixed || (!diag && j0 != b_j0);
+            const bool diag = i0 == j0, stA = i0 != a_i0, stB = !diag && j0 != b_j0;
             a_i0 = i0;
             if (stB) b_j0 = j0;
             if (stA || stB) {
@@ -568,17 +564,16 @@ struct Block {
                 const int tn = next_tile(t + 1);
                 if (tn < nt) {
                     const int i1 = r0 + (tn / ntj) * kCholTile, j1 = c0 + (tn % ntj) * kCholTile;
-                    prefetch_tile(k0, kk, i1, j1, c1, !kMixed || i1 != i0, !kMixed || (i1 != j1 && j1 != b_j0));
+                    prefetch_tile(k0, kk, i1, j1, c1, i1 != i0, i1 != j1 && j1 != b_j0);
                 }
             }
             const double* Bt = diag ? As : Bs;
-            if constexpr (!kMixed) chol_tile_simt<kCholTileStride>(As, Bt, i0, j0, c1, kk, threadIdx.x, blockDim.x);
-            else chol_tile_dmma(As, Bt, i0, j0, c1, kk4, warp, lane, nwarps);
+            chol_tile_dmma(As, Bt, i0, j0, c1, kk4, warp, lane, nwarps);
             __syncthreads();
         }
     }
 
-    // chol_update for the mixed form with its panel rows staged by bulk
+    // chol_update with its panel rows staged by bulk
     // copies (cp.async.bulk, global -> shared, completion on an mbarrier)
     // issued one tile ahead. The panel rows L(x + r, k0 + k), r < kCholTile,
     // k < kk, of the tile row or tile column starting at row x are the same
@@ -774,67 +769,6 @@ struct Block {
         __syncthreads();
     }
 
-    // chol_update for the plain form with 512 threads: a 4x4 micro-tile per
-    // thread covers 256 threads of a tile, so each pass takes two tiles of a
-    // tile-row, (i0, j0) for threads 0-255 and (i0, j0 + 64) for 256-511,
-    // against one staged As and two Bs. The three buffers are unpadded
-    // (every access to them runs along a row). Each element still receives
-    // its products in k order: the arithmetic is the single-tile path's.
-    __device__ void chol_update_pairs(int k0, int k1, int r0, int c0, int c1) {
-        const double* L = Lt;
-        constexpr int TS = kCholTile;
-        const int kk = k1 - k0, kk4 = (kk + 3) & ~3, tot = kk4 * kCholTile;
-        double* As = stage;
-        double* B0 = stage + (int64_t)kk4 * TS;
-        double* B1 = B0 + (int64_t)kk4 * TS;
-        const int nti = (n - r0 + kCholTile - 1) / kCholTile, ntj = (c1 - c0 + kCholTile - 1) / kCholTile;
-        const int half = threadIdx.x >> 8, hl = threadIdx.x & 255;
-        constexpr int kB = 4;  // staged elements per thread per array between loads and stores
-        for (int ti = 0; ti < nti; ++ti) {
-            const int i0 = r0 + ti * kCholTile;
-            // tiles (ti, tj) with tj < tjn reach the diagonal (r0 == c0 in both callers, so i0 >= c0)
-            const int tjn = min(ntj, (i0 + kCholTile - 1 - c0) / kCholTile + 1);
-            for (int tj = 0; tj < tjn; tj += 2) {
-                const int j0 = c0 + tj * kCholTile, j1 = j0 + kCholTile;
-                const bool two = tj + 1 < tjn;
-                for (int e0 = threadIdx.x; e0 < tot; e0 += kB * blockDim.x) {
-                    double va[kB], v0[kB], v1[kB];
-#pragma unroll
-                    for (int u = 0; u < kB; ++u) {
-                        const int e = e0 + u * blockDim.x, k = e / kCholTile, r = e % kCholTile;
-                        const bool kin = e < tot && k < kk;
-                        const double* col = L + (int64_t)(k0 + k) * ldl;
-                        va[u] = (kin && i0 + r < n) ? col[i0 + r] : 0.0;
-                        v0[u] = (kin && j0 + r < c1) ? col[j0 + r] : 0.0;
-                        v1[u] = (two && kin && j1 + r < c1) ? col[j1 + r] : 0.0;
-                    }
-#pragma unroll
-                    for (int u = 0; u < kB; ++u) {
-                        const int e = e0 + u * blockDim.x, k = e / kCholTile, r = e % kCholTile;
-                        if (e < tot) {
-                            As[k * TS + r] = va[u];
-                            B0[k * TS + r] = v0[u];
-                            if (two) B1[k * TS + r] = v1[u];
-                        }
-                    }
-                }
-                __syncthreads();
-                {  // the next pass's panel rows and C tiles into L2 while this one is multiplied
-                    int ti1 = ti, tj1 = tj + 2;
-                    if (tj1 >= tjn) ti1 = ti + 1, tj1 = 0;
-                    if (ti1 < nti) {
-                        const int i1 = r0 + ti1 * kCholTile, n1 = min(ntj, (i1 + kCholTile - 1 - c0) / kCholTile + 1);
-                        prefetch_tile(k0, kk, i1, c0 + tj1 * kCholTile, c1, true, true);
-                        if (tj1 + 1 < n1) prefetch_tile(k0, kk, i1, c0 + (tj1 + 1) * kCholTile, c1, false, true);
-                    }
-                }
-                if (half == 0) chol_tile_simt<TS>(As, B0, i0, j0, c1, kk, hl, 256);
-                else if (two) chol_tile_simt<TS>(As, B1, i0, j1, c1, kk, hl, 256);
-                __syncthreads();
-            }
-        }
-    }
-
     // L2 prefetch hints for the tile at (i0, j0) of chol_update: its staged
     // panel segments L(i0.., k0 + k) (if wantA) and L(j0.., k0 + k) (if
     // wantB), k < kk, and its C columns L(i0.., j), j in [j0, min(j0 +
@@ -910,48 +844,6 @@ struct Block {
         return true;
     }
 
-    // Trailing-update tile, FP64 CUDA cores: 4x4 elements per thread, each
-    // element c = c - a_k * b_k for k = 0, 1, ... (no contraction: the plain
-    // form is compiled without FMA).
-    // Threads take micro-tiles first, first + step, ...; As / Bs rows are TS
-    // doubles apart.
-    template <int TS>
-    __device__ void chol_tile_simt(const double* As, const double* Bs, int i0, int j0, int jend, int kk, int first,
-                                   int step) {
-        double* L = Lt;
-        constexpr int Q = kCholTile / 4;
-        for (int mtl = first; mtl < Q * Q; mtl += step) {
-            const int r0 = (mtl % Q) * 4, c0 = (mtl / Q) * 4;
-            if (i0 + r0 + 3 < j0 + c0) continue;  // all above the diagonal
-            double c[4][4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    const int i = i0 + r0 + u, j = j0 + c0 + v;
-                    c[u][v] = (i < n && j < jend && i >= j) ? L[(int64_t)j * ldl + i] : 0.0;
-                }
-            for (int k = 0; k < kk; ++k) {
-                const double2 a01 = *reinterpret_cast<const double2*>(As + k * TS + r0);
-                const double2 a23 = *reinterpret_cast<const double2*>(As + k * TS + r0 + 2);
-                const double2 b01 = *reinterpret_cast<const double2*>(Bs + k * TS + c0);
-                const double2 b23 = *reinterpret_cast<const double2*>(Bs + k * TS + c0 + 2);
-                const double av[4] = {a01.x, a01.y, a23.x, a23.y}, bv[4] = {b01.x, b01.y, b23.x, b23.y};
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-#pragma unroll
-                    for (int v = 0; v < 4; ++v) c[u][v] = c[u][v] - av[u] * bv[v];
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    const int i = i0 + r0 + u, j = j0 + c0 + v;
-                    if (i < n && j < jend && i >= j) L[(int64_t)j * ldl + i] = c[u][v];
-                }
-        }
-    }
-
     // Trailing-update tile on the FP64 tensor cores. The 64x64 tile is 8x8
     // blocks of 8x8, grouped in 16 strips of one block-row by four
     // block-columns (strip s: rows 8 (s % 8), columns 32 (s / 8) + 8u, u < 4);
@@ -995,7 +887,7 @@ struct Block {
     // Strip s of the tile at (i0, j0): C (loaded into c) -= A B over kk4 staged
     // k rows, stored back. kDmmaChains accumulation chains per fragment (k
     // steps rotate over c and cx, summed at the end) cut the dependent-DMMA
-    // wait; the mixed form's tolerance admits the reassociation.
+    // wait (a reassociation: rounding only).
     template <int kDmmaChains>
     __device__ void dmma_strip(int s, double (&c)[4][2], const double* As, const double* Bs, int i0, int j0, int jend,
                                int kk4, int lane) {
@@ -1477,13 +1369,6 @@ __global__ void __launch_bounds__(512, 1) integrate_kernel(const RunArgs a) {
         B.n = n;
         B.ldl = chol_ld(n);
         B.hi = ch.hstar > 0.0;
-        if constexpr (!kMixed) {
-            B.D = a.d_in_smem ? (sm + lay.D) : (scr + scl.D);
-            B.ldd = a.d_in_smem ? n : a.n_max;
-        } else {
-            B.D = nullptr;
-            B.ldd = 0;
-        }
         double* R = B.slot[0];
         double* Fs = B.slot[1];
         double* Fe = B.slot[2];
@@ -1572,13 +1457,9 @@ __global__ void __launch_bounds__(512, 1) integrate_kernel(const RunArgs a) {
                 ix = (int32_t)ux;
             }
             if (B.hi) {
-                if constexpr (!kMixed) {
-                    B.build_rpy(R, B.D, B.ldd);
-                } else {
-                    if (ch.hi_method == BDCU_HI_CHOLESKY) {
-                        // dense FP64 D straight into the factor's storage (lower part)
-                        B.build_rpy(R, B.Lt, B.ldl);
-                    }
+                if (ch.hi_method == BDCU_HI_CHOLESKY) {
+                    // dense FP64 D straight into the factor's storage (lower part)
+                    B.build_rpy(R, B.Lt, B.ldl);
                 }
             }
             __syncthreads();
@@ -1592,10 +1473,7 @@ __global__ void __launch_bounds__(512, 1) integrate_kernel(const RunArgs a) {
                 for (int i = tid; i < n; i += blockDim.x) dW[i] = sqrt_dt * X0[i];
             } else if (ch.hi_method == BDCU_HI_CHOLESKY) {
                 chol_used = true;
-                bool ok;
-                if constexpr (!kMixed) ok = B.cholesky(B.D, B.ldd, false);
-                else ok = B.cholesky(nullptr, 0, true);
-                if (!ok) {
+                if (!B.cholesky()) {
                     if (tid == 0) ctl.status |= ctl.brk == 2 ? BDCU_ST_TIMEOUT : BDCU_ST_NOT_PD;
                     __syncthreads();
                     break;
@@ -1621,14 +1499,8 @@ __global__ void __launch_bounds__(512, 1) integrate_kernel(const RunArgs a) {
                         ctl.cnt[C_FALLBACK] += 1;
                     }
                     chol_used = true;
-                    bool ok;
-                    if constexpr (!kMixed) {
-                        ok = B.cholesky(B.D, B.ldd, false);
-                    } else {
-                        B.build_rpy(R, B.Lt, B.ldl);
-                        ok = B.cholesky(nullptr, 0, true);
-                    }
-                    if (!ok) {
+                    B.build_rpy(R, B.Lt, B.ldl);
+                    if (!B.cholesky()) {
                         if (tid == 0) ctl.status |= ctl.brk == 2 ? BDCU_ST_TIMEOUT : BDCU_ST_NOT_PD;
                         __syncthreads();
                         break;
@@ -1802,9 +1674,8 @@ __global__ void __launch_bounds__(512, 1) integrate_kernel(const RunArgs a) {
             t += dt;
             __syncthreads();
             if constexpr (!kMixed) {
-                // D (and a factor made this step) are dead until the next
-                // step rebuilds them: drop their L2 lines unwritten
-                if (B.hi && !a.d_in_smem) discard_l2(B.D, (int64_t)n * B.ldd);
+                // a factor made this step is dead until the next step rebuilds
+                // it: drop its L2 lines unwritten
                 if (chol_used) discard_l2(B.Lt, (int64_t)n * B.ldl);
                 __syncthreads();
             }

@@ -23,38 +23,6 @@
 
 namespace bdcu {
 
-// RPY weights of a pair at squared separation sq (src/hydrodynamics.cpp:36-43)
-// with h* folded into the constants. (The two branches meet continuously at
-// r = 2 sqrt(pi) h*.)
-struct RpyConst {
-    double A1, A3, B3, c3, c7, far2;
-    __device__ void set(double h) {
-        const double rpi = 1.7724538509055160, tpi = 6.283185307179586, k = 0.75 * rpi;
-        A1 = k * h;
-        A3 = k * (tpi / 3.0) * h * h * h;
-        B3 = k * tpi * h * h * h;
-        c3 = 0.75 / rpi * 0.375 / h;
-        c7 = 0.09375 / rpi / h;
-        far2 = (2.0 * rpi * h) * (2.0 * rpi * h);
-    }
-    // Far pairs (all but neighbours along the chain and close contacts).
-    __device__ __forceinline__ void far_weights(double sq, double& om1, double& om2) const {
-        const double rho = rsqrt_refined(sq), t = rho * rho;
-        om1 = rho * fma(A3, t, A1);
-        om2 = (rho * t) * fma(-B3, t, A1);
-    }
-    // Any pair, and a bead with itself (omega1 = 1 along the diagonal block).
-    __device__ __forceinline__ void weights(double sq, bool self, double& om1, double& om2) const {
-        far_weights(sq, om1, om2);
-        if (!(sq >= far2)) {
-            sq = fmax(sq, 1.0e-12);
-            const double rho = rsqrt_refined(sq);
-            om1 = self ? 1.0 : fma(-c3, sq * rho, 1.0);
-            om2 = self ? 0.0 : c7 * rho;
-        }
-    }
-};
-
 // Bracket of the target-th eigenvalue boundary by a whole warp: 31 Sturm
 // counts at evenly spaced points per round, a ballot keeps one of the 32
 // parts (five halvings of src/hydrodynamics.cpp:196-207 per round), until the
@@ -74,25 +42,6 @@ __device__ __forceinline__ void warp_multisect(const Count& count, int target, d
         hi = nhi;
         if (done) break;
     }
-}
-
-// Eigenvalues below x of a tridiagonal of up to kLanczosWarm entries in
-// registers (a; b2: squared off-diagonals): the signs of the leading principal
-// minors p_i = (a_i - x) p_{i-1} - b_{i-1}^2 p_{i-2}. |a_i - x| and b^2 lie
-// within [1e-20, (3N)^2] or are zero, so eight factors neither overflow nor
-// vanish.
-__device__ __forceinline__ int sturm_count8(const double (&a)[kLanczosWarm], const double (&b2)[kLanczosWarm], int k,
-                                            double x) {
-    double pm = 1.0, p = a[0] - x;
-    int count = p < 0.0;
-#pragma unroll
-    for (int i = 1; i < kLanczosWarm; ++i) {
-        const double pn = fma(a[i] - x, p, -(b2[i - 1] * pm));
-        count += i < k && ((pn < 0.0) != (p < 0.0));
-        pm = p;
-        p = pn;
-    }
-    return count;
 }
 
 // Beads are staged in pairs, components outermost within a pair: component d of
@@ -140,6 +89,10 @@ static __device__ __noinline__ bool pair_cholesky(double* L, const double* ps, i
     __syncthreads();
     return true;
 }
+
+// Doubles of a chain's factor in shared memory: its 3x3 blocks of the lower
+// triangle, column by column.
+__device__ __forceinline__ int factor_block(int N, int I, int J) { return 9 * (J * N - J * (J - 1) / 2 + (I - J)); }
 
 template <int T>
 struct PairChain {
@@ -544,6 +497,103 @@ struct PairChain {
         }
     }
 
+    // ---- Cholesky method (brownian_step, src/mobility.cpp:58-88) for chains of
+    // up to kPairCholMaxN beads: D at the staged positions, factored in shared
+    // memory (F, in the weights' place) one bead at a time: the 3x3 diagonal
+    // block by every thread for itself, the rows below it one per thread, then
+    // the trailing blocks, one warp per block column (two barriers per bead;
+    // the block kernel takes three per matrix column and one thread's work
+    // between two of them). Each element receives its products in k order
+    // before its division, as in the reference. y = L x. False if not positive
+    // definite.
+    __device__ __forceinline__ bool cholesky_noise(const double (&x0)[3], double (&out)[3]) {
+        double* F = reinterpret_cast<double*>(Wt);
+        for (int J = wi; J < N; J += T)
+            for (int I = J + wl; I < N; I += 32) {
+                double d[3], om1, om2;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) d[k] = ps[pair_at(I, k)] - ps[pair_at(J, k)];
+                rpy.weights(fma(d[2], d[2], fma(d[1], d[1], d[0] * d[0])), I == J, om1, om2);
+                double* f = F + factor_block(N, I, J);
+#pragma unroll
+                for (int i = 0; i < 3; ++i)
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) f[3 * i + j] = om2 * d[i] * d[j] + (i == j ? om1 : 0.0);
+            }
+        __syncthreads();
+#pragma unroll 1
+        for (int K = 0; K < N; ++K) {
+            double* f = F + factor_block(N, K, K);
+            double l[3][3], r[3];
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+                for (int j = 0; j <= i; ++j) l[i][j] = f[3 * i + j];
+            bool pd = true;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const double s = l[k][k];
+                pd = pd && s > 0.0;
+                r[k] = s > 1.0e-30 ? rsqrt_refined(s) : 1.0 / sqrt(s);
+                l[k][k] = s * r[k];
+#pragma unroll
+                for (int i = k + 1; i < 3; ++i) l[i][k] *= r[k];
+#pragma unroll
+                for (int i = k + 1; i < 3; ++i)
+#pragma unroll
+                    for (int j = k + 1; j <= i; ++j) l[i][j] = fma(-l[i][k], l[j][k], l[i][j]);
+            }
+            if (!pd) return false;  // (every thread found the same)
+            for (int I = K + 1 + tid; I < N; I += TT) {
+                double* g = F + factor_block(N, I, K);
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    const double a0 = g[3 * i] * r[0], a1 = fma(-a0, l[1][0], g[3 * i + 1]) * r[1],
+                                 a2 = fma(-a1, l[2][1], fma(-a0, l[2][0], g[3 * i + 2])) * r[2];
+                    g[3 * i] = a0;
+                    g[3 * i + 1] = a1;
+                    g[3 * i + 2] = a2;
+                }
+            }
+            __syncthreads();
+            if (tid == 0)
+#pragma unroll
+                for (int i = 0; i < 3; ++i)
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) f[3 * i + j] = j <= i ? l[i][j] : 0.0;
+            for (int J = K + 1 + wi; J < N; J += T)
+                for (int I = J + wl; I < N; I += 32) {
+                    const double *p = F + factor_block(N, I, K), *q = F + factor_block(N, J, K);
+                    double* c = F + factor_block(N, I, J);
+#pragma unroll
+                    for (int i = 0; i < 3; ++i)
+#pragma unroll
+                        for (int j = 0; j < 3; ++j)
+                            c[3 * i + j] = fma(-p[3 * i + 2], q[3 * j + 2],
+                                               fma(-p[3 * i + 1], q[3 * j + 1], fma(-p[3 * i], q[3 * j], c[3 * i + j])));
+                }
+            __syncthreads();
+        }
+        double* x = sb(0);
+        if (own)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) x[3 * b + d] = x0[d];
+        __syncthreads();
+#pragma unroll
+        for (int d = 0; d < 3; ++d) out[d] = 0.0;
+        if (on)  // the lanes of a bead share its row of blocks
+            for (int J = seg; J <= b; J += S) {
+                const double* f = F + factor_block(N, b, J);
+#pragma unroll
+                for (int d = 0; d < 3; ++d)
+                    out[d] += fma(f[3 * d + 2], x[3 * J + 2], fma(f[3 * d + 1], x[3 * J + 1], f[3 * d] * x[3 * J]));
+            }
+#pragma unroll
+        for (int d = 0; d < 3; ++d) out[d] = bead_sum(out[d]);
+        __syncthreads();  // (x and F are free again)
+        return true;
+    }
+
     // ---- Lanczos extreme eigenvalues (src/hydrodynamics.cpp:146-264) --------
 
     // The sums of c[0..7] over the warp's beads into out[u * T + warp]: halves of the
@@ -937,7 +987,9 @@ __global__ void __launch_bounds__(32 * T, pair_min_blocks(T)) integrate_pair_ker
         C.hi = ch.hstar > 0.0;
         C.status = status0;
         C.np = (Ne / 2 - C.gl + 2 * C.S - 1) / (2 * C.S);
-        C.nc = (int)min((int64_t)C.np, a.w_pairs / (4 * C.S * Ne));
+        // (the Cholesky method keeps its factor in the weights' place: three
+        // products a step do not repay a table)
+        C.nc = ch.hi_method == BDCU_HI_CHOLESKY ? 0 : (int)min((int64_t)C.np, a.w_pairs / (4 * C.S * Ne));
         C.xpar = 0;
         if (C.hi) C.rpy.set(ch.hstar);
         for (int k = 0; k < 8; ++k) C.cnt[k] = 0;
@@ -960,7 +1012,7 @@ __global__ void __launch_bounds__(32 * T, pair_min_blocks(T)) integrate_pair_ker
         const double sqrt_dt = sqrt(dt), inv_n = 1.0 / N;
         double v0[3];  // the Lanczos start vector, kept from step to step
         bool used_cache = false;
-        if (C.hi) {
+        if (C.hi && ch.hi_method == BDCU_HI_CHEBYSHEV) {
             if (own)
                 for (int d = 0; d < 3; ++d) C.seed[3 * b + d] = a.seed_table[3 * b + d] / ch.seed_norm;
             __syncwarp();  // (the lanes of a bead read it back)
@@ -1000,6 +1052,17 @@ __global__ void __launch_bounds__(32 * T, pair_min_blocks(T)) integrate_pair_ker
                     dW[d] = sqrt_dt * X0[d];
                     DF[d] = A[d];
                 }
+            } else if (ch.hi_method == BDCU_HI_CHOLESKY) {
+                double bx[3];
+                if (!C.cholesky_noise(X0, bx)) {
+                    C.status |= BDCU_ST_NOT_PD;
+                    break;
+                }
+#pragma unroll
+                for (int d = 0; d < 3; ++d) dW[d] = sqrt_dt * bx[d];
+                C.apply1(A, DF);
+                C.cnt[C_DX] += 1;  // (D (Fs + Fe) and, by linearity, the reference's D Fs)
+                __syncthreads();
             } else {
                 C.build_weights();
                 double DX0[3], bx[3], lmin, lmax;

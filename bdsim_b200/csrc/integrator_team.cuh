@@ -97,25 +97,21 @@ static __device__ void halfwarp_bisect(const double* al, const double* bb, int k
     }
 }
 
-// Sturm count below x for a tridiagonal of k <= kLanczosWarm entries held in
-// registers (a: diagonal, b: off-diagonal), the divide-free recurrence of
-// sturm_count_products fully unrolled.
-__device__ __forceinline__ int sturm_count_reg(const double (&a)[kLanczosWarm], const double (&b)[kLanczosWarm], int k,
-                                               double x) {
+// Eigenvalues below x of a tridiagonal of up to kLanczosWarm entries in
+// registers (a; b2: squared off-diagonals): the signs of the leading principal
+// minors p_i = (a_i - x) p_{i-1} - b_{i-1}^2 p_{i-2}. |a_i - x| and b^2 lie
+// within [1e-20, (3N)^2] or are zero, so eight factors neither overflow nor
+// vanish.
+__device__ __forceinline__ int sturm_count8(const double (&a)[kLanczosWarm], const double (&b2)[kLanczosWarm], int k,
+                                            double x) {
     double pm = 1.0, p = a[0] - x;
-    int count = (p < 0.0) ? 1 : 0;
+    int count = p < 0.0;
 #pragma unroll
     for (int i = 1; i < kLanczosWarm; ++i) {
-        if (i < k) {
-            const double pn = (a[i] - x) * p - (b[i - 1] * b[i - 1]) * pm;
-            count += ((pn < 0.0) != (p < 0.0)) ? 1 : 0;
-            pm = p;
-            p = pn;
-            if (fabs(p) > 1e150) {
-                p *= 1e-150;
-                pm *= 1e-150;
-            }
-        }
+        const double pn = fma(a[i] - x, p, -(b2[i - 1] * pm));
+        count += i < k && ((pn < 0.0) != (p < 0.0));
+        pm = p;
+        p = pn;
     }
     return count;
 }
@@ -125,13 +121,13 @@ __device__ __forceinline__ int sturm_count_reg(const double (&a)[kLanczosWarm], 
 // ballot finds the sixteenth that holds the boundary (4 bits per round), the
 // iteration of src/hydrodynamics.cpp:196-207 in place of its halvings. Every
 // lane of the half warp ends with the same lo, hi.
-static __device__ void halfwarp_multisect(const double (&a)[kLanczosWarm], const double (&b)[kLanczosWarm], int k,
-                                          int target, double& lo, double& hi) {
+__device__ __forceinline__ void halfwarp_multisect(const double (&a)[kLanczosWarm], const double (&b2)[kLanczosWarm],
+                                                   int k, int target, double& lo, double& hi) {
     const int h = threadIdx.x & 15;
     const int shift = threadIdx.x & 16;
     for (int it = 0; it < 25; ++it) {
         const double w = hi - lo;
-        const bool ge = h < 15 && sturm_count_reg(a, b, k, lo + w * ((double)(h + 1) * 0.0625)) >= target;
+        const bool ge = h < 15 && sturm_count8(a, b2, k, lo + w * ((double)(h + 1) * 0.0625)) >= target;
         const unsigned bal = (__ballot_sync(kFull, ge) >> shift) & 0xffffu;
         const int f = bal ? __ffs(bal) - 1 : 15;
         const double nlo = f == 0 ? lo : lo + w * ((double)f * 0.0625);
@@ -160,20 +156,13 @@ __device__ __forceinline__ uint32_t xorshift_jump(const uint32_t* cols, uint32_t
     return y;
 }
 
-// 1/sqrt(s) for s in [1e-12, 3e38]: the single-precision estimate y (relative
-// error below 2^-21) refined by one third-order step of the Newton-Halley
-// family, y (1 + e/2 + 3 e^2/8) with e = 1 - s y^2, whose error is O(e^3).
-__device__ __forceinline__ double rsqrt_refined(double s) {
-    const double y = (double)rsqrtf((float)s);
-    const double e = fma(-(s * y), y, 1.0);
-    return fma(y * e, fma(e, 0.375, 0.5), y);
-}
-
 // 1/x for |x| in [1e-30, 1e30]: a single-precision seed refined by two
 // Newton-Raphson steps r <- r (2 - x r) (quadratic convergence: 2^-23 ->
 // 2^-46 -> below double rounding).
 __device__ __forceinline__ double rcp_newton(double x) {
-    double r = (double)__frcp_rn((float)x);
+    float f;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(f) : "f"((float)x));
+    double r = (double)f;
     r = r * (2.0 - x * r);
     r = r * (2.0 - x * r);
     return r;
@@ -288,7 +277,7 @@ struct TeamChain {
     int N, n;
     bool hi;
     float4* Wt;     // cached pair weights (omega1 of j, j+1, omega2 of j, j+1): row j/2, column bead
-    int jc;         // partner beads below jc have cached weights (even)
+    int jc;         // partner beads below jc have cached weights (a multiple of four)
     int par, xpar;  // parity of the reduction buffer and of the single products' input rows
     int32_t cnt[8];  // this call's counts for the chain (added to the 64-bit counters at the end)
     int status;
@@ -388,8 +377,8 @@ struct TeamChain {
     // from coordinates and inputs staged by component in shared memory, so
     // one 64-bit broadcast load brings (j, j+1) of a component. Each bead's
     // sum is kept as two interleaved partial sums (even and odd j), added at
-    // the end. An odd N is padded with one zero input (whose contribution
-    // om1 * 0 + om2 (d . 0) d is exactly zero).
+    // the end. N is padded to a multiple of four with zero inputs (whose
+    // contribution om1 * 0 + om2 (d . 0) d is exactly zero).
     // The pair weights of the first jc partner beads are computed once a step
     // (build_weights) and kept in shared memory, 8 bytes per pair: a product
     // then takes 13 packed operations per bead and two partners instead of about
@@ -417,7 +406,8 @@ struct TeamChain {
                 for (int r = 0; r < K; ++r)
 #pragma unroll
                     for (int d = 0; d < 3; ++d) xr[r][d][bead(q)] = x[r][q][d];
-        if ((N & 1) && tid < 3 * K) xr[tid / 3][tid % 3][N] = 0.f;
+        const int pad = -N & 3;  // zero inputs up to a multiple of four beads
+        if (tid < 3 * K * pad) xr[tid / (3 * pad)][tid / pad % 3][N + tid % pad] = 0.f;
         sync();
         bool one_slot = false;
         if constexpr (Q == 2) one_slot = __all_sync(kFull, !valid(1));
@@ -444,21 +434,35 @@ struct TeamChain {
         const int n2 = (N + 1) & ~1;
         int j = 0;
         const float4* w = Wt;
-#pragma unroll(K == 1 ? 2 : 1)
-        for (; j < jc; j += 2, w += N) {
-            float2 pj[3], xj[K][3];
+        // cached weights: four partner beads per step (the second pair of the
+        // last step may lie beyond N: its inputs are zero)
+#pragma unroll 1
+        for (; j < jc; j += 4, w += 2 * N) {
+            float4 pj[3], xj[K][3];
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
-                pj[d] = *reinterpret_cast<const float2*>(&S.ps[d][j]);
+                pj[d] = *reinterpret_cast<const float4*>(&S.ps[d][j]);
 #pragma unroll
-                for (int r = 0; r < K; ++r) xj[r][d] = *reinterpret_cast<const float2*>(&xr[r][d][j]);
+                for (int r = 0; r < K; ++r) xj[r][d] = *reinterpret_cast<const float4*>(&xr[r][d][j]);
             }
 #pragma unroll
             for (int q = 0; q < Q; ++q)
                 if (q < nq) {
-                    const float4 o = w[min(bead(q), N - 1)];
-                    products(q, __fadd2_rn(pj[0], nb[q][0]), __fadd2_rn(pj[1], nb[q][1]), __fadd2_rn(pj[2], nb[q][2]),
-                             make_float2(o.x, o.y), make_float2(o.z, o.w), xj);
+                    const int m = min(bead(q), N - 1);
+                    const float4 o[2] = {w[m], w[N + m]};
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        float2 p[3], x2[K][3];
+#pragma unroll
+                        for (int d = 0; d < 3; ++d) {
+                            p[d] = h ? make_float2(pj[d].z, pj[d].w) : make_float2(pj[d].x, pj[d].y);
+#pragma unroll
+                            for (int r = 0; r < K; ++r)
+                                x2[r][d] = h ? make_float2(xj[r][d].z, xj[r][d].w) : make_float2(xj[r][d].x, xj[r][d].y);
+                        }
+                        products(q, __fadd2_rn(p[0], nb[q][0]), __fadd2_rn(p[1], nb[q][1]), __fadd2_rn(p[2], nb[q][2]),
+                                 make_float2(o[h].x, o[h].y), make_float2(o[h].z, o[h].w), x2);
+                    }
                 }
         }
 #pragma unroll 1
@@ -616,7 +620,8 @@ struct TeamChain {
                 S.ps[1][bead(q)] = y;
                 S.ps[2][bead(q)] = z;
             }
-        if ((N & 1) && tid < 3) S.ps[tid][N] = 0.f;  // the odd-N pad bead (zero input in every pass)
+        const int pad = -N & 3;  // pad beads (zero input in every pass)
+        if (tid < 3 * pad) S.ps[tid / pad][N + tid % pad] = 0.f;
         sync();
     }
 
@@ -676,7 +681,7 @@ struct TeamChain {
 #pragma unroll
             for (int q = 0; q < Q; ++q) pm[q] = valid(q) ? S.pos[bead(q)] : make_float4(0.f, 0.f, 0.f, 0.f);
             const int cd = ch.cd;
-#pragma unroll 2
+#pragma unroll 4
             for (int j = 0; j < N; ++j) {
                 const float4 pj = S.pos[j];
 #pragma unroll
@@ -685,7 +690,7 @@ struct TeamChain {
                     const float dx = pj.x - pm[q].x, dy = pj.y - pm[q].y, dz = pj.z - pm[q].z;
                     const float sq = dx * dx + dy * dy + dz * dz;
                     const int dj = j > m ? j - m : m - j;
-                    const float fac = (dj >= cd && j != m) ? zs * __expf(-sq * p5) : 0.f;
+                    const float fac = ((dj >= cd && j != m) ? zs : 0.f) * __expf(-sq * p5);  // (no branch)
                     fev[q][0] -= fac * dx;
                     fev[q][1] -= fac * dy;
                     fev[q][2] -= fac * dz;
@@ -950,11 +955,12 @@ struct TeamChain {
             // warm-sized tridiagonal in registers: Gershgorin bracket, then
             // lanes 0-15 find the smallest eigenvalue and its Ritz vector,
             // lanes 16-31 the largest
-            double ar[kLanczosWarm], br[kLanczosWarm];
+            double ar[kLanczosWarm], br[kLanczosWarm], b2[kLanczosWarm];
 #pragma unroll
             for (int i = 0; i < kLanczosWarm; ++i) {
                 ar[i] = i < k ? S.alpha[i] : 0.0;
                 br[i] = i < k - 1 ? S.beta[i] : 0.0;
+                b2[i] = br[i] * br[i];
             }
             double lo = ar[0], hi2 = ar[0];
 #pragma unroll
@@ -965,7 +971,7 @@ struct TeamChain {
                     hi2 = dmax_(hi2, ar[i] + rad);
                 }
             }
-            halfwarp_multisect(ar, br, k, wl < 16 ? 1 : k, lo, hi2);
+            halfwarp_multisect(ar, b2, k, wl < 16 ? 1 : k, lo, hi2);
             const double r = 0.5 * (lo + hi2);
             double y[kLanczosWarm];
             tridiag_vec_reg<1>(ar, br, k, r, y);
@@ -1285,7 +1291,7 @@ __global__ void __launch_bounds__(TeamCfg<T, Q>::kCtaThreads, TeamCfg<T, Q>::kMi
         W.team = team;
         W.N = ch.N;
         W.n = 3 * ch.N;
-        W.jc = 2 * (int)min((int64_t)(ch.N + 1) / 2, a.w_pairs / ch.N);
+        W.jc = 4 * (int)min((int64_t)(ch.N + 3) / 4, a.w_pairs / (2 * ch.N));
         W.hi = ch.hstar > 0.0;
         W.status = status;
         for (int k = 0; k < 8; ++k) W.cnt[k] = 0;

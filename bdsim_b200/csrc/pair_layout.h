@@ -1,9 +1,8 @@
 // pair_layout.h -- sizes of the pair kernel's shared and global scratch
 // (integrator_pair.cuh), shared by the host launch code and the kernel.
 //
-// The pair kernel is the FP64 plain form for chains of up to 512 beads that do
-// not use the Cholesky method: one chain per thread block of T warps, S lanes
-// per bead.
+// The pair kernel is the FP64 plain form for chains of up to 512 beads (64 with
+// the Cholesky method): one chain per thread block of T warps, S lanes per bead.
 #pragma once
 
 #include "integrator.cuh"
@@ -11,6 +10,10 @@
 namespace bdcu {
 
 constexpr int kPairMaxN = 512;
+// Cholesky-method chains up to this size factor D in shared memory (150 KB at 64
+// beads); larger ones run on the block kernel.
+constexpr int kPairCholMaxN = 64;
+__host__ __device__ inline int64_t pair_factor_doubles(int N) { return 9 * (int64_t)N * (N + 1) / 2; }
 
 // Blocks per SM a shape's registers and shared memory are sized for. 12 to 16
 // warps per SM: 168 registers per thread at T = 4, 128 at T = 8 and 16.

@@ -17,7 +17,9 @@ namespace bdcu {
 inline int bucket_of(const DevChain& c, int form, bool pair = true) {
     const bool chol = c.hstar > 0.0 && c.hi_method == BDCU_HI_CHOLESKY;
     static_assert(kPairMaxN == kTeamMaxN, "team and pair buckets share their bead ranges");
-    if ((form == BDCU_FORM_MIXED_FP32 || pair) && !chol && c.N <= kTeamMaxN) {
+    const bool fits = form == BDCU_FORM_MIXED_FP32 ? !chol && c.N <= kTeamMaxN
+                                                   : pair && c.N <= (chol ? kPairCholMaxN : kPairMaxN);
+    if (fits) {
         const int T = team_warps_for(c.N);
         return T == 1 ? 0 : T == 2 ? 1 : T == 4 ? 2 : 3;
     }

@@ -81,7 +81,7 @@ template <int T, int Q>
 inline int64_t team_cached(int n_max, size_t max_smem) {
     const int64_t share = ((int64_t)max_smem + 1024) / TeamCfg<T, Q>::kMinBlocks - 1024;
     const int64_t room = (share / TeamCfg<T, Q>::kTeamsPerCta - team_weight_offset<T, Q>(n_max)) / 16;
-    const int64_t N = n_max / 3, all = (N + 1) / 2 * N;
+    const int64_t N = n_max / 3, all = (N + 3) / 4 * 2 * N;
     return room <= 0 ? 0 : room < all ? room : all;
 }
 
