@@ -326,7 +326,7 @@ int fill_launch(bdcu_ctx* ctx, int form, Bucket& b, const Shape* s) {
         }
         const int T = b.team_warps, Q = b.team_q;
         if (!team_shape_fits(T, Q, b.max_beads)) return fail(ctx, BDCU_E_ARG, "team shape does not hold the bucket");
-        b.w_pairs = b.need_d ? team_weights(T, Q, b.n_max, ctx->max_smem) : 0;
+        b.w_pairs = b.need_d ? team_weights(T, Q, b.n_max, b.count, ctx->sm_count, ctx->max_smem) : 0;
         b.smem = (size_t)team_smem(T, Q, b.n_max, b.w_pairs);
         if (b.smem > ctx->max_smem) return fail(ctx, BDCU_E_LIMIT, "team kernel shared memory exceeds the device limit");
         e = occupancy_mixed_team(T, Q, b.smem, &per_sm);
@@ -344,12 +344,17 @@ int fill_launch(bdcu_ctx* ctx, int form, Bucket& b, const Shape* s) {
         const int T = s->block / 32;
         b.block = s->block;
         b.v_cap = b.d_in_smem = 0;
-        b.w_pairs = b.need_lz ? pair_cached(b.n_max, T, ctx->max_smem) : 0;
+        b.w_pairs = b.need_lz ? pair_cached(b.n_max, T, b.count, ctx->sm_count, ctx->max_smem) : 0;
         if (b.chol_beads > 0) b.w_pairs = std::max(b.w_pairs, (pair_factor_doubles(b.chol_beads) + 1) / 2);
         b.smem = (size_t)pair_layout(b.n_max, T, b.w_pairs).total * sizeof(double);
         if (b.smem > ctx->max_smem) return fail(ctx, BDCU_E_LIMIT, "chain too large for the shared-memory layout");
-        e = occupancy_pair(T, b.smem, &per_sm);
-        if (e != cudaSuccess) return cuda_fail(ctx, e, "occupancy_pair");
+        auto& occ = ctx->pair_occ[T == 2 ? 0 : T == 4 ? 1 : T == 8 ? 2 : 3];
+        if (occ.smem != b.smem) {
+            e = occupancy_pair(T, b.smem, &occ.per_sm);
+            if (e != cudaSuccess) return cuda_fail(ctx, e, "occupancy_pair");
+            occ.smem = b.smem;
+        }
+        per_sm = occ.per_sm;
         if (per_sm < 1) return fail(ctx, BDCU_E_LIMIT, "pair kernel shape cannot be resident");
         b.grid = std::max(1, std::min(b.count, per_sm * ctx->sm_count));
         b.scratch_stride = b.need_lz ? pair_scratch_doubles(b.n_max) : 1;
@@ -606,8 +611,7 @@ int bdcu_destroy(bdcu_ctx* ctx) {
     if (!ctx) return BDCU_OK;
     cudaSetDevice(ctx->device);
     cudaDeviceSynchronize();
-    void* ptrs[] = {ctx->chains_d, ctx->arena_d, ctx->seed_d, ctx->work_d, ctx->hR, ctx->hrng, ctx->hcache,
-                    ctx->hvalid, ctx->ht0, ctx->hsteps, ctx->hstatus, ctx->hcnt, ctx->xs_pow_d, ctx->a_pow_d,
+    void* ptrs[] = {ctx->chains_d, ctx->arena_d, ctx->seed_d, ctx->work_d, ctx->hblk, ctx->xs_pow_d, ctx->a_pow_d,
                     ctx->order_d, ctx->rec_dev};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -617,6 +621,7 @@ int bdcu_destroy(bdcu_ctx* ctx) {
         if (ctx->ev_join[i]) cudaEventDestroy(ctx->ev_join[i]);
     }
     if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
+    if (ctx->hpin) cudaFreeHost(ctx->hpin);
     free_staging(ctx->order_stage);
     free_staging(ctx->rec_stage);
     free_staging(ctx->arena_stage);
@@ -686,9 +691,13 @@ int bdcu_set_chains(bdcu_ctx* ctx, int n_chains, const bdcu_phys* phys, const bd
             if (p.hi_method == BDCU_HI_CHOLESKY) any_chol_method = 1;
         }
     }
-    if ((rc = ensure(ctx, &ctx->chains_d, n_chains))) return rc;
+    // records and arena of a batch no larger than before are rewritten in place
+    // (a free and an allocation cost each small integrate call ~100 us); earlier
+    // runs on any stream may still read them, so wait as a free would
+    if (ctx->chains_d) CK(cudaDeviceSynchronize());
+    if ((rc = ensure(ctx, &ctx->chains_d, n_chains, &ctx->chains_bytes))) return rc;
     CK(cudaMemcpy(ctx->chains_d, recs.data(), sizeof(DevChain) * n_chains, cudaMemcpyHostToDevice));
-    if ((rc = ensure(ctx, &ctx->arena_d, arena_len > 0 ? arena_len : 1))) return rc;
+    if ((rc = ensure(ctx, &ctx->arena_d, arena_len > 0 ? arena_len : 1, &ctx->arena_bytes))) return rc;
     if (arena_len > 0 && arena)
         CK(cudaMemcpy(ctx->arena_d, arena, sizeof(double) * arena_len, cudaMemcpyHostToDevice));
     ctx->chains_h.swap(recs);
@@ -930,9 +939,9 @@ int bdcu_reserve(bdcu_ctx* ctx, int n_slots, int64_t bead_capacity, int64_t aren
     int rc;
     if ((rc = ensure_tables(ctx))) return rc;
     CK(cudaDeviceSynchronize());  // the records and arena may be in use by earlier runs
-    if ((rc = ensure(ctx, &ctx->chains_d, n_slots))) return rc;
+    if ((rc = ensure(ctx, &ctx->chains_d, n_slots, &ctx->chains_bytes))) return rc;
     CK(cudaMemset(ctx->chains_d, 0, sizeof(DevChain) * n_slots));
-    if ((rc = ensure(ctx, &ctx->arena_d, arena_len > 0 ? arena_len : 1))) return rc;
+    if ((rc = ensure(ctx, &ctx->arena_d, arena_len > 0 ? arena_len : 1, &ctx->arena_bytes))) return rc;
     CK(cudaMemset(ctx->arena_d, 0, sizeof(double) * std::max<int64_t>(arena_len, 1)));
     // pinned staging for the uploads of a serving loop, sized once here: a
     // pinned buffer that grew later would have to be freed (cudaFreeHost
@@ -1058,19 +1067,21 @@ int bdcu_integrate_host(bdcu_ctx* ctx, double* R_host, int32_t* rng_host, int32_
     const int nc = ctx->n_chains;
     const int64_t nb = ctx->total_beads;
     int rc;
-    if (nb > ctx->hcap_beads) {
-        if ((rc = ensure(ctx, &ctx->hR, 3 * nb))) return rc;
-        if ((rc = ensure(ctx, &ctx->hcache, 3 * nb))) return rc;
-        ctx->hcap_beads = nb;
-    }
-    if (nc > ctx->hcap_chains) {
-        if ((rc = ensure(ctx, &ctx->hrng, 3 * nc))) return rc;
-        if ((rc = ensure(ctx, &ctx->hvalid, nc))) return rc;
-        if ((rc = ensure(ctx, &ctx->ht0, nc))) return rc;
-        if ((rc = ensure(ctx, &ctx->hsteps, nc))) return rc;
-        if ((rc = ensure(ctx, &ctx->hstatus, nc))) return rc;
-        if ((rc = ensure(ctx, &ctx->hcnt, nc))) return rc;
-        ctx->hcap_chains = nc;
+    // one block: inputs (t0, R, rng, steps), what starts at zero (status,
+    // counters, cache_valid), the warm-start vectors; R .. counters come back
+    auto up = [](size_t x) { return (x + 255) / 256 * 256; };
+    const size_t o_t0 = 0, o_R = up(o_t0 + sizeof(double) * nc), o_rng = up(o_R + sizeof(double) * 3 * nb),
+                 o_steps = up(o_rng + sizeof(int32_t) * 3 * nc), o_status = up(o_steps + sizeof(int32_t) * nc),
+                 o_cnt = up(o_status + sizeof(int32_t) * nc), o_valid = up(o_cnt + sizeof(bdcu_counters) * nc),
+                 o_cache = up(o_valid + sizeof(int32_t) * nc), total = up(o_cache + sizeof(double) * 3 * nb);
+    if ((rc = ensure(ctx, &ctx->hblk, total, &ctx->hblk_bytes))) return rc;
+    // small batches go through pinned memory in one copy each way (eight
+    // separate pageable copies cost a 10-bead call ~80 us)
+    constexpr size_t kPinned = 1 << 17;
+    const bool packed = o_valid <= kPinned;
+    if (packed && !ctx->hpin) {
+        CK(cudaHostAlloc(reinterpret_cast<void**>(&ctx->hpin), kPinned, cudaHostAllocDefault));
+        ctx->hpin_bytes = kPinned;
     }
     std::vector<double> t0(nc);
     std::vector<int32_t> steps(nc);
@@ -1082,21 +1093,43 @@ int bdcu_integrate_host(bdcu_ctx* ctx, double* R_host, int32_t* rng_host, int32_
         steps[i] = (int32_t)k;
     }
     cudaStream_t s = ctx->stream;
-    CK(cudaMemcpyAsync(ctx->hR, R_host, sizeof(double) * 3 * nb, cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(ctx->hrng, rng_host, sizeof(int32_t) * 3 * nc, cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(ctx->ht0, t0.data(), sizeof(double) * nc, cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(ctx->hsteps, steps.data(), sizeof(int32_t) * nc, cudaMemcpyHostToDevice, s));
-    CK(cudaMemsetAsync(ctx->hvalid, 0, sizeof(int32_t) * nc, s));
-    CK(cudaMemsetAsync(ctx->hstatus, 0, sizeof(int32_t) * nc, s));
-    CK(cudaMemsetAsync(ctx->hcnt, 0, sizeof(bdcu_counters) * nc, s));
-    rc = bdcu_run(ctx, ctx->hR, ctx->hrng, ctx->hcache, ctx->hvalid, ctx->ht0, ctx->hsteps, ctx->hstatus, ctx->hcnt,
-                  form, BDCU_CACHE_RESET_PER_CALL);
-    if (rc) return rc;
-    CK(cudaMemcpyAsync(R_host, ctx->hR, sizeof(double) * 3 * nb, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(rng_host, ctx->hrng, sizeof(int32_t) * 3 * nc, cudaMemcpyDeviceToHost, s));
-    if (status_host) CK(cudaMemcpyAsync(status_host, ctx->hstatus, sizeof(int32_t) * nc, cudaMemcpyDeviceToHost, s));
+    unsigned char* d = ctx->hblk;
+    if (packed) {
+        memcpy(ctx->hpin + o_t0, t0.data(), sizeof(double) * nc);
+        memcpy(ctx->hpin + o_R, R_host, sizeof(double) * 3 * nb);
+        memcpy(ctx->hpin + o_rng, rng_host, sizeof(int32_t) * 3 * nc);
+        memcpy(ctx->hpin + o_steps, steps.data(), sizeof(int32_t) * nc);
+        CK(cudaMemcpyAsync(d, ctx->hpin, o_status, cudaMemcpyHostToDevice, s));
+    } else {
+        CK(cudaMemcpyAsync(d + o_t0, t0.data(), sizeof(double) * nc, cudaMemcpyHostToDevice, s));
+        CK(cudaMemcpyAsync(d + o_R, R_host, sizeof(double) * 3 * nb, cudaMemcpyHostToDevice, s));
+        CK(cudaMemcpyAsync(d + o_rng, rng_host, sizeof(int32_t) * 3 * nc, cudaMemcpyHostToDevice, s));
+        CK(cudaMemcpyAsync(d + o_steps, steps.data(), sizeof(int32_t) * nc, cudaMemcpyHostToDevice, s));
+    }
+    CK(cudaMemsetAsync(d + o_status, 0, o_cache - o_status, s));
+    rc = bdcu_run(ctx, reinterpret_cast<double*>(d + o_R), reinterpret_cast<int32_t*>(d + o_rng),
+                  reinterpret_cast<double*>(d + o_cache), reinterpret_cast<int32_t*>(d + o_valid),
+                  reinterpret_cast<const double*>(d + o_t0), reinterpret_cast<const int32_t*>(d + o_steps),
+                  reinterpret_cast<int32_t*>(d + o_status), reinterpret_cast<bdcu_counters*>(d + o_cnt), form,
+                  BDCU_CACHE_RESET_PER_CALL);
+    if (rc) {
+        cudaStreamSynchronize(s);  // (the input copies read host memory of this call)
+        return rc;
+    }
+    if (packed) {
+        CK(cudaMemcpyAsync(ctx->hpin + o_R, d + o_R, o_valid - o_R, cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+        memcpy(R_host, ctx->hpin + o_R, sizeof(double) * 3 * nb);
+        memcpy(rng_host, ctx->hpin + o_rng, sizeof(int32_t) * 3 * nc);
+        if (status_host) memcpy(status_host, ctx->hpin + o_status, sizeof(int32_t) * nc);
+        if (counters_host) memcpy(counters_host, ctx->hpin + o_cnt, sizeof(bdcu_counters) * nc);
+        return BDCU_OK;
+    }
+    CK(cudaMemcpyAsync(R_host, d + o_R, sizeof(double) * 3 * nb, cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(rng_host, d + o_rng, sizeof(int32_t) * 3 * nc, cudaMemcpyDeviceToHost, s));
+    if (status_host) CK(cudaMemcpyAsync(status_host, d + o_status, sizeof(int32_t) * nc, cudaMemcpyDeviceToHost, s));
     if (counters_host)
-        CK(cudaMemcpyAsync(counters_host, ctx->hcnt, sizeof(bdcu_counters) * nc, cudaMemcpyDeviceToHost, s));
+        CK(cudaMemcpyAsync(counters_host, d + o_cnt, sizeof(bdcu_counters) * nc, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     return BDCU_OK;
 }

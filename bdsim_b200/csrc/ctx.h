@@ -86,6 +86,7 @@ struct bdcu_ctx {
     std::vector<double> seed_norm_h;  // seed_norm_h[n] = |default_seed(n)|, summed in order
     DevChain* chains_d = nullptr;
     double* arena_d = nullptr;
+    size_t chains_bytes = 0, arena_bytes = 0;  // their allocations
     double* seed_d = nullptr;
     int seed_len = 0;
     int32_t* work_d = nullptr;  // one queue counter per bucket
@@ -93,6 +94,8 @@ struct bdcu_ctx {
     int bounds_every = 1;  // bdcu_set_bounds_refresh
     int single_launch = 0; // bdcu_set_single_launch: every team-kernel chain in one launch
     size_t max_smem = 0;
+    // the pair kernel's last occupancy query per warp count (2, 4, 8, 16)
+    struct { size_t smem = 0; int per_sm = 0; } pair_occ[4];
     // the chains bdcu_run advances: all records (sel_all) or a list (bdcu_select)
     int sel_all = 1;
     std::vector<int32_t> sel;
@@ -112,15 +115,10 @@ struct bdcu_ctx {
     cudaEvent_t ev_fork = nullptr;
     cudaEvent_t ev_join[bdcu::kMaxBuckets] = {};
     bdcu::Shape tuned[2][bdcu::kMaxBuckets];
-    // buffers of bdcu_integrate_host
-    double* hR = nullptr;
-    int32_t* hrng = nullptr;
-    double* hcache = nullptr;
-    int32_t* hvalid = nullptr;
-    double* ht0 = nullptr;
-    int32_t* hsteps = nullptr;
-    int32_t* hstatus = nullptr;
-    bdcu_counters* hcnt = nullptr;
-    int64_t hcap_beads = 0;
-    int hcap_chains = 0;
+    // bdcu_integrate_host: one device block for its state, and a pinned copy of
+    // it for small batches
+    unsigned char* hblk = nullptr;
+    size_t hblk_bytes = 0;
+    unsigned char* hpin = nullptr;
+    size_t hpin_bytes = 0;
 };

@@ -476,15 +476,16 @@ struct RpyConst {
         om1 = rho * fma(A3, t, A1);
         om2 = (rho * t) * fma(-B3, t, A1);
     }
-    // Any pair, and a bead with itself (omega1 = 1 along the diagonal block).
+    // Near pairs, and a bead with itself (omega1 = 1 along the diagonal block).
+    __device__ __forceinline__ void near_weights(double sq, bool self, double& om1, double& om2) const {
+        sq = fmax(sq, 1.0e-12);
+        const double rho = rsqrt_refined(sq);
+        om1 = self ? 1.0 : fma(-c3, sq * rho, 1.0);
+        om2 = self ? 0.0 : c7 * rho;
+    }
     __device__ __forceinline__ void weights(double sq, bool self, double& om1, double& om2) const {
         far_weights(sq, om1, om2);
-        if (!(sq >= far2)) {
-            sq = fmax(sq, 1.0e-12);
-            const double rho = rsqrt_refined(sq);
-            om1 = self ? 1.0 : fma(-c3, sq * rho, 1.0);
-            om2 = self ? 0.0 : c7 * rho;
-        }
+        if (!(sq >= far2)) near_weights(sq, self, om1, om2);
     }
 };
 

@@ -465,6 +465,7 @@ struct TeamChain {
                     }
                 }
         }
+        // the rest: weights evaluated here
 #pragma unroll 1
         for (; j < n2; j += 2) {
             float2 pj[3], xj[K][3];
@@ -477,11 +478,11 @@ struct TeamChain {
 #pragma unroll
             for (int q = 0; q < Q; ++q)
                 if (q < nq) {
-                    const float2 dx = __fadd2_rn(pj[0], nb[q][0]), dy = __fadd2_rn(pj[1], nb[q][1]),
-                                 dz = __fadd2_rn(pj[2], nb[q][2]);
+                    const float2 d[3] = {__fadd2_rn(pj[0], nb[q][0]), __fadd2_rn(pj[1], nb[q][1]),
+                                         __fadd2_rn(pj[2], nb[q][2])};
                     float2 om1, om2;
-                    pair_weights2(dx, dy, dz, om1, om2);
-                    products(q, dx, dy, dz, om1, om2, xj);
+                    pair_weights2(d, om1, om2);
+                    products(q, d[0], d[1], d[2], om1, om2, xj);
                 }
         }
 #pragma unroll
@@ -517,21 +518,21 @@ struct TeamChain {
     // the near ones in a branch that only neighbours along the chain and close
     // contacts take. The self pair (d = 0, s clamped to 1e-24) is a near one
     // with om1 = 1 exactly in FP32 and om2 d = 0: the identity block.
-    __device__ __forceinline__ void pair_weights2(const float2& dx, const float2& dy, const float2& dz, float2& om1,
-                                                  float2& om2) const {
+    __device__ __forceinline__ void pair_weights2(const float2 (&d)[3], float2& om1, float2& om2) const {
         const float2 k1 = make_float2(K1, K1), k2 = make_float2(K2, K2), mk3 = make_float2(-K3, -K3);
-        float2 sq = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
-        sq = make_float2(fmaxf(sq.x, 1e-24f), fmaxf(sq.y, 1e-24f));
+        const float2 sq = __ffma2_rn(d[2], d[2], __ffma2_rn(d[1], d[1], __fmul2_rn(d[0], d[0])));
         const float2 rho = make_float2(rsqrt_approx(sq.x), rsqrt_approx(sq.y));
         const float2 t = __fmul2_rn(rho, rho);
         om1 = __fmul2_rn(rho, __ffma2_rn(k2, t, k1));
         om2 = __fmul2_rn(__fmul2_rn(rho, t), __ffma2_rn(mk3, t, k1));
-        const bool nx = sq.x < 12.566370614359172f, ny = sq.y < 12.566370614359172f;
-        if (nx || ny) {
-            const float2 n1 = __ffma2_rn(make_float2(-C3, -C3), __fmul2_rn(sq, rho), make_float2(1.f, 1.f));
-            const float2 n2 = __fmul2_rn(make_float2(C7, C7), rho);
-            if (nx) om1.x = n1.x, om2.x = n2.x;
-            if (ny) om1.y = n1.y, om2.y = n2.y;
+        constexpr float kNear = 12.566370614359172f;  // 4 pi
+        if (fminf(sq.x, sq.y) < kNear) {
+            const float2 sc = make_float2(fmaxf(sq.x, 1e-24f), fmaxf(sq.y, 1e-24f));
+            const float2 rc = make_float2(rsqrt_approx(sc.x), rsqrt_approx(sc.y));
+            const float2 n1 = __ffma2_rn(make_float2(-C3, -C3), __fmul2_rn(sc, rc), make_float2(1.f, 1.f));
+            const float2 n2 = __fmul2_rn(make_float2(C7, C7), rc);
+            om1 = make_float2(sq.x < kNear ? n1.x : om1.x, sq.y < kNear ? n1.y : om1.y);
+            om2 = make_float2(sq.x < kNear ? n2.x : om2.x, sq.y < kNear ? n2.y : om2.y);
         }
     }
 
@@ -540,16 +541,17 @@ struct TeamChain {
     __device__ __forceinline__ void build_weights() {
         float2 nb[Q][3];
         own_coordinates(nb);
-#pragma unroll 1
+#pragma unroll 2
         for (int j = 0; j < jc; j += 2) {
             float2 pj[3];
 #pragma unroll
             for (int d = 0; d < 3; ++d) pj[d] = *reinterpret_cast<const float2*>(&S.ps[d][j]);
 #pragma unroll
             for (int q = 0; q < Q; ++q) {
+                const float2 d[3] = {__fadd2_rn(pj[0], nb[q][0]), __fadd2_rn(pj[1], nb[q][1]),
+                                     __fadd2_rn(pj[2], nb[q][2])};
                 float2 om1, om2;
-                pair_weights2(__fadd2_rn(pj[0], nb[q][0]), __fadd2_rn(pj[1], nb[q][1]), __fadd2_rn(pj[2], nb[q][2]), om1,
-                              om2);
+                pair_weights2(d, om1, om2);
                 if (valid(q)) Wt[(j >> 1) * N + bead(q)] = make_float4(om1.x, om1.y, om2.x, om2.y);
             }
         }

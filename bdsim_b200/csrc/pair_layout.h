@@ -76,10 +76,13 @@ __host__ __device__ inline PairLayout pair_layout(int n_max, int T, int64_t w_pa
 }
 
 // Pair weights a block of shape T caches: all of the largest chain's when they
-// fit the block's share of an SM's shared memory, else as many rows as fit (the
-// rest is evaluated again in every product).
-__host__ inline int64_t pair_cached(int n_max, int T, size_t max_smem) {
-    const int64_t share = ((int64_t)max_smem + 1024) / pair_min_blocks(T) - 1024;
+// fit the block's share of an SM's shared memory, else as many as fit (the rest
+// is evaluated again in every product). The share is what the launch's `blocks`
+// leave an SM. The split changes no result.
+__host__ inline int64_t pair_cached(int n_max, int T, int blocks, int sm_count, size_t max_smem) {
+    int per_sm = (blocks + sm_count - 1) / sm_count;
+    if (per_sm > pair_min_blocks(T)) per_sm = pair_min_blocks(T);
+    const int64_t share = ((int64_t)max_smem + 1024) / per_sm - 1024;
     const int64_t room = (share / 8 - pair_layout(n_max, T, 0).total) / 2;
     const int64_t all = pair_weights(n_max / 3, T);
     return room <= 0 ? 0 : room < all ? room : all;

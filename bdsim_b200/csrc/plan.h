@@ -46,17 +46,18 @@ inline int64_t team_smem(int T, int Q, int n_max, int64_t w_pairs) {
 #undef BDCU_SMEM
 }
 
-// Cached weights per team of shape (T, Q).
-inline int64_t team_weights(int T, int Q, int n_max, size_t max_smem) {
-#define BDCU_WTS(t, q) (team_cached<t, q>(n_max, max_smem))
-    return BDCU_TEAM_SHAPE_SWITCH(T, Q, BDCU_WTS, (int64_t)0);
-#undef BDCU_WTS
-}
-
 inline int teams_per_cta(int T, int Q) {
 #define BDCU_TPC(t, q) TeamCfg<t, q>::kTeamsPerCta
     return BDCU_TEAM_SHAPE_SWITCH(T, Q, BDCU_TPC, 1);
 #undef BDCU_TPC
+}
+
+// Cached weights per team of shape (T, Q) in a launch over `chains` chains.
+inline int64_t team_weights(int T, int Q, int n_max, int chains, int sm_count, size_t max_smem) {
+    const int blocks = (chains + teams_per_cta(T, Q) - 1) / teams_per_cta(T, Q);
+#define BDCU_WTS(t, q) (team_cached<t, q>(n_max, blocks, sm_count, max_smem))
+    return BDCU_TEAM_SHAPE_SWITCH(T, Q, BDCU_WTS, (int64_t)0);
+#undef BDCU_WTS
 }
 
 // Whether (T, Q) is a compiled team shape that holds chains of `beads`.

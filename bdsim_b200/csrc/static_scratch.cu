@@ -172,7 +172,7 @@ extern "C" int bdcu_run_static(bdcu_ctx* ctx, int n_chains, const bdcu_phys* phy
             any_team = true;
             l.team_warps = kDefaultTeamShape[id][0];
             l.team_q = kDefaultTeamShape[id][1];
-            l.w_pairs = l.need_d ? team_weights(l.team_warps, l.team_q, l.n_max, ctx->max_smem) : 0;
+            l.w_pairs = l.need_d ? team_weights(l.team_warps, l.team_q, l.n_max, l.count, ctx->sm_count, ctx->max_smem) : 0;
             l.smem = (size_t)team_smem(l.team_warps, l.team_q, l.n_max, l.w_pairs);
             if (l.smem > ctx->max_smem) return fail(ctx, BDCU_E_LIMIT, "bdcu_run_static: team kernel shared memory too large");
             e = occupancy_mixed_team(l.team_warps, l.team_q, l.smem, &per_sm);

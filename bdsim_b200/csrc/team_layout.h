@@ -75,11 +75,16 @@ __host__ __device__ inline int64_t team_smem_bytes(int n_max, int64_t w_pairs) {
     return team_area_stride<T, Q>(n_max, w_pairs) * TeamCfg<T, Q>::kTeamsPerCta;
 }
 // Cached weights per team (16 bytes: a bead with two partners): all of the
-// largest chain's when they fit the team's share of an SM's shared memory at the
-// blocks per SM the registers are sized for, else as many as fit.
+// largest chain's when they fit the team's share of an SM's shared memory, else
+// as many as fit. The share is what the launch's `blocks` leave an SM: the
+// blocks per SM the registers are sized for, or fewer when the launch cannot
+// fill the SMs anyway (96 chains of N = 137 on 148 SMs keep all weights instead
+// of a quarter). The split changes no result.
 template <int T, int Q>
-inline int64_t team_cached(int n_max, size_t max_smem) {
-    const int64_t share = ((int64_t)max_smem + 1024) / TeamCfg<T, Q>::kMinBlocks - 1024;
+inline int64_t team_cached(int n_max, int blocks, int sm_count, size_t max_smem) {
+    int per_sm = (blocks + sm_count - 1) / sm_count;
+    if (per_sm > TeamCfg<T, Q>::kMinBlocks) per_sm = TeamCfg<T, Q>::kMinBlocks;
+    const int64_t share = ((int64_t)max_smem + 1024) / per_sm - 1024;
     const int64_t room = (share / TeamCfg<T, Q>::kTeamsPerCta - team_weight_offset<T, Q>(n_max)) / 16;
     const int64_t N = n_max / 3, all = (N + 3) / 4 * 2 * N;
     return room <= 0 ? 0 : room < all ? room : all;
