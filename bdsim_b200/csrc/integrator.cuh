@@ -880,14 +880,15 @@ struct Block {
             if (i0 + tr + 7 < j0 + tcs) continue;  // the whole strip above the diagonal (warp-uniform)
             double c[4][2];
             dmma_load_c(s, i0, j0, jend, lane, c);
-            dmma_strip<4>(s, c, As, Bs, i0, j0, jend, kk4, lane);
+            dmma_strip<3>(s, c, As, Bs, i0, j0, jend, kk4, lane);
         }
     }
 
     // Strip s of the tile at (i0, j0): C (loaded into c) -= A B over kk4 staged
-    // k rows, stored back. kDmmaChains accumulation chains per fragment (k
-    // steps rotate over c and cx, summed at the end) cut the dependent-DMMA
-    // wait (a reassociation: rounding only).
+    // k rows, stored back. kDmmaChains accumulation chains per fragment, all from
+    // zero (k steps rotate over them), cut the dependent-DMMA wait, and C is
+    // added last, so that its loads from L2 or DRAM have the whole multiply to
+    // arrive in (a reassociation: rounding only).
     template <int kDmmaChains>
     __device__ void dmma_strip(int s, double (&c)[4][2], const double* As, const double* Bs, int i0, int j0, int jend,
                                int kk4, int lane) {
@@ -897,9 +898,9 @@ struct Block {
         {
             // blocks u < nact are active: the columns grow with u (warp-uniform)
             const int d = i0 + tr + 7 - j0 - tcs, nact = d >= 24 ? 4 : d / 8 + 1;
-            double cx[kDmmaChains - 1][4][2];
+            double cx[kDmmaChains][4][2];
 #pragma unroll
-            for (int h = 0; h < kDmmaChains - 1; ++h)
+            for (int h = 0; h < kDmmaChains; ++h)
 #pragma unroll
                 for (int u = 0; u < 4; ++u) cx[h][u][0] = cx[h][u][1] = 0.0;
             int k = 0;
@@ -911,8 +912,7 @@ struct Block {
                     for (int u = 0; u < 4; ++u) {
                         if (u < nact) {
                             const double bv = Bs[(k + 4 * h + q) * kCholTileStride + tcs + 8 * u + g];
-                            double& d0 = h == 0 ? c[u][0] : cx[h > 0 ? h - 1 : 0][u][0];
-                            double& d1 = h == 0 ? c[u][1] : cx[h > 0 ? h - 1 : 0][u][1];
+                            double &d0 = cx[h][u][0], &d1 = cx[h][u][1];
                             asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
                                          : "+d"(d0), "+d"(d1)
                                          : "d"(av), "d"(bv));
@@ -927,15 +927,17 @@ struct Block {
                     if (u < nact) {
                         const double bv = Bs[(k + q) * kCholTileStride + tcs + 8 * u + g];
                         asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-                                     : "+d"(c[u][0]), "+d"(c[u][1])
+                                     : "+d"(cx[0][u][0]), "+d"(cx[0][u][1])
                                      : "d"(av), "d"(bv));
                     }
                 }
             }
 #pragma unroll
-            for (int h = 0; h < kDmmaChains - 1; ++h)
+            for (int h = 1; h < kDmmaChains; ++h)
 #pragma unroll
-                for (int u = 0; u < 4; ++u) c[u][0] += cx[h][u][0], c[u][1] += cx[h][u][1];
+                for (int u = 0; u < 4; ++u) cx[0][u][0] += cx[h][u][0], cx[0][u][1] += cx[h][u][1];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) c[u][0] += cx[0][u][0], c[u][1] += cx[0][u][1];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const int i = i0 + tr + g, ja = j0 + tcs + 8 * u + 2 * q, jb = ja + 1;

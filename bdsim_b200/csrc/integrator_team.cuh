@@ -475,15 +475,33 @@ struct TeamChain {
 #pragma unroll
                 for (int r = 0; r < K; ++r) xj[r][d] = *reinterpret_cast<const float2*>(&xr[r][d][j]);
             }
+            if (K == 1 && Q == 2 && nq == 2) {
+                // both beads' chains of operations side by side, with one branch
+                // for their near pairs (N = 500: two warps per scheduler leave
+                // the FP32 pipe 46% busy with the beads one after the other)
+                float2 d[Q][3], sq[Q], om1[Q], om2[Q];
 #pragma unroll
-            for (int q = 0; q < Q; ++q)
-                if (q < nq) {
-                    const float2 d[3] = {__fadd2_rn(pj[0], nb[q][0]), __fadd2_rn(pj[1], nb[q][1]),
-                                         __fadd2_rn(pj[2], nb[q][2])};
-                    float2 om1, om2;
-                    pair_weights2(d, om1, om2);
-                    products(q, d[0], d[1], d[2], om1, om2, xj);
+                for (int q = 0; q < Q; ++q) {
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) d[q][c] = __fadd2_rn(pj[c], nb[q][c]);
+                    far_weights2(d[q], sq[q], om1[q], om2[q]);
                 }
+                if (fminf(fminf(sq[0].x, sq[0].y), fminf(sq[Q - 1].x, sq[Q - 1].y)) < kNear)
+#pragma unroll
+                    for (int q = 0; q < Q; ++q) near_weights2(sq[q], om1[q], om2[q]);
+#pragma unroll
+                for (int q = 0; q < Q; ++q) products(q, d[q][0], d[q][1], d[q][2], om1[q], om2[q], xj);
+            } else {
+#pragma unroll
+                for (int q = 0; q < Q; ++q)
+                    if (q < nq) {
+                        const float2 d[3] = {__fadd2_rn(pj[0], nb[q][0]), __fadd2_rn(pj[1], nb[q][1]),
+                                             __fadd2_rn(pj[2], nb[q][2])};
+                        float2 om1, om2;
+                        pair_weights2(d, om1, om2);
+                        products(q, d[0], d[1], d[2], om1, om2, xj);
+                    }
+            }
         }
 #pragma unroll
         for (int q = 0; q < Q; ++q)
@@ -518,22 +536,27 @@ struct TeamChain {
     // the near ones in a branch that only neighbours along the chain and close
     // contacts take. The self pair (d = 0, s clamped to 1e-24) is a near one
     // with om1 = 1 exactly in FP32 and om2 d = 0: the identity block.
-    __device__ __forceinline__ void pair_weights2(const float2 (&d)[3], float2& om1, float2& om2) const {
+    static constexpr float kNear = 12.566370614359172f;  // 4 pi
+    __device__ __forceinline__ void far_weights2(const float2 (&d)[3], float2& sq, float2& om1, float2& om2) const {
         const float2 k1 = make_float2(K1, K1), k2 = make_float2(K2, K2), mk3 = make_float2(-K3, -K3);
-        const float2 sq = __ffma2_rn(d[2], d[2], __ffma2_rn(d[1], d[1], __fmul2_rn(d[0], d[0])));
+        sq = __ffma2_rn(d[2], d[2], __ffma2_rn(d[1], d[1], __fmul2_rn(d[0], d[0])));
         const float2 rho = make_float2(rsqrt_approx(sq.x), rsqrt_approx(sq.y));
         const float2 t = __fmul2_rn(rho, rho);
         om1 = __fmul2_rn(rho, __ffma2_rn(k2, t, k1));
         om2 = __fmul2_rn(__fmul2_rn(rho, t), __ffma2_rn(mk3, t, k1));
-        constexpr float kNear = 12.566370614359172f;  // 4 pi
-        if (fminf(sq.x, sq.y) < kNear) {
-            const float2 sc = make_float2(fmaxf(sq.x, 1e-24f), fmaxf(sq.y, 1e-24f));
-            const float2 rc = make_float2(rsqrt_approx(sc.x), rsqrt_approx(sc.y));
-            const float2 n1 = __ffma2_rn(make_float2(-C3, -C3), __fmul2_rn(sc, rc), make_float2(1.f, 1.f));
-            const float2 n2 = __fmul2_rn(make_float2(C7, C7), rc);
-            om1 = make_float2(sq.x < kNear ? n1.x : om1.x, sq.y < kNear ? n1.y : om1.y);
-            om2 = make_float2(sq.x < kNear ? n2.x : om2.x, sq.y < kNear ? n2.y : om2.y);
-        }
+    }
+    __device__ __forceinline__ void near_weights2(const float2& sq, float2& om1, float2& om2) const {
+        const float2 sc = make_float2(fmaxf(sq.x, 1e-24f), fmaxf(sq.y, 1e-24f));
+        const float2 rc = make_float2(rsqrt_approx(sc.x), rsqrt_approx(sc.y));
+        const float2 n1 = __ffma2_rn(make_float2(-C3, -C3), __fmul2_rn(sc, rc), make_float2(1.f, 1.f));
+        const float2 n2 = __fmul2_rn(make_float2(C7, C7), rc);
+        om1 = make_float2(sq.x < kNear ? n1.x : om1.x, sq.y < kNear ? n1.y : om1.y);
+        om2 = make_float2(sq.x < kNear ? n2.x : om2.x, sq.y < kNear ? n2.y : om2.y);
+    }
+    __device__ __forceinline__ void pair_weights2(const float2 (&d)[3], float2& om1, float2& om2) const {
+        float2 sq;
+        far_weights2(d, sq, om1, om2);
+        if (fminf(sq.x, sq.y) < kNear) near_weights2(sq, om1, om2);
     }
 
     // Weights of the thread's beads with partners below jc at the staged
