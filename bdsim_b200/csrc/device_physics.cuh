@@ -271,30 +271,6 @@ __device__ __forceinline__ double clamped_len(double b0, double b1, double b2) {
     return sqrt(sq);
 }
 
-// gauss_factor / lj_factor / sdk_factor (src/excluded_volume.cpp:36-58)
-__device__ inline double ev_factor(const DevChain& c, double r, double phi_pair) {
-    switch (c.ev_type) {
-        case BDCU_EV_GAUSS: return c.zsbyds5 * exp(-r * r * c.pt5bydssq);
-        case BDCU_EV_LJ: {
-            const double Rcut = c.equil ? c.Rcutg : c.Rcutp;
-            if (r <= Rcut && r >= c.Rmin) return c.LJa / pow(r, 14.0) - c.LJb / pow(r, 8.0);
-            if (r < c.Rmin) return c.lj_rmin_fac;
-            return 0.0;
-        }
-        case BDCU_EV_SDK: {
-            double fac = 0.0;
-            if (r <= c.Rcutg && r >= c.Rmin)
-                fac = c.SDKa / pow(r, 14.0) - c.SDKb / pow(r, 8.0);
-            else if (r < c.Rmin)
-                fac = c.sdk_rmin_fac;
-            if (!c.equil && r <= c.RcutpSDK && r > c.Rcutg)
-                fac += 1.530633312 * phi_pair * sin(1.530633312 * r * r + 1.213115524);
-            return fac;
-        }
-        default: return 0.0;
-    }
-}
-
 // Distance beyond which the LJ and SDK factors are zero (0: everywhere).
 __device__ __forceinline__ double ev_outer_cutoff(const DevChain& c) {
     switch (c.ev_type) {
@@ -304,9 +280,10 @@ __device__ __forceinline__ double ev_outer_cutoff(const DevChain& c) {
     }
 }
 
-// lj_factor / sdk_factor as ev_factor, at squared distance sq, with the 14th
-// and 8th powers of r as products of 1/r^2. phi: the pair's attractive
-// strength (null: zero).
+// lj_factor / sdk_factor (src/excluded_volume.cpp:42-58) at squared distance sq,
+// with the 14th and 8th powers of r as products of 1/r^2 (the library's pow()
+// costs a hundred operations each). phi: the pair's attractive strength (null:
+// zero). gauss_factor is written out in the pair loops.
 __device__ inline double ev_factor_short(const DevChain& c, double sq, const double* phi) {
     const double r = sqrt(sq);
     const bool sdk = c.ev_type == BDCU_EV_SDK;

@@ -402,31 +402,27 @@ struct Block {
     }
 
     // ---- RPY tensor (rpy_diffusion_matrix, src/hydrodynamics.cpp:12-54) --
-    // Writes the dense D at ptr with leading dimension ld. For pair mu<nu the
-    // value of element (3mu+i, 3nu+j) and its mirror is
-    // om2*b_i*b_j + (i==j ? om1 : 0).
-    __device__ void build_rpy(const double* R, double* Dp, int ld) {
-        for (int idx = threadIdx.x; idx < 9 * N; idx += blockDim.x) {
-            const int mu = idx / 9, i = (idx % 9) / 3, j = idx % 3;
-            Dp[(int64_t)(3 * mu + i) * ld + 3 * mu + j] = (i == j) ? 1.0 : 0.0;
-        }
-        const int npairs = N * (N - 1) / 2;
-        for (int pidx = threadIdx.x; pidx < npairs; pidx += blockDim.x) {
-            int nu = (int)((1.0 + sqrt(1.0 + 8.0 * (double)pidx)) * 0.5);
-            while (nu * (nu - 1) / 2 > pidx) --nu;
-            while ((nu + 1) * nu / 2 <= pidx) ++nu;
-            const int mu = pidx - nu * (nu - 1) / 2;
-            double b[3];
-            for (int d = 0; d < 3; ++d) b[d] = R[3 * nu + d] - R[3 * mu + d];
-            const double sq = b[0] * b[0] + b[1] * b[1] + b[2] * b[2];
-            double om1, om2;
-            rpy_weights(ch.hstar, sq, om1, om2);
-            for (int i = 0; i < 3; ++i)
-                for (int j = 0; j < 3; ++j) {
-                    const double val = om2 * b[i] * b[j] + (i == j ? om1 : 0.0);
-                    Dp[(int64_t)(3 * mu + i) * ld + 3 * nu + j] = val;
-                    Dp[(int64_t)(3 * nu + j) * ld + 3 * mu + i] = val;
-                }
+    // The lower part of D at R into Lp, column-major with leading dimension ld
+    // (the factor's storage): for beads mu <= nu element (3nu+i, 3mu+j) is
+    // om2*b_i*b_j + (i==j ? om1 : 0). One warp per bead column, lanes along the
+    // rows, so that a warp's stores fill consecutive lines. (Both halves written
+    // pair by pair, each value to a line of its own, took 19% of a N = 500
+    // Cholesky step with the forces.)
+    __device__ void build_rpy(const double* R, double* Lp, int ld) {
+        RpyConst rpy;
+        rpy.set(ch.hstar);
+        for (int mu = threadIdx.x >> 5; mu < N; mu += blockDim.x >> 5) {
+            const double r0 = R[3 * mu], r1 = R[3 * mu + 1], r2 = R[3 * mu + 2];
+            for (int nu = mu + (threadIdx.x & 31); nu < N; nu += 32) {
+                const double b[3] = {R[3 * nu] - r0, R[3 * nu + 1] - r1, R[3 * nu + 2] - r2};
+                double om1, om2;
+                rpy.weights(fma(b[2], b[2], fma(b[1], b[1], b[0] * b[0])), nu == mu, om1, om2);
+                double* col = Lp + (int64_t)(3 * mu) * ld + 3 * nu;
+#pragma unroll
+                for (int j = 0; j < 3; ++j)
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) col[(int64_t)j * ld + i] = om2 * b[i] * b[j] + (i == j ? om1 : 0.0);
+            }
         }
     }
 
@@ -995,55 +991,51 @@ struct Block {
     }
 
     // Excluded-volume force on bead b (ExcludedVolume::force,
-    // src/excluded_volume.cpp:60-89): bead b receives -f(j,b) for j<b, then
-    // +f(b,j) for j>b, in ascending j -- the reference loop's order.
+    // src/excluded_volume.cpp:60-89): the force from j is -fac (R_j - R_b),
+    // contour distance at least cd. LJ and SDK pairs beyond the outer cutoff are
+    // passed over on the squared distance, before the pair's phi is read.
     __device__ void ev_on_bead(const double* R, int b, double f[3]) {
         f[0] = f[1] = f[2] = 0.0;
         if (ch.ev_type == BDCU_EV_NONE) return;
+        const bool gauss = ch.ev_type == BDCU_EV_GAUSS;
         const double* phi = (ch.ev_type == BDCU_EV_SDK && ch.phi_off >= 0) ? a.arena + ch.phi_off : nullptr;
+        const double cut = ev_outer_cutoff(ch);
         if constexpr (!kMixed) {
+            const double cut2 = cut * cut * (1.0 + 1e-9);
+            const double r0 = R[3 * b], r1 = R[3 * b + 1], r2 = R[3 * b + 2];
+#pragma unroll 2
             for (int j = 0; j < N; ++j) {
-                if (j == b) continue;
+                const double q0 = R[3 * j] - r0, q1 = R[3 * j + 1] - r1, q2 = R[3 * j + 2] - r2;
+                const double sq = fmax(fma(q2, q2, fma(q1, q1, q0 * q0)), 1.0e-12);
+                const int dj = j > b ? j - b : b - j;
+                if (dj < ch.cd || j == b || (!gauss && sq > cut2)) continue;
                 const int mu = j < b ? j : b, nu = j < b ? b : j;
-                if ((nu - mu) < ch.cd) continue;
-                const double q0 = R[3 * nu] - R[3 * mu], q1 = R[3 * nu + 1] - R[3 * mu + 1],
-                             q2 = R[3 * nu + 2] - R[3 * mu + 2];
-                double sq = q0 * q0 + q1 * q1 + q2 * q2;
-                if (sq < 1.0e-12) sq = 1.0e-12;
-                const double r = sqrt(sq);
-                const double fac = ev_factor(ch, r, phi ? phi[mu * N + nu] : 0.0);
-                const double g0 = (-fac) * q0, g1 = (-fac) * q1, g2 = (-fac) * q2;
-                if (b == mu) {
-                    f[0] = f[0] + g0; f[1] = f[1] + g1; f[2] = f[2] + g2;
-                } else {
-                    f[0] = f[0] - g0; f[1] = f[1] - g1; f[2] = f[2] - g2;
-                }
+                const double fac = gauss ? ch.zsbyds5 * exp(-(sq * ch.pt5bydssq))
+                                         : ev_factor_short(ch, sq, phi ? phi + (int64_t)mu * N + nu : nullptr);
+                f[0] = fma(-fac, q0, f[0]);
+                f[1] = fma(-fac, q1, f[1]);
+                f[2] = fma(-fac, q2, f[2]);
             }
         } else {
-            // FP32 pair sums from the staged FP32 coordinates.
+            // FP32 pair sums from the staged FP32 coordinates (a margin of 1e-5
+            // on the cutoff covers their rounding)
+            const float cut2 = (float)(cut * cut * 1.00001);
             const float4 rb = pos32[b];
             float f0 = 0.f, f1 = 0.f, f2 = 0.f;
             const float zs = (float)ch.zsbyds5, p5 = (float)ch.pt5bydssq;
+#pragma unroll 2
             for (int j = 0; j < N; ++j) {
-                if (j == b) continue;
-                const int mu = j < b ? j : b, nu = j < b ? b : j;
-                if ((nu - mu) < ch.cd) continue;
                 const float4 rj = pos32[j];
-                // q = R_nu - R_mu; the force on b is -fac*q if b == mu, +fac*q if b == nu
-                const float s = (b == mu) ? 1.f : -1.f;
-                const float q0 = s * (rj.x - rb.x), q1 = s * (rj.y - rb.y), q2 = s * (rj.z - rb.z);
-                float sq = fmaxf(q0 * q0 + q1 * q1 + q2 * q2, 1e-12f);
-                const float r = sqrtf(sq);
-                float fac;
-                if (ch.ev_type == BDCU_EV_GAUSS) {
-                    fac = zs * __expf(-sq * p5);
-                } else {
-                    fac = (float)ev_factor(ch, (double)r, phi ? phi[mu * N + nu] : 0.0);
-                }
-                const float g = (b == mu) ? -fac : fac;
-                f0 += g * q0;
-                f1 += g * q1;
-                f2 += g * q2;
+                const float q0 = rj.x - rb.x, q1 = rj.y - rb.y, q2 = rj.z - rb.z;
+                const float sq = fmaxf(q0 * q0 + q1 * q1 + q2 * q2, 1e-12f);
+                const int dj = j > b ? j - b : b - j;
+                if (dj < ch.cd || j == b || (!gauss && !(sq <= cut2))) continue;
+                const int mu = j < b ? j : b, nu = j < b ? b : j;
+                const float fac = gauss ? zs * __expf(-sq * p5)
+                                        : (float)ev_factor_short(ch, (double)sq, phi ? phi + (int64_t)mu * N + nu : nullptr);
+                f0 -= fac * q0;
+                f1 -= fac * q1;
+                f2 -= fac * q2;
             }
             f[0] = f0;
             f[1] = f1;
