@@ -18,15 +18,16 @@ namespace bdcu {
 // Buckets of a launch plan. Buckets 0..3 hold the chains of N <= 64, 128, 256
 // and 512 beads that do not use the Cholesky method: the team kernel in the
 // FP32-mixed form, the pair kernel (one chain per block, reported as block
-// buckets 4..7) in the plain form, which takes Cholesky chains of N <= 64 too. Buckets 4..7 run one chain per block on the
-// general block kernel and split the rest by bead count at 64, 128 and 256.
+// buckets 4..7) in the plain form, which takes Cholesky chains of N <= 64 too.
+// Buckets 4..7 run one chain per block on the general block kernel and split the
+// rest by bead count at 64, 128 and 256.
 constexpr int kMaxBuckets = 8;
 constexpr int kFirstBlockBucket = 4;
 constexpr int kKernelPair = 2;  // Bucket::kernel of the pair kernel (BDCU_KERNEL_BLOCK outside)
 constexpr int kBucketBeads[kMaxBuckets] = {64, 128, 256, 512, 64, 128, 256, kMaxBeads};
 
 // A launch shape chosen by bdcu_autotune. Block kernel: threads per block,
-// Lanczos vectors in shared memory, dense D in shared memory. Team kernel:
+// Lanczos vectors in shared memory (pair kernel: threads only). Team kernel:
 // warps per team and beads per thread.
 struct Shape {
     int block = 0;  // 0: not tuned

@@ -437,7 +437,7 @@ __device__ __forceinline__ double rsqrt_refined(double s) {
 // with h* folded into the constants. (The two branches meet continuously at
 // r = 2 sqrt(pi) h*.)
 struct RpyConst {
-    double A1, A3, B3, c3, c7, far2;
+    double A1, A3, B3, c3, c7, far2, near2;
     __device__ void set(double h) {
         const double rpi = 1.7724538509055160, tpi = 6.283185307179586, k = 0.75 * rpi;
         A1 = k * h;
@@ -446,6 +446,7 @@ struct RpyConst {
         c3 = 0.75 / rpi * 0.375 / h;
         c7 = 0.09375 / rpi / h;
         far2 = (2.0 * rpi * h) * (2.0 * rpi * h);
+        near2 = fmax(far2, 1.0e-12);
     }
     // Far pairs (all but neighbours along the chain and close contacts).
     __device__ __forceinline__ void far_weights(double sq, double& om1, double& om2) const {
@@ -453,16 +454,23 @@ struct RpyConst {
         om1 = rho * fma(A3, t, A1);
         om2 = (rho * t) * fma(-B3, t, A1);
     }
-    // Near pairs, and a bead with itself (omega1 = 1 along the diagonal block).
+    // Near pairs, separations below the reference's clamp (which an h* below
+    // 3e-7 can make far ones), and a bead with itself (omega1 = 1 along the
+    // diagonal block).
     __device__ __forceinline__ void near_weights(double sq, bool self, double& om1, double& om2) const {
         sq = fmax(sq, 1.0e-12);
         const double rho = rsqrt_refined(sq);
-        om1 = self ? 1.0 : fma(-c3, sq * rho, 1.0);
-        om2 = self ? 0.0 : c7 * rho;
+        if (sq >= far2) {
+            far_weights(sq, om1, om2);
+        } else {
+            om1 = fma(-c3, sq * rho, 1.0);
+            om2 = c7 * rho;
+        }
+        if (self) om1 = 1.0, om2 = 0.0;
     }
     __device__ __forceinline__ void weights(double sq, bool self, double& om1, double& om2) const {
         far_weights(sq, om1, om2);
-        if (!(sq >= far2)) near_weights(sq, self, om1, om2);
+        if (!(sq >= near2)) near_weights(sq, self, om1, om2);
     }
 };
 

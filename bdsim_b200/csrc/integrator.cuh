@@ -82,8 +82,9 @@ __host__ __device__ inline SmemLayout smem_layout(int n_max, int d_in_smem, int 
 // bulk copies of the blocked factorisation need 16-byte alignment).
 __host__ __device__ inline int chol_ld(int n) { return (n + 15) / 16 * 16; }
 
-// Global scratch per thread block (doubles): dense D when it is not in shared
-// memory (plain form), the Cholesky factor, and the cold Lanczos basis.
+// Global scratch per thread block (doubles): the Cholesky factor and the cold
+// Lanczos basis. The room for a dense D is kept where need_d asks for it: the
+// static-scratch entry point states its limit with it.
 struct ScratchLayout {
     int64_t D, Lt, V, total;
 };

@@ -1,6 +1,5 @@
 // plan.h -- which kernel and launch shape a chain gets: shared by bdcu_run's
-// launch plans (api.cu) and the static-scratch entry point (static_scratch.cu),
-// so that both run every chain on the same kernel.
+// launch plans (api.cu) and the static-scratch entry point (static_scratch.cu).
 #pragma once
 
 #include <algorithm>

@@ -4,7 +4,9 @@
 // Some callers cannot call cudaMalloc: a host application whose memory pool
 // already owns all of the GPU's memory, or a serving loop that must never take
 // the implicit device-wide synchronisation cudaMalloc/cudaFree imply. For them
-// this entry point runs the same kernels as bdcu_run, bucket by bucket, but
+// this entry point runs bdcu_run's buckets one by one (the mixed form on the same
+// kernels, the plain form on the general block kernel, whose scratch its limit is
+// stated for), but
 // every device buffer it needs beyond the caller's inputs and outputs -- the
 // chain parameter records, the work lists, the parameter arena, the Lanczos
 // seed table, the RNG jump-ahead tables, the work queue counters and the

@@ -138,7 +138,7 @@ class Context:
 
     def autotune(self, form, R, rng, cache, cache_valid, t_start, probe_steps: int = 3) -> list:
         """Time every launch shape of each bucket (block kernel: block size,
-        Lanczos vectors and D in shared memory; team kernel: warps per chain
+        Lanczos vectors in shared memory; team kernel: warps per chain
         x beads per thread) on copies of the given state and keep the
         fastest; returns the tuned plan. Probe from a warmed-up state (valid
         warm-start cache): probes from a cold cache are dominated by the

@@ -279,7 +279,10 @@ int bdcu_ran1(bdcu_ctx* ctx, int n_chains, int32_t* rng, int n_per_chain, double
    beads (and no Cholesky method) runs on the team kernel in buckets 0..3 (N <=
    64, 128, 256, 512), by default with (warps per chain, beads per thread) =
    (2,1), (4,1), (4,2), (8,2) unless tuned or pinned; every other chain runs one chain per
-   thread block, in buckets 4..7 split at N = 64, 128 and 256. Once a plan is
+   thread block, in buckets 4..7 split at N = 64, 128 and 256. (The plain form
+   runs its Chebyshev chains of N <= 512 and its Cholesky chains of N <= 64 on a
+   kernel of their own; a plan then names a bucket twice where it holds chains
+   of both kinds.) Once a plan is
    built (first bdcu_run after a change of records, selection or form) a
    bdcu_run enqueues only a memset, event records/waits and kernel launches,
    so it may be captured in a CUDA graph. */
@@ -295,7 +298,7 @@ typedef struct bdcu_bucket_info {
     int32_t block;       /* threads per block */
     int32_t grid;        /* persistent blocks */
     int32_t v_cap;       /* Lanczos basis vectors kept in shared memory */
-    int32_t d_in_smem;   /* dense D in shared memory (plain form) */
+    int32_t d_in_smem;   /* 0 (no launch keeps a dense D) */
     int32_t tuned;       /* 1: shape chosen by bdcu_autotune */
     int32_t team_beads_per_thread;  /* team kernel: 1 or 2 beads per thread (0 for the block kernel) */
     int64_t smem_bytes;  /* dynamic shared memory per block */
@@ -308,7 +311,7 @@ int bdcu_describe_plan(bdcu_ctx* ctx, int form, bdcu_bucket_info* out, int cap, 
    probe_steps steps on device copies of the given state -- the caller's buffers
    are read, never written -- and keep the fastest shape per (form, bucket) for
    later bdcu_run calls. Block-kernel buckets: threads per block x Lanczos
-   vectors in shared memory x, in the plain form, D in shared memory.
+   vectors in shared memory (plain form up to N = 512: threads per block).
    Team-kernel buckets (FP32-mixed form): warps per team x beads per thread,
    every compiled team shape that holds any chain of the bucket, up to twice
    its width. No
@@ -371,7 +374,8 @@ int bdcu_check_chains(int n_chains, const bdcu_phys* phys, const bdcu_sim* sim, 
    already owns the GPU's memory, or a serving loop that must not take the
    implicit device-wide synchronisation cudaMalloc/cudaFree imply. This entry
    point takes the parameters on the host (as bdcu_set_chains does) and runs
-   the same kernels as bdcu_run (its buckets, one after another) on the
+   bdcu_run's buckets one after another (the mixed form on the same kernels, the
+   plain form on the general block kernel: the same results to rounding) on the
    caller's device buffers; the parameter records, work lists, arena, work
    counters and per-block scratch live in one
    file-scope device array of BDCU_STATIC_SCRATCH_BYTES that every GPU using

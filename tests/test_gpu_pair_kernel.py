@@ -124,3 +124,13 @@ def test_warm_vector_of_any_length(port):
     ens.cache_valid.fill_(1)
     ens.advance(0.0, 1, _abi.CACHE_PERSIST)
     assert rel(ens.positions()[0], want) <= CALL_TOL
+
+
+@pytest.mark.parametrize("method", [DelSMethod.Chebyshev, DelSMethod.Cholesky])
+def test_coincident_beads_at_small_hstar(port, method):
+    """Two beads in one place: their separation is clamped to 1e-6, which at
+    h* = 1e-8 is a far pair."""
+    p, s, R0 = chain("gauss", 9, 4)
+    R0[6] = R0[2]
+    p.hstar, p.hi_method = 1e-8, method
+    against_oracle(port, p, s, R0, 8, 1, "plain")
