@@ -447,6 +447,14 @@ struct RpyConst {
         c7 = 0.09375 / rpi / h;
         far2 = (2.0 * rpi * h) * (2.0 * rpi * h);
         near2 = fmax(far2, 1.0e-12);
+        if (far2 < 1.0e-12) {
+            // an h* below 3e-7: separations under the reference's clamp of 1e-6
+            // are far pairs at 1e-6. The near formulas, evaluated at the clamp,
+            // are given constants that return those weights.
+            const double t = 1.0e12;
+            c3 = (1.0 - 1.0e6 * fma(A3, t, A1)) * 1.0e6;
+            c7 = t * fma(-B3, t, A1);
+        }
     }
     // Far pairs (all but neighbours along the chain and close contacts).
     __device__ __forceinline__ void far_weights(double sq, double& om1, double& om2) const {
@@ -454,19 +462,13 @@ struct RpyConst {
         om1 = rho * fma(A3, t, A1);
         om2 = (rho * t) * fma(-B3, t, A1);
     }
-    // Near pairs, separations below the reference's clamp (which an h* below
-    // 3e-7 can make far ones), and a bead with itself (omega1 = 1 along the
-    // diagonal block).
+    // Near pairs, separations below the clamp, and a bead with itself (omega1 =
+    // 1 along the diagonal block).
     __device__ __forceinline__ void near_weights(double sq, bool self, double& om1, double& om2) const {
         sq = fmax(sq, 1.0e-12);
         const double rho = rsqrt_refined(sq);
-        if (sq >= far2) {
-            far_weights(sq, om1, om2);
-        } else {
-            om1 = fma(-c3, sq * rho, 1.0);
-            om2 = c7 * rho;
-        }
-        if (self) om1 = 1.0, om2 = 0.0;
+        om1 = self ? 1.0 : fma(-c3, sq * rho, 1.0);
+        om2 = self ? 0.0 : c7 * rho;
     }
     __device__ __forceinline__ void weights(double sq, bool self, double& om1, double& om2) const {
         far_weights(sq, om1, om2);
