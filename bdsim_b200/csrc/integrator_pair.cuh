@@ -685,7 +685,7 @@ struct PairChain {
     // tests the eigenvalues agree with the reference's scheme to 2e-14, the
     // basis is orthogonal to 1e-11. (Projecting in every step read the basis from
     // L2 twice a step: 12.9 thousand cycles a step at N = 50, 2.7 of them the
-    // product; now 8.0.) Returns its steps; the tridiagonal is left in alpha and
+    // product; now 6.6.) Returns its steps; the tridiagonal is left in alpha and
     // beta.
     __device__ __forceinline__ int lanczos(double* V, bool cold, double (&v)[3], double (&w)[3], bool have_w) {
         const int m = min(n, cold ? kLanczosCold : kLanczosWarm);
