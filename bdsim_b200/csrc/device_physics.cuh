@@ -283,18 +283,21 @@ __device__ __forceinline__ double ev_outer_cutoff(const DevChain& c) {
 // lj_factor / sdk_factor (src/excluded_volume.cpp:42-58) at squared distance sq,
 // with the 14th and 8th powers of r as products of 1/r^2 (the library's pow()
 // costs a hundred operations each). phi: the pair's attractive strength (null:
-// zero). gauss_factor is written out in the pair loops.
+// zero). The SDK attraction acts on every Rcutg < r <= RcutpSDK, below Rmin too
+// (Rmin lies above Rcutg for dstar < 0.62 at the default min_cutoff).
+// gauss_factor is written out in the pair loops.
 __device__ inline double ev_factor_short(const DevChain& c, double sq, const double* phi) {
     const double r = sqrt(sq);
     const bool sdk = c.ev_type == BDCU_EV_SDK;
-    if (r < c.Rmin) return sdk ? c.sdk_rmin_fac : c.lj_rmin_fac;
     double fac = 0.0;
-    if (r <= (sdk || c.equil ? c.Rcutg : c.Rcutp)) {
+    if (r < c.Rmin) {
+        fac = sdk ? c.sdk_rmin_fac : c.lj_rmin_fac;
+    } else if (r <= (sdk || c.equil ? c.Rcutg : c.Rcutp)) {
         const double i2 = 1.0 / sq, i4 = i2 * i2, i8 = i4 * i4;
         fac = (sdk ? c.SDKa : c.LJa) * ((i8 * i4) * i2) - (sdk ? c.SDKb : c.LJb) * i8;
-    } else if (sdk && !c.equil && r <= c.RcutpSDK && phi) {
-        fac = 1.530633312 * *phi * sin(1.530633312 * sq + 1.213115524);
     }
+    if (sdk && !c.equil && r > c.Rcutg && r <= c.RcutpSDK && phi)
+        fac += 1.530633312 * *phi * sin(1.530633312 * sq + 1.213115524);
     return fac;
 }
 
