@@ -297,20 +297,13 @@ std::vector<Shape> block_shapes(const bdcu_ctx* ctx, const Bucket& b, int form) 
     return out;
 }
 
-// Warps per chain of the pair kernel that hold a chain of `beads`, the
-// bucket's default first.
-std::vector<Shape> pair_shapes(int id, int beads) {
-    std::vector<Shape> out;
-    auto add = [&](int T) {
-        if (32 * T < beads) return;
-        Shape s;
-        s.block = 32 * T;
-        out.push_back(s);
-    };
-    add(kDefaultPairWarps[id]);
-    for (int T : kPairWarps)
-        if (T != kDefaultPairWarps[id] && 32 * T <= 4 * kBucketBeads[id]) add(T);
-    return out;
+// The pair kernel's one shape for a bucket: its sums run in the order of the
+// lanes per bead and the warps, so that a chain's result does not depend on the
+// launch it is in the warps follow from the chain alone (not from a timing).
+Shape pair_shape(int id) {
+    Shape s;
+    s.block = 32 * kPairWarps[id];
+    return s;
 }
 
 // Fill the launch fields of a bucket for a shape (block or pair kernel) or for
@@ -348,7 +341,7 @@ int fill_launch(bdcu_ctx* ctx, int form, Bucket& b, const Shape* s) {
         if (b.chol_beads > 0) b.w_pairs = std::max(b.w_pairs, (pair_factor_doubles(b.chol_beads) + 1) / 2);
         b.smem = (size_t)pair_layout(b.n_max, T, b.w_pairs).total * sizeof(double);
         if (b.smem > ctx->max_smem) return fail(ctx, BDCU_E_LIMIT, "chain too large for the shared-memory layout");
-        auto& occ = ctx->pair_occ[T == 2 ? 0 : T == 4 ? 1 : T == 8 ? 2 : 3];
+        auto& occ = ctx->pair_occ[T == 4 ? 0 : T == 8 ? 1 : 2];
         if (occ.smem != b.smem) {
             e = occupancy_pair(T, b.smem, &occ.per_sm);
             if (e != cudaSuccess) return cuda_fail(ctx, e, "occupancy_pair");
@@ -455,11 +448,9 @@ int build_plan(bdcu_ctx* ctx, int form) {
             if ((rc = fill_launch(ctx, form, b, use ? &t : nullptr))) return rc;
             b.tuned = use ? 1 : 0;
         } else if (b.kernel == kKernelPair) {
-            const Shape& t = ctx->tuned[mixed][id];
-            const bool use = t.block > 0 && t.block >= b.max_beads;
-            const Shape pick = use ? t : pair_shapes(id, b.max_beads).front();
+            const Shape pick = pair_shape(id);
             if ((rc = fill_launch(ctx, form, b, &pick))) return rc;
-            b.tuned = use ? 1 : 0;
+            b.tuned = ctx->tuned[mixed][id].block > 0 ? 1 : 0;
         } else {
             const std::vector<Shape> shapes = block_shapes(ctx, b, form);
             if (shapes.empty()) return fail(ctx, BDCU_E_LIMIT, "chain too large for the shared-memory layout");
@@ -853,10 +844,12 @@ int bdcu_autotune(bdcu_ctx* ctx, int form, const double* R, const int32_t* rng, 
         float best_ms = 1e30f;
         Shape best;
         std::vector<Shape> shapes;
+        if (base.kernel == kKernelPair) {  // one shape: nothing to time
+            ctx->tuned[mixed][base.id] = pair_shape(base.id);
+            continue;
+        }
         if (base.kernel == BDCU_KERNEL_BLOCK) {
             shapes = block_shapes(ctx, base, form);
-        } else if (base.kernel == kKernelPair) {
-            shapes = pair_shapes(base.id, base.max_beads);
         } else {
             // team shapes that hold any chain of the bucket, up to twice its width
             for (int i = 0; i < kNumTeamShapes; ++i) {

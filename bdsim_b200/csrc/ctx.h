@@ -27,8 +27,8 @@ constexpr int kKernelPair = 2;  // Bucket::kernel of the pair kernel (BDCU_KERNE
 constexpr int kBucketBeads[kMaxBuckets] = {64, 128, 256, 512, 64, 128, 256, kMaxBeads};
 
 // A launch shape chosen by bdcu_autotune. Block kernel: threads per block,
-// Lanczos vectors in shared memory (pair kernel: threads only). Team kernel:
-// warps per team and beads per thread.
+// Lanczos vectors in shared memory. Team kernel: warps per team and beads per
+// thread. (The pair kernel has one shape per bucket.)
 struct Shape {
     int block = 0;  // 0: not tuned
     int v_cap = -1;
@@ -95,8 +95,8 @@ struct bdcu_ctx {
     int bounds_every = 1;  // bdcu_set_bounds_refresh
     int single_launch = 0; // bdcu_set_single_launch: every team-kernel chain in one launch
     size_t max_smem = 0;
-    // the pair kernel's last occupancy query per warp count (2, 4, 8, 16)
-    struct { size_t smem = 0; int per_sm = 0; } pair_occ[4];
+    // the pair kernel's last occupancy query per warp count (4, 8, 16)
+    struct { size_t smem = 0; int per_sm = 0; } pair_occ[3];
     // the chains bdcu_run advances: all records (sel_all) or a list (bdcu_select)
     int sel_all = 1;
     std::vector<int32_t> sel;

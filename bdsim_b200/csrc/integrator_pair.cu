@@ -24,7 +24,6 @@ static cudaError_t launch_pair_t(const RunArgs& a, int grid, size_t smem, cudaSt
 
 cudaError_t launch_pair(int warps, const RunArgs& a, int grid, size_t smem, cudaStream_t s) {
     switch (warps) {
-        case 2: return launch_pair_t<2>(a, grid, smem, s);
         case 4: return launch_pair_t<4>(a, grid, smem, s);
         case 8: return launch_pair_t<8>(a, grid, smem, s);
         case 16: return launch_pair_t<16>(a, grid, smem, s);
@@ -34,7 +33,6 @@ cudaError_t launch_pair(int warps, const RunArgs& a, int grid, size_t smem, cuda
 
 cudaError_t occupancy_pair(int warps, size_t smem, int* per_sm) {
     switch (warps) {
-        case 2: return occupancy_pair_t<2>(smem, per_sm);
         case 4: return occupancy_pair_t<4>(smem, per_sm);
         case 8: return occupancy_pair_t<8>(smem, per_sm);
         case 16: return occupancy_pair_t<16>(smem, per_sm);

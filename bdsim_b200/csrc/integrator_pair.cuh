@@ -165,7 +165,7 @@ struct PairChain {
     // the eight published at r (one load per four warps, two shuffles).
     __device__ __forceinline__ double total8(const double* r) const {
         const double* q = r + (wl & 7) * T + (wl >> 3);
-        double t = T >= 4 || (wl >> 3) < T ? q[0] : 0.0;
+        double t = q[0];
 #pragma unroll
         for (int w = 4; w < T; w += 4) t += q[w];
         t += __shfl_xor_sync(kFull, t, 8);

@@ -17,12 +17,10 @@ __host__ __device__ inline int64_t pair_factor_doubles(int N) { return 9 * (int6
 
 // Blocks per SM a shape's registers and shared memory are sized for. 12 to 16
 // warps per SM: 168 registers per thread at T = 4, 128 at T = 8 and 16.
-__host__ __device__ constexpr int pair_min_blocks(int T) { return T == 2 ? 6 : T == 4 ? 3 : T == 8 ? 2 : 1; }
+__host__ __device__ constexpr int pair_min_blocks(int T) { return T == 4 ? 3 : T == 8 ? 2 : 1; }
 
-// Default warps per chain of buckets 0..3 (N <= 64, 128, 256, 512).
-constexpr int kDefaultPairWarps[4] = {4, 8, 8, 16};
-constexpr int kNumPairShapes = 4;
-constexpr int kPairWarps[kNumPairShapes] = {2, 4, 8, 16};
+// Warps per chain of buckets 0..3 (N <= 64, 128, 256, 512).
+constexpr int kPairWarps[4] = {4, 8, 8, 16};
 
 struct PairLayout {
     int64_t chain, red, alpha, beta, ymin, ymax, tot, ctl, jcols, ps, pq, xs, buf, s3, s4, seed, area, w, total;  // in doubles

@@ -311,14 +311,14 @@ int bdcu_describe_plan(bdcu_ctx* ctx, int form, bdcu_bucket_info* out, int cap, 
    probe_steps steps on device copies of the given state -- the caller's buffers
    are read, never written -- and keep the fastest shape per (form, bucket) for
    later bdcu_run calls. Block-kernel buckets: threads per block x Lanczos
-   vectors in shared memory (plain form up to N = 512: threads per block).
+   vectors in shared memory, which leaves a chain's result bit for bit as it was
+   (the plain form's own kernel has one shape per bucket: nothing is timed).
    Team-kernel buckets (FP32-mixed form): warps per team x beads per thread,
    every compiled team shape that holds any chain of the bucket, up to twice
    its width. No
    counterpart in the reference (one chain per call on the CPU). Synchronous;
-   allocates and frees its copies. The shape changes only the speed and,
-   through the order of block and team reductions, the rounding of the
-   Lanczos and Chebyshev dot products. */
+   allocates and frees its copies. A shape changes only the speed and, on the
+   team kernel, the order of the team reductions (rounding). */
 int bdcu_autotune(bdcu_ctx* ctx, int form, const double* R, const int32_t* rng, const double* cache,
                   const int32_t* cache_valid, const double* t_start, int probe_steps);
 
