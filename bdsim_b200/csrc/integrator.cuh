@@ -463,10 +463,13 @@ struct Block {
 
     // Column-block width of the blocked factorisation (0: unblocked): up to
     // kCholMaxBlock columns, a multiple of 8, such that two staged tiles of
-    // panel rows fit the staging area.
+    // panel rows fit the staging area of a launch of such chains alone: the
+    // width sets the order of the trailing products, so it follows from the
+    // chain, not from the largest chain of its launch (whose staging area is
+    // at least as large).
     __device__ int chol_panel_width() const {
         if (n < kBlockedCholMin || stage == nullptr) return 0;
-        int64_t nb = stage_cap / (2 * kCholTileStride);
+        int64_t nb = (kSlots - kCholFirstSlot) * round_up8(n) / (2 * kCholTileStride);
         nb = nb > kCholMaxBlock ? kCholMaxBlock : nb;
         nb &= ~7;
         return nb >= 8 ? (int)nb : 0;

@@ -29,3 +29,22 @@ def test_autotune_changes_no_result(N, copies, method):
         ens.advance(0.0, 2, _abi.CACHE_RESET_PER_CALL)
         ends.append(ens.R.cpu().numpy())
     assert np.array_equal(ends[0], ends[1])
+
+
+@pytest.mark.parametrize("form", ["plain", "mixed"])
+@pytest.mark.parametrize("N,other", [(66, 128), (101, 127), (110, 128), (150, 250), (258, 500)])
+def test_cholesky_does_not_depend_on_the_other_chains(form, N, other):
+    """The blocked factorisation (3N >= 300) among longer chains of its bucket."""
+    ends = []
+    for Ns in ([N], [other, N, other]):
+        phys, sims, R0 = [], [], []
+        for n in Ns:
+            p, s = workloads.batched_cheb_phys(n)
+            p.hi_method = DelSMethod.Cholesky
+            phys.append(p)
+            sims.append(s)
+            R0.append(B.gaussian_chain(n, bond_std=1.0, seed=n))
+        ens = B.Ensemble(phys, sims, R0, [(1, -1, n) for n in Ns], form=form)
+        ens.advance(0.0, 2, _abi.CACHE_RESET_PER_CALL)
+        ends.append(ens.positions()[Ns.index(N)])
+    assert np.array_equal(ends[0], ends[1])
