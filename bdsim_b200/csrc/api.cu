@@ -302,7 +302,7 @@ std::vector<Shape> block_shapes(const bdcu_ctx* ctx, const Bucket& b, int form) 
 // launch it is in the warps follow from the chain alone (not from a timing).
 Shape pair_shape(int id) {
     Shape s;
-    s.block = 32 * kPairWarps[id];
+    s.block = 32 * (id == kPairCholBucket ? kPairCholWarps : kPairWarps[id]);
     return s;
 }
 
@@ -337,8 +337,8 @@ int fill_launch(bdcu_ctx* ctx, int form, Bucket& b, const Shape* s) {
         const int T = s->block / 32;
         b.block = s->block;
         b.v_cap = b.d_in_smem = 0;
-        b.w_pairs = b.need_lz ? pair_cached(b.n_max, T, b.count, ctx->sm_count, ctx->max_smem) : 0;
-        if (b.chol_beads > 0) b.w_pairs = std::max(b.w_pairs, (pair_factor_doubles(b.chol_beads) + 1) / 2);
+        if (b.id == kPairCholBucket) b.w_pairs = (pair_factor_doubles(b.max_beads) + 1) / 2;
+        else b.w_pairs = b.need_lz ? pair_cached(b.n_max, T, b.count, ctx->sm_count, ctx->max_smem) : 0;
         b.smem = (size_t)pair_layout(b.n_max, T, b.w_pairs).total * sizeof(double);
         if (b.smem > ctx->max_smem) return fail(ctx, BDCU_E_LIMIT, "chain too large for the shared-memory layout");
         auto& occ = ctx->pair_occ[T == 4 ? 0 : T == 8 ? 1 : 2];
@@ -415,16 +415,14 @@ int build_plan(bdcu_ctx* ctx, int form) {
     ctx->plan.clear();
     ctx->order_h.clear();
     int rc;
-    // largest chains' buckets are launched first: the block kernel's, then the
-    // team kernel's from the widest team down
-    for (int id = kMaxBuckets - 1; id >= 0; --id) {
+    for (int id : kBucketOrder) {
         std::vector<int32_t>& L = lists[id];
         if (L.empty()) continue;
         std::stable_sort(L.begin(), L.end(),
                          [&](int32_t x, int32_t y) { return ctx->chains_h[x].N > ctx->chains_h[y].N; });
         Bucket b;
         b.id = id;
-        b.kernel = id >= kFirstBlockBucket ? BDCU_KERNEL_BLOCK : mixed ? BDCU_KERNEL_TEAM : kKernelPair;
+        b.kernel = bucket_kernel(id, form);
         b.team_warps = b.kernel == BDCU_KERNEL_TEAM ? kDefaultTeamShape[id][0] : 0;
         b.team_q = b.kernel == BDCU_KERNEL_TEAM ? kDefaultTeamShape[id][1] : 0;
         b.count = (int)L.size();
@@ -437,7 +435,6 @@ int build_plan(bdcu_ctx* ctx, int form) {
                 b.need_d = 1;
                 b.need_chol = 1;  // Cholesky method, or the Chebyshev fallback
                 if (ch.hi_method == BDCU_HI_CHEBYSHEV) b.need_lz = 1;
-                if (ch.hi_method == BDCU_HI_CHOLESKY) b.chol_beads = std::max(b.chol_beads, (int)ch.N);
             }
         }
         b.order_off = (int64_t)ctx->order_h.size();
@@ -770,7 +767,8 @@ int bdcu_describe_plan(bdcu_ctx* ctx, int form, bdcu_bucket_info* out, int cap, 
     for (int i = 0; i < cap && i < (int)ctx->plan.size(); ++i) {
         const Bucket& b = ctx->plan[i];
         bdcu_bucket_info& o = out[i];
-        o.bucket = b.kernel == kKernelPair ? b.id + kFirstBlockBucket : b.id;
+        o.bucket = b.id == kPairCholBucket ? kFirstBlockBucket
+                   : b.kernel == kKernelPair ? b.id + kFirstBlockBucket : b.id;
         o.kernel = b.kernel == kKernelPair ? (int)BDCU_KERNEL_BLOCK : b.kernel;
         o.team_warps = b.team_warps;
         o.team_beads_per_thread = b.team_q;

@@ -17,14 +17,20 @@ namespace bdcu {
 
 // Buckets of a launch plan. Buckets 0..3 hold the chains of N <= 64, 128, 256
 // and 512 beads that do not use the Cholesky method: the team kernel in the
-// FP32-mixed form, the pair kernel (one chain per block, reported as block
-// buckets 4..7) in the plain form, which takes Cholesky chains of N <= 64 too.
+// FP32-mixed form, the pair kernel (one chain per block) in the plain form.
 // Buckets 4..7 run one chain per block on the general block kernel and split the
-// rest by bead count at 64, 128 and 256.
-constexpr int kMaxBuckets = 8;
+// rest by bead count at 64, 128 and 256. Bucket 8: the plain form's Cholesky
+// chains of N <= 64, on the pair kernel in a launch of their own, as their
+// factors take up to 150 KB of shared memory a block (2000 Chebyshev chains of
+// N = 50 and one Cholesky chain of N = 64 in one launch: one block per SM instead
+// of three, 10.3 ms for 10 steps; in two launches 5.4).
+constexpr int kMaxBuckets = 9;
 constexpr int kFirstBlockBucket = 4;
+constexpr int kPairCholBucket = 8;
 constexpr int kKernelPair = 2;  // Bucket::kernel of the pair kernel (BDCU_KERNEL_BLOCK outside)
-constexpr int kBucketBeads[kMaxBuckets] = {64, 128, 256, 512, 64, 128, 256, kMaxBeads};
+constexpr int kBucketBeads[kMaxBuckets] = {64, 128, 256, 512, 64, 128, 256, kMaxBeads, 64};
+// the launches of a plan, largest chains first
+constexpr int kBucketOrder[kMaxBuckets] = {7, 6, 5, 4, 3, 2, 1, 8, 0};
 
 // A launch shape chosen by bdcu_autotune. Block kernel: threads per block,
 // Lanczos vectors in shared memory. Team kernel: warps per team and beads per
@@ -45,7 +51,6 @@ struct Bucket {
     int count = 0, min_beads = 0, max_beads = 0;
     int n_max = 0;  // 3 * max_beads
     int need_chol = 0, need_d = 0, need_lz = 0;
-    int chol_beads = 0;  // largest chain of the Cholesky method
     int64_t order_off = 0;  // first entry of this bucket's work list in order_d
     int block = 0, grid = 0, v_cap = 0, d_in_smem = 0, tuned = 0;
     int64_t w_pairs = 0;  // pair and team kernels: cached pair weights (per block, per team)

@@ -19,8 +19,10 @@ __host__ __device__ inline int64_t pair_factor_doubles(int N) { return 9 * (int6
 // warps per SM: 168 registers per thread at T = 4, 128 at T = 8 and 16.
 __host__ __device__ constexpr int pair_min_blocks(int T) { return T == 4 ? 3 : T == 8 ? 2 : 1; }
 
-// Warps per chain of buckets 0..3 (N <= 64, 128, 256, 512).
+// Warps per chain of buckets 0..3 (N <= 64, 128, 256, 512), and of the Cholesky
+// method's.
 constexpr int kPairWarps[4] = {4, 8, 8, 16};
+constexpr int kPairCholWarps = 4;
 
 struct PairLayout {
     int64_t chain, red, alpha, beta, ymin, ymax, tot, ctl, jcols, ps, pq, xs, buf, s3, s4, seed, area, w, total;  // in doubles

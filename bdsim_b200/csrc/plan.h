@@ -15,16 +15,23 @@ namespace bdcu {
 // the block kernel, whose scratch its limit is stated for).
 inline int bucket_of(const DevChain& c, int form, bool pair = true) {
     const bool chol = c.hstar > 0.0 && c.hi_method == BDCU_HI_CHOLESKY;
+    const bool mixed = form == BDCU_FORM_MIXED_FP32;
     static_assert(kPairMaxN == kTeamMaxN, "team and pair buckets share their bead ranges");
-    const bool fits = form == BDCU_FORM_MIXED_FP32 ? !chol && c.N <= kTeamMaxN
-                                                   : pair && c.N <= (chol ? kPairCholMaxN : kPairMaxN);
-    if (fits) {
+    if (!mixed && pair && chol && c.N <= kPairCholMaxN) return kPairCholBucket;
+    if (!chol && c.N <= kTeamMaxN && (mixed || pair)) {
         const int T = team_warps_for(c.N);
         return T == 1 ? 0 : T == 2 ? 1 : T == 4 ? 2 : 3;
     }
-    for (int b = kFirstBlockBucket; b < kMaxBuckets - 1; ++b)
+    for (int b = kFirstBlockBucket; b < 7; ++b)
         if (c.N <= kBucketBeads[b]) return b;
-    return kMaxBuckets - 1;
+    return 7;
+}
+
+// The kernel of a bucket (BDCU_KERNEL_*, kKernelPair).
+inline int bucket_kernel(int id, int form) {
+    if (id == kPairCholBucket) return kKernelPair;
+    if (id >= kFirstBlockBucket) return BDCU_KERNEL_BLOCK;
+    return form == BDCU_FORM_MIXED_FP32 ? (int)BDCU_KERNEL_TEAM : kKernelPair;
 }
 
 #define BDCU_TEAM_SHAPE_SWITCH(T, Q, EXPR, FALLBACK)            \

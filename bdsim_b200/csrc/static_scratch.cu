@@ -153,7 +153,7 @@ extern "C" int bdcu_run_static(bdcu_ctx* ctx, int n_chains, const bdcu_phys* phy
     std::vector<int32_t> order;
     bool any_team = false;
     size_t max_block_scratch = 0;
-    for (int id = kMaxBuckets - 1; id >= 0; --id) {
+    for (int id : kBucketOrder) {
         std::vector<int32_t>& L = lists[id];
         if (L.empty()) continue;
         std::stable_sort(L.begin(), L.end(), [&](int32_t x, int32_t y) { return recs[x].N > recs[y].N; });

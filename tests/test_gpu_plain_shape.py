@@ -48,3 +48,35 @@ def test_cholesky_does_not_depend_on_the_other_chains(form, N, other):
         ens.advance(0.0, 2, _abi.CACHE_RESET_PER_CALL)
         ends.append(ens.positions()[Ns.index(N)])
     assert np.array_equal(ends[0], ends[1])
+
+
+def both_methods(specs):
+    """One plain ensemble of (N, method, copies) groups."""
+    phys, sims, R0 = [], [], []
+    for N, method, copies in specs:
+        p, s = workloads.batched_cheb_phys(N)
+        p.hi_method = method
+        phys += [p] * copies
+        sims += [s] * copies
+        R0 += [B.gaussian_chain(N, bond_std=1.0, seed=100 * N + i) for i in range(copies)]
+    return B.Ensemble(phys, sims, R0, [(1, -1, 5 + i) for i in range(len(R0))], form="plain")
+
+
+def test_a_cholesky_chain_leaves_the_chebyshev_launch_as_it_was():
+    """A Cholesky chain of N <= 64 keeps its factor in shared memory, which its
+    Chebyshev neighbours do not pay for."""
+    cheb, chol = DelSMethod.Chebyshev, DelSMethod.Cholesky
+    alone = both_methods([(50, cheb, 500)])
+    mixed = both_methods([(50, cheb, 500), (64, chol, 1)])
+    want = alone.plan()[0]
+    got = [b for b in mixed.plan() if b["n_chains"] == 500]
+    assert len(got) == 1
+    for k in ("block", "grid", "smem_bytes", "max_beads"):
+        assert got[0][k] == want[k], k
+    one = both_methods([(64, chol, 1)])
+    one.rng.copy_(mixed.rng[500:])
+    for ens in (alone, mixed, one):
+        ens.advance(0.0, 2, _abi.CACHE_RESET_PER_CALL)
+    end = mixed.positions()
+    assert all(np.array_equal(a, b) for a, b in zip(end, alone.positions()))
+    assert np.array_equal(end[500], one.positions()[0])
