@@ -763,12 +763,27 @@ int bdcu_describe_plan(bdcu_ctx* ctx, int form, bdcu_bucket_info* out, int cap, 
     CK(cudaSetDevice(ctx->device));
     int rc = build_plan(ctx, form);
     if (rc) return rc;
-    *n_out = (int)ctx->plan.size();
-    for (int i = 0; i < cap && i < (int)ctx->plan.size(); ++i) {
+    const int nb = (int)ctx->plan.size();
+    *n_out = nb;
+    // one chain per block: listed as 4 + its size class; where a class has more
+    // than one launch (the plain form runs the Cholesky method apart), the one
+    // without the Cholesky method keeps that id and each further one is four higher
+    std::vector<int> ids(nb, -1);
+    auto taken = [&](int id) { return std::find(ids.begin(), ids.end(), id) != ids.end(); };
+    for (int i = 0; i < nb; ++i) {
+        const Bucket& b = ctx->plan[i];
+        if (b.id < kFirstBlockBucket) ids[i] = b.kernel == kKernelPair ? b.id + kFirstBlockBucket : b.id;
+    }
+    for (int i = 0; i < nb; ++i)
+        if (ids[i] < 0) {
+            int id = ctx->plan[i].id == kPairCholBucket ? kFirstBlockBucket : ctx->plan[i].id;
+            while (taken(id)) id += 4;
+            ids[i] = id;
+        }
+    for (int i = 0; i < cap && i < nb; ++i) {
         const Bucket& b = ctx->plan[i];
         bdcu_bucket_info& o = out[i];
-        o.bucket = b.id == kPairCholBucket ? kFirstBlockBucket
-                   : b.kernel == kKernelPair ? b.id + kFirstBlockBucket : b.id;
+        o.bucket = ids[i];
         o.kernel = b.kernel == kKernelPair ? (int)BDCU_KERNEL_BLOCK : b.kernel;
         o.team_warps = b.team_warps;
         o.team_beads_per_thread = b.team_q;

@@ -280,17 +280,17 @@ int bdcu_ran1(bdcu_ctx* ctx, int n_chains, int32_t* rng, int n_per_chain, double
    64, 128, 256, 512), by default with (warps per chain, beads per thread) =
    (2,1), (4,1), (4,2), (8,2) unless tuned or pinned; every other chain runs one chain per
    thread block, in buckets 4..7 split at N = 64, 128 and 256. (The plain form
-   runs its Chebyshev chains of N <= 512 and its Cholesky chains of N <= 64 on a
-   kernel of their own; a plan then names a bucket twice where it holds chains
-   of both kinds.) Once a plan is
+   launches its Cholesky chains, and any chain of N > 512, apart from the other
+   chains of their size: such a launch has the id of its size where no other
+   does, else 8..11. A plan names no bucket twice.) Once a plan is
    built (first bdcu_run after a change of records, selection or form) a
    bdcu_run enqueues only a memset, event records/waits and kernel launches,
    so it may be captured in a CUDA graph. */
 enum { BDCU_KERNEL_BLOCK = 0, BDCU_KERNEL_TEAM = 1 };
 #define BDCU_MAX_BUCKETS 8
 typedef struct bdcu_bucket_info {
-    int32_t bucket;      /* 0..3: team kernel; 4..7: block kernel */
-    int32_t kernel;      /* BDCU_KERNEL_* */
+    int32_t bucket;      /* 0..3: team kernel; 4 and up: one chain per block */
+    int32_t kernel;      /* BDCU_KERNEL_*: a team of warps, or a block, per chain */
     int32_t team_warps;  /* team kernel: warps per chain (0 for the block kernel) */
     int32_t n_chains;    /* chains in the bucket */
     int32_t min_beads;

@@ -80,3 +80,18 @@ def test_a_cholesky_chain_leaves_the_chebyshev_launch_as_it_was():
     end = mixed.positions()
     assert all(np.array_equal(a, b) for a, b in zip(end, alone.positions()))
     assert np.array_equal(end[500], one.positions()[0])
+
+
+def test_a_plan_names_each_bucket_once():
+    """The plain form launches both methods apart in every size class."""
+    cheb, chol = DelSMethod.Chebyshev, DelSMethod.Cholesky
+    groups = [(N, m, k) for k, N in enumerate((20, 100, 200, 300, 400), 1) for m in (cheb, chol)] + [(520, cheb, 1)]
+    plan = both_methods(groups).plan()
+    by_id = {b["bucket"]: b for b in plan}
+    assert len(by_id) == len(plan) == 8
+    assert sum(b["n_chains"] for b in plan) == sum(g[2] for g in groups)
+    # the chains without the Cholesky method keep the ids of a plan without it
+    for b in both_methods([g for g in groups if g[1] == cheb and g[0] <= 512]).plan():
+        for k in ("n_chains", "min_beads", "max_beads", "block"):
+            assert by_id[b["bucket"]][k] == b[k], (b["bucket"], k)
+    assert sorted(b["bucket"] for b in both_methods([g for g in groups if g[1] == chol]).plan()) == [4, 5, 6, 7]
