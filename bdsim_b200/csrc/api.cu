@@ -297,12 +297,9 @@ std::vector<Shape> block_shapes(const bdcu_ctx* ctx, const Bucket& b, int form) 
     return out;
 }
 
-// The pair kernel's one shape for a bucket: its sums run in the order of the
-// lanes per bead and the warps, so that a chain's result does not depend on the
-// launch it is in the warps follow from the chain alone (not from a timing).
 Shape pair_shape(int id) {
     Shape s;
-    s.block = 32 * (id == kPairCholBucket ? kPairCholWarps : kPairWarps[id]);
+    s.block = 32 * pair_warps(id);
     return s;
 }
 
@@ -337,8 +334,7 @@ int fill_launch(bdcu_ctx* ctx, int form, Bucket& b, const Shape* s) {
         const int T = s->block / 32;
         b.block = s->block;
         b.v_cap = b.d_in_smem = 0;
-        if (b.id == kPairCholBucket) b.w_pairs = (pair_factor_doubles(b.max_beads) + 1) / 2;
-        else b.w_pairs = b.need_lz ? pair_cached(b.n_max, T, b.count, ctx->sm_count, ctx->max_smem) : 0;
+        b.w_pairs = pair_shared(b.id, b.n_max, b.need_lz, b.count, ctx->sm_count, ctx->max_smem);
         b.smem = (size_t)pair_layout(b.n_max, T, b.w_pairs).total * sizeof(double);
         if (b.smem > ctx->max_smem) return fail(ctx, BDCU_E_LIMIT, "chain too large for the shared-memory layout");
         auto& occ = ctx->pair_occ[T == 4 ? 0 : T == 8 ? 1 : 2];

@@ -1,5 +1,6 @@
 // plan.h -- which kernel and launch shape a chain gets: shared by bdcu_run's
-// launch plans (api.cu) and the static-scratch entry point (static_scratch.cu).
+// launch plans (api.cu) and the static-scratch entry point (static_scratch.cu),
+// so that both run every chain on the same kernel.
 #pragma once
 
 #include <algorithm>
@@ -11,8 +12,8 @@
 namespace bdcu {
 
 // Bucket of a chain for `form` (bucket ids as in ctx.h). pair: whether the
-// plain form's pair kernel may be used (the static-scratch entry point keeps
-// the block kernel, whose scratch its limit is stated for).
+// plain form's pair kernel may be used (the static-scratch entry point goes
+// without where its array does not hold the pair kernel's scratch).
 inline int bucket_of(const DevChain& c, int form, bool pair = true) {
     const bool chol = c.hstar > 0.0 && c.hi_method == BDCU_HI_CHOLESKY;
     const bool mixed = form == BDCU_FORM_MIXED_FP32;
@@ -32,6 +33,18 @@ inline int bucket_kernel(int id, int form) {
     if (id == kPairCholBucket) return kKernelPair;
     if (id >= kFirstBlockBucket) return BDCU_KERNEL_BLOCK;
     return form == BDCU_FORM_MIXED_FP32 ? (int)BDCU_KERNEL_TEAM : kKernelPair;
+}
+
+// The pair kernel's one shape for a bucket: its sums run in the order of the
+// lanes per bead and the warps, so that a chain's result does not depend on the
+// launch it is in the warps follow from the chain alone (not from a timing).
+inline int pair_warps(int id) { return id == kPairCholBucket ? kPairCholWarps : kPairWarps[id]; }
+
+// Pair weights in shared memory (16 bytes each) of a block of a pair bucket's
+// launch over `chains` chains; a Cholesky bucket's factor takes their place.
+inline int64_t pair_shared(int id, int n_max, bool need_lz, int chains, int sm_count, size_t max_smem) {
+    if (id == kPairCholBucket) return (pair_factor_doubles(n_max / 3) + 1) / 2;
+    return need_lz ? pair_cached(n_max, pair_warps(id), chains, sm_count, max_smem) : 0;
 }
 
 #define BDCU_TEAM_SHAPE_SWITCH(T, Q, EXPR, FALLBACK)            \

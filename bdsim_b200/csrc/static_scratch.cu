@@ -4,9 +4,9 @@
 // Some callers cannot call cudaMalloc: a host application whose memory pool
 // already owns all of the GPU's memory, or a serving loop that must never take
 // the implicit device-wide synchronisation cudaMalloc/cudaFree imply. For them
-// this entry point runs bdcu_run's buckets one by one (the mixed form on the same
-// kernels, the plain form on the general block kernel, whose scratch its limit is
-// stated for), but
+// this entry point runs the same kernels as bdcu_run, bucket by bucket (where the
+// array does not hold the pair kernel's scratch beside the parameters, a plain
+// batch runs on the general block kernel, which needs less), but
 // every device buffer it needs beyond the caller's inputs and outputs -- the
 // chain parameter records, the work lists, the parameter arena, the Lanczos
 // seed table, the RNG jump-ahead tables, the work queue counters and the
@@ -44,6 +44,8 @@ cudaError_t occupancy_plain(int block, size_t smem, int* per_sm);
 cudaError_t occupancy_mixed(int block, size_t smem, int* per_sm);
 cudaError_t launch_mixed_team(int team_warps, int team_q, const RunArgs& a, int grid, size_t smem, cudaStream_t s);
 cudaError_t occupancy_mixed_team(int team_warps, int team_q, size_t smem, int* per_sm);
+cudaError_t launch_pair(int warps, const RunArgs& a, int grid, size_t smem, cudaStream_t s);
+cudaError_t occupancy_pair(int warps, size_t smem, int* per_sm);
 DevChain derive_record(const bdcu_phys& p, const bdcu_sim& s, int64_t bead_off);
 int validate_chain(bdcu_ctx* ctx, int i, const bdcu_phys& p, const bdcu_sim& s, const double* arena,
                    int64_t arena_len);
@@ -142,80 +144,129 @@ extern "C" int bdcu_run_static(bdcu_ctx* ctx, int n_chains, const bdcu_phys* phy
 
     // buckets, as bdcu_run plans them (largest chains first within a bucket)
     const int mixed = (form == BDCU_FORM_MIXED_FP32);
-    std::vector<std::vector<int32_t>> lists(kMaxBuckets);
-    for (int i = 0; i < n_chains; ++i) lists[bucket_of(recs[i], form, false)].push_back(i);
     struct Launch {
-        int id, team_warps, team_q, block, grid, v_cap, d_in_smem, n_max, need_d, need_lz, count;
+        int id, kernel, team_warps, team_q, block, grid, v_cap, d_in_smem, n_max, need_d, need_lz, count;
         size_t smem, per_block;
         int64_t stride, order_off, w_pairs;
     };
     std::vector<Launch> launches;
     std::vector<int32_t> order;
-    bool any_team = false;
+    bool jumps = false;  // some launch takes the RNG jump-ahead tables
     size_t max_block_scratch = 0;
-    for (int id : kBucketOrder) {
-        std::vector<int32_t>& L = lists[id];
-        if (L.empty()) continue;
-        std::stable_sort(L.begin(), L.end(), [&](int32_t x, int32_t y) { return recs[x].N > recs[y].N; });
-        Launch l;
-        memset(&l, 0, sizeof(l));
-        l.id = id;
-        l.count = (int)L.size();
-        l.n_max = 3 * recs[L.front()].N;
-        for (int32_t c : L)
-            if (recs[c].hstar > 0.0) {
-                l.need_d = 1;
-                if (recs[c].hi_method == BDCU_HI_CHEBYSHEV) l.need_lz = 1;
-            }
-        l.order_off = (int64_t)order.size();
-        order.insert(order.end(), L.begin(), L.end());
-        int per_sm = 0;
-        if (id < kFirstBlockBucket) {
-            any_team = true;
-            l.team_warps = kDefaultTeamShape[id][0];
-            l.team_q = kDefaultTeamShape[id][1];
-            l.w_pairs = l.need_d ? team_weights(l.team_warps, l.team_q, l.n_max, l.count, ctx->sm_count, ctx->max_smem) : 0;
-            l.smem = (size_t)team_smem(l.team_warps, l.team_q, l.n_max, l.w_pairs);
-            if (l.smem > ctx->max_smem) return fail(ctx, BDCU_E_LIMIT, "bdcu_run_static: team kernel shared memory too large");
-            e = occupancy_mixed_team(l.team_warps, l.team_q, l.smem, &per_sm);
-            l.stride = l.need_d ? team_scratch_doubles(l.n_max) : 1;
-            l.per_block = sizeof(double) * (size_t)l.stride * teams_per_cta(l.team_warps, l.team_q);
-            l.block = 32 * l.team_warps * teams_per_cta(l.team_warps, l.team_q);
-            l.grid = (l.count + teams_per_cta(l.team_warps, l.team_q) - 1) / teams_per_cta(l.team_warps, l.team_q);
-        } else {
-            std::vector<int> d_opts = (!mixed && l.need_d) ? std::vector<int>{1, 0} : std::vector<int>{0};
-            std::vector<int> v_opts = l.need_lz ? std::vector<int>{kLanczosCold, kLanczosWarm, 0} : std::vector<int>{0};
-            l.d_in_smem = -1;
-            for (int d : d_opts) {
-                for (int v : v_opts) {
-                    const size_t bytes = (size_t)smem_layout(l.n_max, d, v, mixed).total * sizeof(double);
-                    if (bytes <= ctx->max_smem) {
-                        l.d_in_smem = d;
-                        l.v_cap = v;
-                        l.smem = bytes;
-                        break;
-                    }
+    auto plan = [&](bool pair) -> int {
+        launches.clear();
+        order.clear();
+        jumps = false;
+        max_block_scratch = 0;
+        std::vector<std::vector<int32_t>> lists(kMaxBuckets);
+        for (int i = 0; i < n_chains; ++i) lists[bucket_of(recs[i], form, pair)].push_back(i);
+        for (int id : kBucketOrder) {
+            std::vector<int32_t>& L = lists[id];
+            if (L.empty()) continue;
+            std::stable_sort(L.begin(), L.end(), [&](int32_t x, int32_t y) { return recs[x].N > recs[y].N; });
+            Launch l;
+            memset(&l, 0, sizeof(l));
+            l.id = id;
+            l.kernel = bucket_kernel(id, form);
+            l.count = (int)L.size();
+            l.n_max = 3 * recs[L.front()].N;
+            for (int32_t c : L)
+                if (recs[c].hstar > 0.0) {
+                    l.need_d = 1;
+                    if (recs[c].hi_method == BDCU_HI_CHEBYSHEV) l.need_lz = 1;
                 }
-                if (l.d_in_smem >= 0) break;
+            l.order_off = (int64_t)order.size();
+            order.insert(order.end(), L.begin(), L.end());
+            jumps = jumps || l.kernel != BDCU_KERNEL_BLOCK;
+            int per_sm = 0;
+            if (l.kernel == BDCU_KERNEL_TEAM) {
+                l.team_warps = kDefaultTeamShape[id][0];
+                l.team_q = kDefaultTeamShape[id][1];
+                l.w_pairs = l.need_d ? team_weights(l.team_warps, l.team_q, l.n_max, l.count, ctx->sm_count, ctx->max_smem) : 0;
+                l.smem = (size_t)team_smem(l.team_warps, l.team_q, l.n_max, l.w_pairs);
+                if (l.smem > ctx->max_smem) return fail(ctx, BDCU_E_LIMIT, "bdcu_run_static: team kernel shared memory too large");
+                e = occupancy_mixed_team(l.team_warps, l.team_q, l.smem, &per_sm);
+                l.stride = l.need_d ? team_scratch_doubles(l.n_max) : 1;
+                l.per_block = sizeof(double) * (size_t)l.stride * teams_per_cta(l.team_warps, l.team_q);
+                l.block = 32 * l.team_warps * teams_per_cta(l.team_warps, l.team_q);
+                l.grid = (l.count + teams_per_cta(l.team_warps, l.team_q) - 1) / teams_per_cta(l.team_warps, l.team_q);
+            } else if (l.kernel == kKernelPair) {
+                const int T = pair_warps(id);
+                l.block = 32 * T;
+                l.w_pairs = pair_shared(id, l.n_max, l.need_lz, l.count, ctx->sm_count, ctx->max_smem);
+                l.smem = (size_t)pair_layout(l.n_max, T, l.w_pairs).total * sizeof(double);
+                if (l.smem > ctx->max_smem) return fail(ctx, BDCU_E_LIMIT, "bdcu_run_static: chain too large for the shared-memory layout");
+                e = occupancy_pair(T, l.smem, &per_sm);
+                l.stride = l.need_lz ? pair_scratch_doubles(l.n_max) : 1;
+                l.per_block = sizeof(double) * (size_t)l.stride;
+                l.grid = l.count;
+            } else {
+                std::vector<int> d_opts = (!mixed && l.need_d) ? std::vector<int>{1, 0} : std::vector<int>{0};
+                std::vector<int> v_opts = l.need_lz ? std::vector<int>{kLanczosCold, kLanczosWarm, 0} : std::vector<int>{0};
+                l.d_in_smem = -1;
+                for (int d : d_opts) {
+                    for (int v : v_opts) {
+                        const size_t bytes = (size_t)smem_layout(l.n_max, d, v, mixed).total * sizeof(double);
+                        if (bytes <= ctx->max_smem) {
+                            l.d_in_smem = d;
+                            l.v_cap = v;
+                            l.smem = bytes;
+                            break;
+                        }
+                    }
+                    if (l.d_in_smem >= 0) break;
+                }
+                if (l.d_in_smem < 0) return fail(ctx, BDCU_E_LIMIT, "bdcu_run_static: chain too large for the shared-memory layout");
+                l.block = widest_block(l.n_max);
+                const ScratchLayout scl = scratch_layout(l.n_max, l.d_in_smem, l.v_cap, l.need_d, mixed, l.need_d, l.need_lz);
+                l.stride = std::max<int64_t>(scl.total, 1);
+                l.per_block = sizeof(double) * (size_t)l.stride;
+                e = mixed ? occupancy_mixed(l.block, l.smem, &per_sm) : occupancy_plain(l.block, l.smem, &per_sm);
+                l.grid = l.count;
             }
-            if (l.d_in_smem < 0) return fail(ctx, BDCU_E_LIMIT, "bdcu_run_static: chain too large for the shared-memory layout");
-            l.block = widest_block(l.n_max);
-            const ScratchLayout scl = scratch_layout(l.n_max, l.d_in_smem, l.v_cap, l.need_d, mixed, l.need_d, l.need_lz);
-            l.stride = std::max<int64_t>(scl.total, 1);
-            l.per_block = sizeof(double) * (size_t)l.stride;
-            e = mixed ? occupancy_mixed(l.block, l.smem, &per_sm) : occupancy_plain(l.block, l.smem, &per_sm);
-            l.grid = l.count;
+            if (e != cudaSuccess) return fail(ctx, BDCU_E_CUDA, std::string("occupancy query: ") + cudaGetErrorString(e));
+            if (per_sm < 1) return fail(ctx, BDCU_E_LIMIT, "bdcu_run_static: kernel shape cannot be resident");
+            l.grid = std::max(1, std::min(l.grid, per_sm * ctx->sm_count));
+            max_block_scratch = std::max(max_block_scratch, l.per_block);
+            launches.push_back(l);
         }
-        if (e != cudaSuccess) return fail(ctx, BDCU_E_CUDA, std::string("occupancy query: ") + cudaGetErrorString(e));
-        if (per_sm < 1) return fail(ctx, BDCU_E_LIMIT, "bdcu_run_static: kernel shape cannot be resident");
-        l.grid = std::max(1, std::min(l.grid, per_sm * ctx->sm_count));
-        max_block_scratch = std::max(max_block_scratch, l.per_block);
-        launches.push_back(l);
-    }
+        return BDCU_OK;
+    };
 
-    // RNG jump-ahead rows k = 0..n_max for the team kernel's noise
+    // layout of the static array: queue counters | records | work lists | seed
+    // table | arena | jump-ahead tables (rows k = 0..n_max) | scratch (reused by
+    // each bucket in turn)
+    const size_t o_cnt = 0;
+    const size_t o_rec = 256;
+    const size_t o_ord = align256(o_rec + sizeof(DevChain) * (size_t)n_chains);
+    const size_t o_seed = align256(o_ord + sizeof(int32_t) * (size_t)n_chains);
+    const size_t o_arena = align256(o_seed + sizeof(double) * (size_t)n_max);
+    const size_t o_cols = align256(o_arena + sizeof(double) * (size_t)std::max<int64_t>(arena_len, 1));
+    size_t o_apow = 0, o_scr = 0;
+    auto lay_out = [&]() {
+        const size_t rows = jumps ? (size_t)n_max + 1 : 0;
+        o_apow = align256(o_cols + sizeof(uint32_t) * 32 * rows);
+        o_scr = align256(o_apow + sizeof(uint32_t) * rows);
+        return o_scr + max_block_scratch <= kStaticScratchBytes;
+    };
+    int rc = plan(true);
+    if (rc != BDCU_OK) return rc;
+    bool fits = lay_out();
+    if (!fits && !mixed) {  // without the pair kernel's cold basis and jump-ahead tables
+        if ((rc = plan(false)) != BDCU_OK) return rc;
+        fits = lay_out();
+    }
+    if (!fits)
+        return fail(ctx, BDCU_E_LIMIT,
+                    "bdcu_run_static: needs " + std::to_string(o_scr + max_block_scratch) +
+                    " bytes of static device scratch for this batch (parameters plus one block's scratch); the "
+                    "maximum is " + std::to_string(kStaticScratchBytes) + " bytes. Use bdcu_run, or fewer/smaller chains.");
+    for (Launch& l : launches)
+        l.grid = (int)std::max<size_t>(1, std::min<size_t>((size_t)l.grid, (kStaticScratchBytes - o_scr) / l.per_block));
+
+    // RNG jump-ahead rows k = 0..n_max for the team and pair kernels' noise
     std::vector<uint32_t> cols, apow;
-    if (any_team) {
+    if (jumps) {
         cols.resize((size_t)(n_max + 1) * 32);
         apow.resize(n_max + 1);
         for (int i = 0; i < 32; ++i) cols[i] = 1u << i;
@@ -232,24 +283,6 @@ extern "C" int bdcu_run_static(bdcu_ctx* ctx, int n_chains, const bdcu_phys* phy
         }
     }
 
-    // layout of the static array: queue counters | records | work lists | seed
-    // table | arena | jump-ahead tables | scratch (reused by each bucket in turn)
-    const size_t o_cnt = 0;
-    const size_t o_rec = 256;
-    const size_t o_ord = align256(o_rec + sizeof(DevChain) * (size_t)n_chains);
-    const size_t o_seed = align256(o_ord + sizeof(int32_t) * order.size());
-    const size_t o_arena = align256(o_seed + sizeof(double) * (size_t)n_max);
-    const size_t o_cols = align256(o_arena + sizeof(double) * (size_t)std::max<int64_t>(arena_len, 1));
-    const size_t o_apow = align256(o_cols + sizeof(uint32_t) * cols.size());
-    const size_t o_scr = align256(o_apow + sizeof(uint32_t) * apow.size());
-    if (o_scr + max_block_scratch > kStaticScratchBytes)
-        return fail(ctx, BDCU_E_LIMIT,
-                    "bdcu_run_static: needs " + std::to_string(o_scr + max_block_scratch) +
-                    " bytes of static device scratch for this batch (parameters plus one block's scratch); the "
-                    "maximum is " + std::to_string(kStaticScratchBytes) + " bytes. Use bdcu_run, or fewer/smaller chains.");
-    for (Launch& l : launches)
-        l.grid = (int)std::max<size_t>(1, std::min<size_t>((size_t)l.grid, (kStaticScratchBytes - o_scr) / l.per_block));
-
     void* base = nullptr;
     e = static_base(ctx->device, &base);
     if (e != cudaSuccess) return fail(ctx, BDCU_E_CUDA, std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e));
@@ -261,9 +294,9 @@ extern "C" int bdcu_run_static(bdcu_ctx* ctx, int n_chains, const bdcu_phys* phy
     if (e == cudaSuccess) e = cudaMemcpyAsync(b + o_seed, seed.data(), sizeof(double) * n_max, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess && arena_len > 0)
         e = cudaMemcpyAsync(b + o_arena, arena, sizeof(double) * arena_len, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess && any_team)
+    if (e == cudaSuccess && jumps)
         e = cudaMemcpyAsync(b + o_cols, cols.data(), sizeof(uint32_t) * cols.size(), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess && any_team)
+    if (e == cudaSuccess && jumps)
         e = cudaMemcpyAsync(b + o_apow, apow.data(), sizeof(uint32_t) * apow.size(), cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) return fail(ctx, BDCU_E_CUDA, std::string("staging parameters: ") + cudaGetErrorString(e));
 
@@ -297,8 +330,10 @@ extern "C" int bdcu_run_static(bdcu_ctx* ctx, int n_chains, const bdcu_phys* phy
         a.scratch_stride = l.stride;
         a.xs_pow = reinterpret_cast<const uint32_t*>(b + o_cols);
         a.a_pow = reinterpret_cast<const uint32_t*>(b + o_apow);
-        if (l.id < kFirstBlockBucket)
+        if (l.kernel == BDCU_KERNEL_TEAM)
             e = launch_mixed_team(l.team_warps, l.team_q, a, l.grid, l.smem, s);
+        else if (l.kernel == kKernelPair)
+            e = launch_pair(l.block / 32, a, l.grid, l.smem, s);
         else
             e = mixed ? launch_mixed(a, l.grid, l.block, l.smem, s) : launch_plain(a, l.grid, l.block, l.smem, s);
         if (e != cudaSuccess)

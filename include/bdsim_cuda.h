@@ -374,8 +374,7 @@ int bdcu_check_chains(int n_chains, const bdcu_phys* phys, const bdcu_sim* sim, 
    already owns the GPU's memory, or a serving loop that must not take the
    implicit device-wide synchronisation cudaMalloc/cudaFree imply. This entry
    point takes the parameters on the host (as bdcu_set_chains does) and runs
-   bdcu_run's buckets one after another (the mixed form on the same kernels, the
-   plain form on the general block kernel: the same results to rounding) on the
+   the same kernels as bdcu_run (its buckets, one after another) on the
    caller's device buffers; the parameter records, work lists, arena, work
    counters and per-block scratch live in one
    file-scope device array of BDCU_STATIC_SCRATCH_BYTES that every GPU using
@@ -387,7 +386,10 @@ int bdcu_check_chains(int n_chains, const bdcu_phys* phys, const bdcu_sim* sim, 
      chain beyond the bead limit BDCU_E_LIMIT.
    - Batches whose parameters plus one block's scratch exceed the array return
      BDCU_E_LIMIT with a message; smaller batches run with as many concurrent
-     blocks as fit (fewer than bdcu_run may use).
+     blocks as fit (fewer than bdcu_run may use). A plain batch that fits only
+     without the scratch its usual kernel takes beyond the general one's (30
+     vectors of 3N and the generator's tables) runs on the general block kernel:
+     then its results equal bdcu_run's to rounding instead of bit for bit.
    - The first call on a device takes the array's device address
      (cudaGetSymbolAddress), and so does the first call after the device's
      context was replaced (cudaDeviceReset).

@@ -95,3 +95,45 @@ def test_a_plan_names_each_bucket_once():
         for k in ("n_chains", "min_beads", "max_beads", "block"):
             assert by_id[b["bucket"]][k] == b[k], (b["bucket"], k)
     assert sorted(b["bucket"] for b in both_methods([g for g in groups if g[1] == chol]).plan()) == [4, 5, 6, 7]
+
+
+def run_static(phys, sims, R0, rng, steps, form, pad=0):
+    """bdcu_run_static from t = 0; pad: unused doubles at the arena's end. Returns
+    its code and the final positions."""
+    import torch
+    n, dev = len(R0), torch.device("cuda", 0)
+    prec, srec, arena = _abi.pack_batch(phys, sims, [len(r) for r in R0])
+    arena = np.concatenate([arena, np.zeros(pad)])
+    R = torch.from_numpy(np.concatenate(R0)).to(dev)
+    state = torch.tensor(rng, dtype=torch.int32, device=dev)
+    cache, t0 = torch.zeros_like(R), torch.zeros(n, dtype=torch.float64, device=dev)
+    valid, status = (torch.zeros(n, dtype=torch.int32, device=dev) for _ in range(2))
+    k = torch.full((n,), steps, dtype=torch.int32, device=dev)
+    cnt = torch.zeros((n, 8), dtype=torch.int64, device=dev)
+    ctx = B.Context(0)
+    ctx.use_stream()
+    rc = ctx.lib.bdcu_run_static(ctx.h, n, prec, srec, arena.ctypes.data_as(_abi.c_double_p), arena.size,
+                                 _abi.dptr(R), _abi.dptr(state), _abi.dptr(cache), _abi.dptr(valid), _abi.dptr(t0),
+                                 _abi.dptr(k), _abi.dptr(status), _abi.dptr(cnt),
+                                 _abi.FORM_PLAIN_FP64 if form == "plain" else _abi.FORM_MIXED_FP32,
+                                 _abi.CACHE_RESET_PER_CALL)
+    torch.cuda.synchronize()
+    return rc, R.cpu().numpy()
+
+
+@pytest.mark.parametrize("form", ["plain", "mixed"])
+def test_static_entry_point_runs_the_same_kernels(form):
+    phys, sims, R0 = [], [], []
+    for N, method, hstar in [(10, "Chebyshev", 0.25), (50, "Chebyshev", 0.25), (64, "Cholesky", 0.25),
+                             (30, "Cholesky", 0.25), (100, "Chebyshev", 0.25), (100, "Cholesky", 0.25),
+                             (250, "Chebyshev", 0.25), (40, "Chebyshev", 0.0)]:
+        p, s = workloads.batched_cheb_phys(N)
+        p.hi_method, p.hstar = DelSMethod[method], hstar
+        phys.append(p)
+        sims.append(s)
+        R0.append(B.gaussian_chain(N, bond_std=1.0, seed=N))
+    rng = [(1, -1, 5 + i) for i in range(len(R0))]
+    ens = B.Ensemble(phys, sims, R0, rng, form=form)
+    ens.advance(0.0, 2, _abi.CACHE_RESET_PER_CALL)
+    rc, got = run_static(phys, sims, R0, rng, 2, form)
+    assert rc == 0 and np.array_equal(got, ens.R.cpu().numpy())
