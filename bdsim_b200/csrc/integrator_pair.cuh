@@ -49,45 +49,69 @@ __device__ __forceinline__ void warp_multisect(const Count& count, int target, d
 // with 16-byte loads at fixed offsets from one pointer.
 __device__ __forceinline__ int pair_at(int j, int d) { return 6 * (j >> 1) + 2 * d + (j & 1); }
 
-// Cholesky fallback (src/mobility.cpp:69-81): dense D in global scratch from
-// the staged positions ps, right-looking factor L, y = L x (3N vectors in shared
-// memory). Returns false if not positive definite. Out of line, with plain
+// Cholesky fallback (src/mobility.cpp:69-81): the lower part of the dense D in
+// global scratch from the staged positions ps (element (i, k) at L[k * ld + i]),
+// right-looking factor L, y = L x (3N vectors in shared memory). From 3N =
+// kBlockedCholMin on (kBlocked: shapes that hold such chains) the factorisation is
+// the block kernel's blocked one, staged in the `room` doubles at `stage`; its
+// column-block width follows from the chain's own size. (Column by column, every
+// column streams the trailing triangle through L2: 148 chains of N = 300 and 500,
+// two steps that fall back: FALLBACK_BEFORE ms, blocked FALLBACK_AFTER.) Returns 0, or a status
+// bit: not positive definite, a staging wait expired. Out of line, with plain
 // arguments: the chain's state stays in registers around the call.
-static __device__ __noinline__ bool pair_cholesky(double* L, const double* ps, int N, double hstar, const double* x,
-                                                  double* y) {
-    const int tid = threadIdx.x, TT = blockDim.x, wl = tid & 31, wi = tid >> 5, n = 3 * N;
-    for (int64_t e = tid; e < (int64_t)N * N; e += TT) {
-        const int mu = (int)(e / N), nu = (int)(e % N);
-        double d[3], om1 = 1.0, om2 = 0.0;
-        for (int k = 0; k < 3; ++k) d[k] = ps[pair_at(nu, k)] - ps[pair_at(mu, k)];
-        if (mu != nu) rpy_weights(hstar, d[0] * d[0] + d[1] * d[1] + d[2] * d[2], om1, om2);
-        for (int i = 0; i < 3; ++i)
+template <bool kBlocked>
+static __device__ __noinline__ int pair_cholesky(const RunArgs& a, const DevChain& ch, double* L, const double* ps,
+                                                 double* stage, int64_t room, const double* x, double* y) {
+    const int tid = threadIdx.x, TT = blockDim.x, wl = tid & 31, wi = tid >> 5, N = ch.N, n = 3 * N, ld = chol_ld(n);
+    for (int mu = wi; mu < N; mu += TT / 32)
+        for (int nu = mu + wl; nu < N; nu += 32) {
+            double d[3], om1 = 1.0, om2 = 0.0;
+            for (int k = 0; k < 3; ++k) d[k] = ps[pair_at(nu, k)] - ps[pair_at(mu, k)];
+            if (mu != nu) rpy_weights(ch.hstar, d[0] * d[0] + d[1] * d[1] + d[2] * d[2], om1, om2);
+            double* col = L + (int64_t)(3 * mu) * ld + 3 * nu;
             for (int j = 0; j < 3; ++j)
-                L[(int64_t)(3 * mu + i) * n + 3 * nu + j] = om2 * d[i] * d[j] + (i == j ? om1 : 0.0);
-    }
-    __syncthreads();
-    for (int k = 0; k < n; ++k) {
-        const double s = L[(int64_t)k * n + k];
-        if (!(s > 0.0)) return false;
-        const double dk = sqrt(s);
-        __syncthreads();
-        if (tid == 0) L[(int64_t)k * n + k] = dk;
-        for (int i = k + 1 + tid; i < n; i += TT) L[(int64_t)k * n + i] = L[(int64_t)k * n + i] / dk;
-        __syncthreads();
-        const double* colk = L + (int64_t)k * n;
-        for (int j = k + 1 + wi; j < n; j += TT / 32) {
-            const double ljk = colk[j];
-            for (int i = j + wl; i < n; i += 32) L[(int64_t)j * n + i] -= colk[i] * ljk;
+                for (int i = 0; i < 3; ++i) col[(int64_t)j * ld + i] = om2 * d[i] * d[j] + (i == j ? om1 : 0.0);
         }
+    __syncthreads();
+    if (kBlocked && n >= kBlockedCholMin) {
+        Ctl& ctl = *reinterpret_cast<Ctl*>(stage);
+        constexpr int kCtl = (int)((sizeof(Ctl) + 63) / 64 * 8);
+        if (tid == 0) ctl.brk = 0;
         __syncthreads();
+        Block<BDCU_FORM_PLAIN_FP64> B(a, ctl, ch);
+        B.N = N;
+        B.n = n;
+        B.Lt = L;
+        B.ldl = ld;
+        B.stage = stage + kCtl;
+        B.stage_cap = room - kCtl;
+        int nb = (int)((kLanczosWarm * round_up8(n) - kCtl) / (2 * kCholTileStride)) & ~7;
+        if (!B.cholesky_blocked(nb < kCholMaxBlock ? nb : kCholMaxBlock))
+            return ctl.brk == 2 ? BDCU_ST_TIMEOUT : BDCU_ST_NOT_PD;
+    } else {
+        for (int k = 0; k < n; ++k) {
+            const double s = L[(int64_t)k * ld + k];
+            if (!(s > 0.0)) return BDCU_ST_NOT_PD;
+            const double dk = sqrt(s);
+            __syncthreads();
+            if (tid == 0) L[(int64_t)k * ld + k] = dk;
+            for (int i = k + 1 + tid; i < n; i += TT) L[(int64_t)k * ld + i] = L[(int64_t)k * ld + i] / dk;
+            __syncthreads();
+            const double* colk = L + (int64_t)k * ld;
+            for (int j = k + 1 + wi; j < n; j += TT / 32) {
+                const double ljk = colk[j];
+                for (int i = j + wl; i < n; i += 32) L[(int64_t)j * ld + i] -= colk[i] * ljk;
+            }
+            __syncthreads();
+        }
     }
     for (int i = tid; i < n; i += TT) {
         double s = 0.0;
-        for (int j = 0; j <= i; ++j) s += L[(int64_t)j * n + i] * x[j];
+        for (int j = 0; j <= i; ++j) s += L[(int64_t)j * ld + i] * x[j];
         y[i] = s;
     }
     __syncthreads();
-    return true;
+    return 0;
 }
 
 // Doubles of a chain's factor in shared memory: its 3x3 blocks of the lower
@@ -1077,10 +1101,14 @@ __global__ void __launch_bounds__(32 * T, pair_min_blocks(T)) integrate_pair_ker
                     if (own)
                         for (int d = 0; d < 3; ++d) x[3 * b + d] = X0[d];
                     __syncthreads();
-                    if (!pair_cholesky(C.Lt, C.ps, N, ch.hstar, x, y)) {
-                        C.status |= BDCU_ST_NOT_PD;
+                    // (staged in the tables' place, dead by now, and the cached weights')
+                    const int bad = pair_cholesky<(T > 4)>(a, ch, C.Lt, C.ps, C.area,
+                                                                                  lay.total - lay.area, x, y);
+                    if (bad) {
+                        C.status |= bad;
                         break;
                     }
+                    C.build_weights();
 #pragma unroll
                     for (int d = 0; d < 3; ++d) bx[d] = on ? y[3 * b + d] : 0.0;
                 }

@@ -137,3 +137,53 @@ def test_static_entry_point_runs_the_same_kernels(form):
     ens.advance(0.0, 2, _abi.CACHE_RESET_PER_CALL)
     rc, got = run_static(phys, sims, R0, rng, 2, form)
     assert rc == 0 and np.array_equal(got, ens.R.cpu().numpy())
+
+
+def falling_back(N, copies, fd_err_max=-1.0, method=DelSMethod.Chebyshev):
+    """Chains whose series starts at its largest order and, for a negative bound
+    on its error, falls back to the Cholesky factor in every step."""
+    p, s = workloads.batched_cheb_phys(N)
+    p.ncheb_multiplier, p.fd_err_max, p.hi_method = 1e4, fd_err_max, method
+    R0 = [B.gaussian_chain(N, bond_std=1.0, seed=N)] * copies
+    return B.Ensemble([p] * copies, [s] * copies, R0, [(1, -1, 7)] * copies, form="plain")
+
+
+@pytest.mark.parametrize("N", [64, 65, 99, 100, 101, 128, 170, 257])
+def test_fallback_sizes(port, N):
+    """The blocked factorisation (3N >= 300) against the oracle, and the same bits
+    among enough chains that the launch caches fewer weights (the factor is staged
+    in their place)."""
+    p, s = workloads.batched_cheb_phys(N)
+    p.ncheb_multiplier, p.fd_err_max = 1e4, -1.0
+    s.time_start, s.time_end = 0.0, s.dt
+    R0 = B.gaussian_chain(N, bond_std=1.0, seed=N)
+    want, _, _, cnt = port.integrate(R0, p, s, (1, -1, 7))
+    ends = []
+    for copies in (1, 450):
+        ens = falling_back(N, copies)
+        ens.advance(0.0, 2, _abi.CACHE_RESET_PER_CALL)
+        assert cnt["cheb_fallbacks"] == 2 and int(ens.counters[0, 6]) == 2
+        ends.append(ens.positions()[0])
+    assert np.max(np.abs(ends[0] - want)) <= 1e-10 * max(1.0, np.max(np.abs(want)))
+    assert np.array_equal(ends[0], ends[1])
+
+
+def test_fallback_costs_no_more_than_the_cholesky_method():
+    """Both factor one tensor; column by column the fallback's factor took 17 times
+    the Cholesky method's whole step."""
+    import torch
+
+    def ms(ens):
+        best, R = 1e9, ens.R.clone()
+        for _ in range(4):
+            ens.R.copy_(R)
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            ens.advance(0.0, 1, _abi.CACHE_RESET_PER_CALL)
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b))
+        return best
+
+    factor = ms(falling_back(300, 148)) - ms(falling_back(300, 148, fd_err_max=1.0))
+    assert factor <= 4.0 * ms(falling_back(300, 148, method=DelSMethod.Cholesky))
