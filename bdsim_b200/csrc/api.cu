@@ -24,8 +24,8 @@ cudaError_t occupancy_plain(int block, size_t smem, int* per_sm);
 cudaError_t occupancy_mixed(int block, size_t smem, int* per_sm);
 cudaError_t launch_mixed_team(int team_warps, int team_q, const RunArgs& a, int grid, size_t smem, cudaStream_t s);
 cudaError_t occupancy_mixed_team(int team_warps, int team_q, size_t smem, int* per_sm);
-cudaError_t launch_pair(int warps, const RunArgs& a, int grid, size_t smem, cudaStream_t s);
-cudaError_t occupancy_pair(int warps, size_t smem, int* per_sm);
+cudaError_t launch_pair(int warps, bool hi, const RunArgs& a, int grid, size_t smem, cudaStream_t s);
+cudaError_t occupancy_pair(int warps, bool hi, size_t smem, int* per_sm);
 cudaError_t launch_forces(const DevChain* chains, int n_chains, int n_max, const double* arena, const double* R,
                           double t, int which, double* F, cudaStream_t s);
 cudaError_t launch_ran1(int n_chains, int32_t* rng, int n_per, double* out, cudaStream_t s);
@@ -297,11 +297,6 @@ std::vector<Shape> block_shapes(const bdcu_ctx* ctx, const Bucket& b, int form) 
     return out;
 }
 
-Shape pair_shape(int id) {
-    Shape s;
-    s.block = 32 * pair_warps(id);
-    return s;
-}
 
 // Fill the launch fields of a bucket for a shape (block or pair kernel) or for
 // the team kernel; 0 when the shape cannot run.
@@ -331,15 +326,16 @@ int fill_launch(bdcu_ctx* ctx, int form, Bucket& b, const Shape* s) {
         return BDCU_OK;
     }
     if (b.kernel == kKernelPair) {
-        const int T = s->block / 32;
-        b.block = s->block;
+        const int T = pair_warps(b.id, b.n_max, b.count, ctx->sm_count);
+        b.block = 32 * T;
         b.v_cap = b.d_in_smem = 0;
-        b.w_pairs = pair_shared(b.id, b.n_max, b.need_lz, b.count, ctx->sm_count, ctx->max_smem);
+        b.pair_hi = pair_hi(T, b.need_d, b.count, ctx->sm_count);
+        b.w_pairs = pair_shared(b.id, T, b.n_max, b.need_lz, b.count, ctx->sm_count, ctx->max_smem);
         b.smem = (size_t)pair_layout(b.n_max, T, b.w_pairs).total * sizeof(double);
         if (b.smem > ctx->max_smem) return fail(ctx, BDCU_E_LIMIT, "chain too large for the shared-memory layout");
-        auto& occ = ctx->pair_occ[T == 4 ? 0 : T == 8 ? 1 : 2];
+        auto& occ = ctx->pair_occ[T][b.pair_hi];
         if (occ.smem != b.smem) {
-            e = occupancy_pair(T, b.smem, &occ.per_sm);
+            e = occupancy_pair(T, b.pair_hi, b.smem, &occ.per_sm);
             if (e != cudaSuccess) return cuda_fail(ctx, e, "occupancy_pair");
             occ.smem = b.smem;
         }
@@ -441,8 +437,7 @@ int build_plan(bdcu_ctx* ctx, int form) {
             if ((rc = fill_launch(ctx, form, b, use ? &t : nullptr))) return rc;
             b.tuned = use ? 1 : 0;
         } else if (b.kernel == kKernelPair) {
-            const Shape pick = pair_shape(id);
-            if ((rc = fill_launch(ctx, form, b, &pick))) return rc;
+            if ((rc = fill_launch(ctx, form, b, nullptr))) return rc;
             b.tuned = ctx->tuned[mixed][id].block > 0 ? 1 : 0;
         } else {
             const std::vector<Shape> shapes = block_shapes(ctx, b, form);
@@ -539,7 +534,7 @@ int launch_bucket(bdcu_ctx* ctx, int form, const Bucket& b, const State& st, int
     if (b.kernel == BDCU_KERNEL_TEAM)
         e = launch_mixed_team(b.team_warps, b.team_q, a, b.grid, b.smem, s);
     else if (b.kernel == kKernelPair)
-        e = launch_pair(b.block / 32, a, b.grid, b.smem, s);
+        e = launch_pair(b.block / 32, b.pair_hi, a, b.grid, b.smem, s);
     else
         e = (form == BDCU_FORM_MIXED_FP32) ? launch_mixed(a, b.grid, b.block, b.smem, s)
                                            : launch_plain(a, b.grid, b.block, b.smem, s);
@@ -854,7 +849,7 @@ int bdcu_autotune(bdcu_ctx* ctx, int form, const double* R, const int32_t* rng, 
         Shape best;
         std::vector<Shape> shapes;
         if (base.kernel == kKernelPair) {  // one shape: nothing to time
-            ctx->tuned[mixed][base.id] = pair_shape(base.id);
+            ctx->tuned[mixed][base.id].block = base.block;
             continue;
         }
         if (base.kernel == BDCU_KERNEL_BLOCK) {

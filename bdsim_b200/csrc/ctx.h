@@ -53,6 +53,7 @@ struct Bucket {
     int need_chol = 0, need_d = 0, need_lz = 0;
     int64_t order_off = 0;  // first entry of this bucket's work list in order_d
     int block = 0, grid = 0, v_cap = 0, d_in_smem = 0, tuned = 0;
+    bool pair_hi = true;  // pair kernel: the build with HI
     int64_t w_pairs = 0;  // pair and team kernels: cached pair weights (per block, per team)
     size_t smem = 0;
     int64_t scratch_stride = 1;  // doubles per block (per warp)
@@ -100,8 +101,8 @@ struct bdcu_ctx {
     int bounds_every = 1;  // bdcu_set_bounds_refresh
     int single_launch = 0; // bdcu_set_single_launch: every team-kernel chain in one launch
     size_t max_smem = 0;
-    // the pair kernel's last occupancy query per warp count (4, 8, 16)
-    struct { size_t smem = 0; int per_sm = 0; } pair_occ[3];
+    // the pair kernel's last occupancy query per warps and build (without, with HI)
+    struct { size_t smem = 0; int per_sm = 0; } pair_occ[17][2];
     // the chains bdcu_run advances: all records (sel_all) or a list (bdcu_select)
     int sel_all = 1;
     std::vector<int32_t> sel;

@@ -56,9 +56,9 @@ __device__ __forceinline__ int pair_at(int j, int d) { return 6 * (j >> 1) + 2 *
 // the block kernel's blocked one, staged in the `room` doubles at `stage`; its
 // column-block width follows from the chain's own size. (Column by column, every
 // column streams the trailing triangle through L2: 148 chains of N = 300 and 500,
-// two steps that fall back: FALLBACK_BEFORE ms, blocked FALLBACK_AFTER.) Returns 0, or a status
-// bit: not positive definite, a staging wait expired. Out of line, with plain
-// arguments: the chain's state stays in registers around the call.
+// one step that falls back after 500 products: 170 and 712 ms, blocked 34 and 78.)
+// Returns 0, or a status bit: not positive definite, a staging wait expired. Out of
+// line, with plain arguments: the chain's state stays in registers around the call.
 template <bool kBlocked>
 static __device__ __noinline__ int pair_cholesky(const RunArgs& a, const DevChain& ch, double* L, const double* ps,
                                                  double* stage, int64_t room, const double* x, double* y) {
@@ -179,7 +179,7 @@ struct PairChain {
 #pragma unroll
         for (int m = 0; m < M; ++m) {
             const double2* q = reinterpret_cast<const double2*>(r + m * T);
-            double a0 = 0.0;
+            double a0 = T == 1 ? 0.0 + r[m] : 0.0;
 #pragma unroll
             for (int w = 0; w < T / 2; ++w) a0 += q[w].x + q[w].y;
             v[m] = a0;
@@ -189,7 +189,7 @@ struct PairChain {
     // the eight published at r (one load per four warps, two shuffles).
     __device__ __forceinline__ double total8(const double* r) const {
         const double* q = r + (wl & 7) * T + (wl >> 3);
-        double t = q[0];
+        double t = T >= 4 || (wl >> 3) < T ? q[0] : 0.0;
 #pragma unroll
         for (int w = 4; w < T; w += 4) t += q[w];
         t += __shfl_xor_sync(kFull, t, 8);
@@ -762,14 +762,14 @@ struct PairChain {
             for (int d = 0; d < 3; ++d) ritz[d] = on ? 2.0 * V[3 * b + d] : 0.0;
             return;
         }
-        if (wi < 2) {  // warp 0 the smallest eigenvalue, warp 1 the largest
+        for (int e = wi; e < 2; e += T) {  // warp 0 the smallest eigenvalue, warp 1 (or 0 too) the largest
             double lo = alpha[0], hi2 = alpha[0];
             for (int i = 0; i < k; ++i) {
                 const double rad = (i > 0 ? fabs(beta[i - 1]) : 0.0) + (i < k - 1 ? fabs(beta[i]) : 0.0);
                 lo = dmin_(lo, alpha[i] - rad);
                 hi2 = dmax_(hi2, alpha[i] + rad);
             }
-            double* y = wi == 0 ? ymin : ymax;
+            double* y = e == 0 ? ymin : ymax;
             double r;
             if (k <= kLanczosWarm) {
                 double ar[kLanczosWarm], br[kLanczosWarm], b2[kLanczosWarm], yr[kLanczosWarm];
@@ -779,7 +779,7 @@ struct PairChain {
                     br[i] = i < k - 1 ? beta[i] : 0.0;
                     b2[i] = br[i] * br[i];
                 }
-                warp_multisect([&](double x) { return sturm_count8(ar, b2, k, x); }, wi == 0 ? 1 : k, lo, hi2);
+                warp_multisect([&](double x) { return sturm_count8(ar, b2, k, x); }, e == 0 ? 1 : k, lo, hi2);
                 r = 0.5 * (lo + hi2);
                 tridiag_vec_reg<2>(ar, br, k, r, yr);
                 if (wl == 0)
@@ -787,12 +787,12 @@ struct PairChain {
                     for (int i = 0; i < kLanczosWarm; ++i)
                         if (i < k) y[i] = yr[i];
             } else {
-                warp_multisect([&](double x) { return sturm_count_products(alpha, beta, k, x); }, wi == 0 ? 1 : k, lo,
+                warp_multisect([&](double x) { return sturm_count_products(alpha, beta, k, x); }, e == 0 ? 1 : k, lo,
                                hi2);
                 r = 0.5 * (lo + hi2);
-                if (wl == 0) wk_tridiag_vec(alpha, beta, k, r, y, s3 + 32 * wi, s4 + 32 * wi);
+                if (wl == 0) wk_tridiag_vec(alpha, beta, k, r, y, s3 + 32 * e, s4 + 32 * e);
             }
-            if (wl == 0) tot[wi] = r;
+            if (wl == 0) tot[e] = r;
         }
         __syncthreads();
         rmin = tot[0];
@@ -933,8 +933,8 @@ struct PairChain {
 
 // -------------------------------------------------------------- the kernel
 
-template <int T>
-__global__ void __launch_bounds__(32 * T, pair_min_blocks(T)) integrate_pair_kernel(const RunArgs a) {
+template <int T, bool kHi>
+__global__ void __launch_bounds__(32 * T, pair_min_blocks(T, kHi)) integrate_pair_kernel(const RunArgs a) {
     extern __shared__ __align__(16) double psm[];
     constexpr int TT = 32 * T;
     const PairLayout lay = pair_layout(a.n_max, T, a.w_pairs);
@@ -1008,7 +1008,7 @@ __global__ void __launch_bounds__(32 * T, pair_min_blocks(T)) integrate_pair_ker
         C.bc = min(C.b, N - 1);
         C.on = C.b < N;
         C.own = C.on && C.seg == 0;
-        C.hi = ch.hstar > 0.0;
+        C.hi = kHi && ch.hstar > 0.0;
         C.status = status0;
         C.np = (Ne / 2 - C.gl + 2 * C.S - 1) / (2 * C.S);
         // (the Cholesky method keeps its factor in the weights' place: three
@@ -1036,7 +1036,7 @@ __global__ void __launch_bounds__(32 * T, pair_min_blocks(T)) integrate_pair_ker
         const double sqrt_dt = sqrt(dt), inv_n = 1.0 / N;
         double v0[3];  // the Lanczos start vector, kept from step to step
         bool used_cache = false;
-        if (C.hi && ch.hi_method == BDCU_HI_CHEBYSHEV) {
+        if (kHi && C.hi && ch.hi_method == BDCU_HI_CHEBYSHEV) {
             if (own)
                 for (int d = 0; d < 3; ++d) C.seed[3 * b + d] = a.seed_table[3 * b + d] / ch.seed_norm;
             __syncwarp();  // (the lanes of a bead read it back)
@@ -1070,7 +1070,7 @@ __global__ void __launch_bounds__(32 * T, pair_min_blocks(T)) integrate_pair_ker
             C.noise(ux, iy, X0);
             drew = true;
             // brownian_step (src/mobility.cpp:58-88)
-            if (!C.hi) {
+            if (!kHi || !C.hi) {
 #pragma unroll
                 for (int d = 0; d < 3; ++d) {
                     dW[d] = sqrt_dt * X0[d];

@@ -16,11 +16,15 @@ constexpr int kPairCholMaxN = 64;
 __host__ __device__ inline int64_t pair_factor_doubles(int N) { return 9 * (int64_t)N * (N + 1) / 2; }
 
 // Blocks per SM a shape's registers and shared memory are sized for. 12 to 16
-// warps per SM: 168 registers per thread at T = 4, 128 at T = 8 and 16.
-__host__ __device__ constexpr int pair_min_blocks(int T) { return T == 4 ? 3 : T == 8 ? 2 : 1; }
+// warps per SM: 168 registers per thread up to T = 4, 128 at T = 8 and 16. hi:
+// whether the launch has a chain with HI; the build without leaves its code out and
+// runs 8 blocks of T = 4 (64 registers) instead of 3.
+__host__ __device__ constexpr int pair_min_blocks(int T, bool hi) {
+    return T <= 4 ? (hi || T < 4 ? 12 / T : 8) : T == 8 ? 2 : 1;
+}
 
-// Warps per chain of buckets 0..3 (N <= 64, 128, 256, 512), and of the Cholesky
-// method's.
+// Warps per chain of buckets 0..3 (N <= 64, 128, 256, 512; fewer in launches of the
+// shortest chains), and of the Cholesky method's.
 constexpr int kPairWarps[4] = {4, 8, 8, 16};
 constexpr int kPairCholWarps = 4;
 
@@ -81,7 +85,7 @@ __host__ __device__ inline PairLayout pair_layout(int n_max, int T, int64_t w_pa
 // leave an SM. The split changes no result.
 __host__ inline int64_t pair_cached(int n_max, int T, int blocks, int sm_count, size_t max_smem) {
     int per_sm = (blocks + sm_count - 1) / sm_count;
-    if (per_sm > pair_min_blocks(T)) per_sm = pair_min_blocks(T);
+    if (per_sm > pair_min_blocks(T, true)) per_sm = pair_min_blocks(T, true);
     const int64_t share = ((int64_t)max_smem + 1024) / per_sm - 1024;
     const int64_t room = (share / 8 - pair_layout(n_max, T, 0).total) / 2;
     const int64_t all = pair_weights(n_max / 3, T);

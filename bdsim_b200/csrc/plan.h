@@ -35,16 +35,32 @@ inline int bucket_kernel(int id, int form) {
     return form == BDCU_FORM_MIXED_FP32 ? (int)BDCU_KERNEL_TEAM : kKernelPair;
 }
 
-// The pair kernel's one shape for a bucket: its sums run in the order of the
-// lanes per bead and the warps, so that a chain's result does not depend on the
-// launch it is in the warps follow from the chain alone (not from a timing).
-inline int pair_warps(int id) { return id == kPairCholBucket ? kPairCholWarps : kPairWarps[id]; }
+// The pair kernel's warps per chain in a launch over `chains` chains of up to
+// n_max/3 beads. Its sums run in the order of the lanes per bead and the warps, so
+// that a chain's result does not depend on the launch it is in the warps follow
+// from its bucket (not from a timing). Chains that have their 16 lanes per bead on
+// fewer warps (N = 2 on one, N <= 4 on two) end in the same bits there: the further
+// warps would add zeros. They take the fewer warps where the chains outnumber the
+// blocks of four warps on the SMs (3 each); below that one chain's latency counts.
+// (16384 dumbbells, 10 steps: with HI 12.5 -> 5.3 ms, without 2.97 -> 0.94.)
+inline int pair_warps(int id, int n_max, int chains, int sm_count) {
+    if (id == kPairCholBucket) return kPairCholWarps;
+    if (chains > 3 * sm_count && n_max <= 12) return n_max <= 6 ? 1 : 2;
+    return kPairWarps[id];
+}
+
+// Whether such a launch on T warps takes the build with HI: a launch without it
+// takes the other one at T = 4 where it has more chains than the build with HI has
+// blocks on the SMs (both give a chain the same bits). (4096 free-draining chains,
+// 10 steps: N = 5 0.86 -> 0.56 ms, N = 64 2.09 -> 1.83; 400 chains of N = 64 were
+// 0.27 -> 0.31.)
+inline bool pair_hi(int T, bool hi, int chains, int sm_count) { return hi || T != 4 || chains <= 3 * sm_count; }
 
 // Pair weights in shared memory (16 bytes each) of a block of a pair bucket's
 // launch over `chains` chains; a Cholesky bucket's factor takes their place.
-inline int64_t pair_shared(int id, int n_max, bool need_lz, int chains, int sm_count, size_t max_smem) {
+inline int64_t pair_shared(int id, int T, int n_max, bool need_lz, int chains, int sm_count, size_t max_smem) {
     if (id == kPairCholBucket) return (pair_factor_doubles(n_max / 3) + 1) / 2;
-    return need_lz ? pair_cached(n_max, pair_warps(id), chains, sm_count, max_smem) : 0;
+    return need_lz ? pair_cached(n_max, T, chains, sm_count, max_smem) : 0;
 }
 
 #define BDCU_TEAM_SHAPE_SWITCH(T, Q, EXPR, FALLBACK)            \

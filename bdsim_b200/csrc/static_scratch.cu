@@ -44,8 +44,8 @@ cudaError_t occupancy_plain(int block, size_t smem, int* per_sm);
 cudaError_t occupancy_mixed(int block, size_t smem, int* per_sm);
 cudaError_t launch_mixed_team(int team_warps, int team_q, const RunArgs& a, int grid, size_t smem, cudaStream_t s);
 cudaError_t occupancy_mixed_team(int team_warps, int team_q, size_t smem, int* per_sm);
-cudaError_t launch_pair(int warps, const RunArgs& a, int grid, size_t smem, cudaStream_t s);
-cudaError_t occupancy_pair(int warps, size_t smem, int* per_sm);
+cudaError_t launch_pair(int warps, bool hi, const RunArgs& a, int grid, size_t smem, cudaStream_t s);
+cudaError_t occupancy_pair(int warps, bool hi, size_t smem, int* per_sm);
 DevChain derive_record(const bdcu_phys& p, const bdcu_sim& s, int64_t bead_off);
 int validate_chain(bdcu_ctx* ctx, int i, const bdcu_phys& p, const bdcu_sim& s, const double* arena,
                    int64_t arena_len);
@@ -145,7 +145,7 @@ extern "C" int bdcu_run_static(bdcu_ctx* ctx, int n_chains, const bdcu_phys* phy
     // buckets, as bdcu_run plans them (largest chains first within a bucket)
     const int mixed = (form == BDCU_FORM_MIXED_FP32);
     struct Launch {
-        int id, kernel, team_warps, team_q, block, grid, v_cap, d_in_smem, n_max, need_d, need_lz, count;
+        int id, kernel, pair_hi, team_warps, team_q, block, grid, v_cap, d_in_smem, n_max, need_d, need_lz, count;
         size_t smem, per_block;
         int64_t stride, order_off, w_pairs;
     };
@@ -191,12 +191,13 @@ extern "C" int bdcu_run_static(bdcu_ctx* ctx, int n_chains, const bdcu_phys* phy
                 l.block = 32 * l.team_warps * teams_per_cta(l.team_warps, l.team_q);
                 l.grid = (l.count + teams_per_cta(l.team_warps, l.team_q) - 1) / teams_per_cta(l.team_warps, l.team_q);
             } else if (l.kernel == kKernelPair) {
-                const int T = pair_warps(id);
+                const int T = pair_warps(id, l.n_max, l.count, ctx->sm_count);
                 l.block = 32 * T;
-                l.w_pairs = pair_shared(id, l.n_max, l.need_lz, l.count, ctx->sm_count, ctx->max_smem);
+                l.pair_hi = pair_hi(T, l.need_d, l.count, ctx->sm_count);
+                l.w_pairs = pair_shared(id, T, l.n_max, l.need_lz, l.count, ctx->sm_count, ctx->max_smem);
                 l.smem = (size_t)pair_layout(l.n_max, T, l.w_pairs).total * sizeof(double);
                 if (l.smem > ctx->max_smem) return fail(ctx, BDCU_E_LIMIT, "bdcu_run_static: chain too large for the shared-memory layout");
-                e = occupancy_pair(T, l.smem, &per_sm);
+                e = occupancy_pair(T, l.pair_hi, l.smem, &per_sm);
                 l.stride = l.need_lz ? pair_scratch_doubles(l.n_max) : 1;
                 l.per_block = sizeof(double) * (size_t)l.stride;
                 l.grid = l.count;
@@ -333,7 +334,7 @@ extern "C" int bdcu_run_static(bdcu_ctx* ctx, int n_chains, const bdcu_phys* phy
         if (l.kernel == BDCU_KERNEL_TEAM)
             e = launch_mixed_team(l.team_warps, l.team_q, a, l.grid, l.smem, s);
         else if (l.kernel == kKernelPair)
-            e = launch_pair(l.block / 32, a, l.grid, l.smem, s);
+            e = launch_pair(l.block / 32, l.pair_hi, a, l.grid, l.smem, s);
         else
             e = mixed ? launch_mixed(a, l.grid, l.block, l.smem, s) : launch_plain(a, l.grid, l.block, l.smem, s);
         if (e != cudaSuccess)

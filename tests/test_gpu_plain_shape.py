@@ -187,3 +187,22 @@ def test_fallback_costs_no_more_than_the_cholesky_method():
 
     factor = ms(falling_back(300, 148)) - ms(falling_back(300, 148, fd_err_max=1.0))
     assert factor <= 4.0 * ms(falling_back(300, 148, method=DelSMethod.Cholesky))
+
+
+@pytest.mark.parametrize("hstar", [0.25, 0.0])
+@pytest.mark.parametrize("N,blocks", [(2, 12), (3, 6), (4, 6), (5, 8), (64, 6)])
+def test_many_short_chains_fill_the_sms(hstar, N, blocks):
+    """Short chains, and chains without HI, in numbers: more blocks on an SM than a
+    few of them get (three of four warps), and the same bits as alone, whatever the
+    launch's width and build."""
+    ends = []
+    for copies in (3, 2000):
+        p, s = workloads.batched_cheb_phys(N)
+        p.hstar = hstar
+        R0 = [B.gaussian_chain(N, bond_std=1.0, seed=i % 3) for i in range(copies)]
+        ens = B.Ensemble([p] * copies, [s] * copies, R0, [(1, -1, 5 + i % 3) for i in range(copies)], form="plain")
+        grid = ens.plan()[0]["grid"]
+        assert grid == copies if copies < 2000 else grid >= min(2000, 148 * (3 if N > 4 and hstar > 0.0 else blocks))
+        ens.advance(0.0, 4, _abi.CACHE_RESET_PER_CALL)
+        ends.append(ens.positions())
+    assert all(np.array_equal(r, ends[0][i % 3]) for i, r in enumerate(ends[1]))
