@@ -206,3 +206,27 @@ def test_many_short_chains_fill_the_sms(hstar, N, blocks):
         ens.advance(0.0, 4, _abi.CACHE_RESET_PER_CALL)
         ends.append(ens.positions())
     assert all(np.array_equal(r, ends[0][i % 3]) for i, r in enumerate(ends[1]))
+
+
+def test_mixed_fallback_costs_no_more_than_twice_the_cholesky_method():
+    """N = 50: a factor of the team kernel (2.9 ms while each column waited for L2)
+    against a step of the Cholesky method on the block kernel."""
+    import torch
+
+    def ms(method, fd_err_max):
+        p, s = workloads.batched_cheb_phys(50)
+        p.ncheb_multiplier, p.fd_err_max, p.hi_method = 1e4, fd_err_max, method
+        ens = B.Ensemble([p], [s], [B.gaussian_chain(50, bond_std=1.0, seed=1)], [(1, -1, 7)], form="mixed")
+        best, R = 1e9, ens.R.clone()
+        for _ in range(6):
+            ens.R.copy_(R)
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            ens.advance(0.0, 1, _abi.CACHE_RESET_PER_CALL)
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b))
+        return best
+
+    factor = ms(DelSMethod.Chebyshev, -1.0) - ms(DelSMethod.Chebyshev, 1.0)
+    assert factor <= 2.0 * ms(DelSMethod.Cholesky, 1.0)
