@@ -10,8 +10,9 @@
 // or segment order and the pair products use fma, so results differ from the
 // reference's by rounding only (this file is compiled with --fmad=false: the
 // spring, bending and connector arithmetic rounds as the reference's). The
-// Lanczos runs orthogonalise each vector against the whole basis as the
-// reference does, but all projections of a step are reduced together.
+// Lanczos runs project on the whole basis where a bound on the loss of orthogonality
+// asks for it, all projections of a step reduced together (the reference projects
+// every vector).
 //
 // Reference: src/integrator.cpp:61-170 of the bdsim project and the physics it
 // calls; each stage cites its reference function.
@@ -700,27 +701,33 @@ struct PairChain {
     // so that its norm (explicit: |Du|^2 - alpha^2 - beta^2 loses digits from
     // step to step), alpha and the next vector follow at once.
     // Orthogonality: the reference projects every vector on the whole basis. In 8
-    // steps the three-term recurrence alone gives the same extreme eigenvalues
-    // (to 5e-14) and start vector (to 5e-14). A cold run projects in two steps
-    // of every six (from 3N = 64; in every step below, where the Krylov space is
-    // soon exhausted): two consecutive steps restore orthogonality, and between
-    // them it stays far below the square root of rounding that the
-    // tridiagonal's accuracy needs. Over the chain lengths and potentials of the
-    // tests the eigenvalues agree with the reference's scheme to 2e-14, the
-    // basis is orthogonal to 1e-11. (Projecting in every step read the basis from
+    // steps the three-term recurrence alone gives the same extreme eigenvalues to
+    // 1e-12 relative (3e-10 for the smallest one of chains whose beads nearly
+    // coincide). A cold run projects where BasisLoss says so (from 3N = 64; in
+    // every step below, where the Krylov space is soon exhausted), which keeps the
+    // basis orthogonal to 1e-9, far below the square root of rounding that the
+    // tridiagonal's accuracy needs. (Projecting in every step read the basis from
     // L2 twice a step: 12.9 thousand cycles a step at N = 50, 2.7 of them the
-    // product; now 6.6.) Returns its steps; the tridiagonal is left in alpha and
-    // beta.
+    // product.) Returns its steps; the tridiagonal is left in alpha and beta.
     __device__ __forceinline__ int lanczos(double* V, bool cold, double (&v)[3], double (&w)[3], bool have_w) {
         const int m = min(n, cold ? kLanczosCold : kLanczosWarm);
         const bool every = n < 64;
-        double u[3] = {v[0], v[1], v[2]}, vp[3] = {0.0, 0.0, 0.0}, bprev = 1.0;
-        bool due = false;
+        double u[3] = {v[0], v[1], v[2]}, vp[3] = {0.0, 0.0, 0.0};
+        BasisLoss loss;
 #pragma unroll 1
         for (int j = 0;; ++j) {
             if (j > 0 || !have_w) apply1(u, w);
             double g2[2] = {fma(u[2], u[2], fma(u[1], u[1], u[0] * u[0])), fma(u[2], w[2], fma(u[1], w[1], u[0] * w[0]))};
-            sums(g2);
+            double ww = 0.0;
+            if (cold) {
+                double g3[3] = {g2[0], g2[1], fma(w[2], w[2], fma(w[1], w[1], w[0] * w[0]))};
+                sums(g3);
+                g2[0] = g3[0];
+                g2[1] = g3[1];
+                ww = g3[2];
+            } else {
+                sums(g2);
+            }
             const double bsq = g2[0];
             if (j > 0 && bsq < 1.0e-20) {
                 cnt[C_DX] -= 1;  // (the reference stops before this product)
@@ -744,11 +751,8 @@ struct PairChain {
                 vp[d] = v[d];
             }
             if (cold) {
-                // a beta far below its neighbours magnifies what orthogonality was lost
-                due = due ? bt < 0.1 * bprev : bt < 0.03 * fabs(al) || bt < 0.1 * bprev;
-                bprev = bt;
                 __syncwarp();  // (the lanes of a bead read its basis entries back)
-                if (every || due || j % 6 >= 4) project(j + 1, u);
+                if (every || loss.project(j, al, bt, (ww * ib) * ib, 1.0e-15, 1.0e-9, 1.0e-10)) project(j + 1, u);
             }
         }
     }

@@ -258,6 +258,45 @@ static __device__ void wk_tridiag_vec(const double* a, const double* b, int m, d
 }
 
 
+// Which vectors of a cold Lanczos run are projected on the whole basis (the reference
+// projects every one, src/hydrodynamics.cpp:171-186): a bound on their loss of
+// orthogonality, carried along by the recurrence that the loss follows (H. D. Simon,
+// "The Lanczos algorithm with partial reorthogonalization", Math. Comp. 42, 1984),
+//   |v_{j+1}.v_i| <= ((|a_i - a_j| + b_i + b_{i+1}) w_j + b_j w_{j-1} + eps |D|) / b_{j+1}
+// with the largest factor over i. Once it passes `tol` two consecutive vectors are
+// projected, as both enter the recurrence. tol is the square root of the products'
+// rounding, up to which the tridiagonal is the projection of D to that rounding, with
+// a margin. b_{j+1} comes from |D v_j|^2 by Pythagoras; where that cancels (below
+// `tiny` of it) the vectors are projected in any case. (Two of every six, whatever the
+// spectrum, lost all orthogonality within four steps on chains whose beads lie close
+// together: bounds off by up to 18x in FP64 and 1e4x on FP32 products. Projected in
+// FP64: 25% of the vectors on coils, 37% on collapsed chains.)
+struct BasisLoss {
+    double w = 0.0, wp = 0.0, lo = 0.0, hi = 0.0, bmax = 0.0;
+    bool again = false;
+    // After step j's alpha, beta (none at j = 0) and ww = |D v_j|^2: project the next vector?
+    __device__ __forceinline__ bool project(int j, double al, double bt, double ww, double eps, double tol, double tiny) {
+        if (j == 0) {
+            lo = hi = al;
+            bt = 0.0;
+        }
+        lo = fmin(lo, al);
+        hi = fmax(hi, al);
+        bmax = fmax(bmax, bt);
+        const double bsq = ww - al * al - bt * bt;
+        const bool lost = !(bsq > tiny * ww);
+        const double ib = lost ? 1.0 : rsqrt_refined(bsq), bn = lost ? 1.0 : bsq * ib;
+        const double f = fmax(hi - al, al - lo) + 2.0 * fmax(bmax, bn);
+        double wn = (f * w + bt * wp + eps * (fabs(al) + bt + bn)) * ib;
+        const bool hit = lost || !(wn <= tol), now = hit || again;
+        again = lost || (hit && !again);
+        if (now) wn = eps;
+        wp = w;
+        w = wn;
+        return now;
+    }
+};
+
 // Right-looking Cholesky factor (cholesky_lower, src/linalg.cpp:91-107) of the n x n
 // matrix at L in global scratch, by a team of T warps. Returns false if not positive
 // definite. The trailing update takes eight columns at a time, so that a thread's
@@ -944,9 +983,10 @@ struct TeamChain {
     // loss of orthogonality leaves the extreme Ritz values far inside the 2x /
     // 2% padding of the bounds, and the Chebyshev fluctuation-dissipation check
     // polices the result. Cold runs (30 steps, the first step of a call) project
-    // on the whole basis in two steps of every six (below 3N = 64 in every
-    // step), which keeps it orthogonal to about 1e-11; the reference's modified
-    // Gram-Schmidt took up to 30 reductions in turn per step. One reduction per
+    // on the whole basis where BasisLoss says so (below 3N = 64 in every step),
+    // which keeps it orthogonal to the square root of the FP32 products' rounding;
+    // the reference's modified Gram-Schmidt took up to 30 reductions in turn per
+    // step. One reduction per
     // step: the new vector u goes into the product unnormalised, and u.u and u.Du
     // are summed together.
     __device__ int lanczos(int m, bool warm, const double (&v0)[Q][3], const double (&dv0)[Q][3], bool have_dv0,
@@ -963,20 +1003,28 @@ struct TeamChain {
                 vp[q][d] = 0.0;
             }
         int k = 0;
-        double bprev = 1.0;
-        bool due = false;
+        BasisLoss loss;
 #pragma unroll 1
         for (int j = 0;; ++j) {
             if (j > 0 || !have_dv0) apply(u, w);
-            double g[2] = {0.0, 0.0};
+            double g[2] = {0.0, 0.0}, ww = 0.0;
 #pragma unroll
             for (int q = 0; q < Q; ++q)
 #pragma unroll
                 for (int d = 0; d < 3; ++d) {
                     g[0] += u[q][d] * u[q][d];
                     g[1] += u[q][d] * w[q][d];
+                    ww += w[q][d] * w[q][d];
                 }
-            sums(g);
+            if (cold) {
+                double g3[3] = {g[0], g[1], ww};
+                sums(g3);
+                g[0] = g3[0];
+                g[1] = g3[1];
+                ww = g3[2];
+            } else {
+                sums(g);
+            }
             if (j > 0 && g[0] < 1.0e-20) {
                 cnt[C_DX] -= 1;  // (the reference stops before this product)
                 break;
@@ -1002,12 +1050,7 @@ struct TeamChain {
                     if (j > 0) u[q][d] -= bt * vp[q][d];
                     vp[q][d] = v[q][d];
                 }
-            if (cold) {
-                // a beta far below its neighbours magnifies what orthogonality was lost
-                due = due ? bt < 0.1 * bprev : bt < 0.03 * fabs(al) || bt < 0.1 * bprev;
-                bprev = bt;
-                if (every || due || j % 6 >= 4) project(j + 1, u);
-            }
+            if (cold && (every || loss.project(j, al, bt, (ww * ib) * ib, 1.0e-7, 3.0e-4, 1.0e-5))) project(j + 1, u);
         }
         sync();
         if (k == 1) {
