@@ -51,68 +51,80 @@ __device__ __forceinline__ void warp_multisect(const Count& count, int target, d
 __device__ __forceinline__ int pair_at(int j, int d) { return 6 * (j >> 1) + 2 * d + (j & 1); }
 
 // Cholesky fallback (src/mobility.cpp:69-81): the lower part of the dense D in
-// global scratch from the staged positions ps (element (i, k) at L[k * ld + i]),
-// right-looking factor L, y = L x (3N vectors in shared memory). From 3N =
-// kBlockedCholMin on (kBlocked: shapes that hold such chains) the factorisation is
-// the block kernel's blocked one, staged in the `room` doubles at `stage`; its
-// column-block width follows from the chain's own size. (Column by column, every
-// column streams the trailing triangle through L2: 148 chains of N = 300 and 500,
-// one step that falls back after 500 products: 170 and 712 ms, blocked 34 and 78.)
-// Returns 0, or a status bit: not positive definite, a staging wait expired. Out of
+// global scratch from the staged positions ps (element (i, k) at L[k n + i]), its
+// right-looking factor, y = L x (3N vectors in shared memory). Eight columns at a
+// time are factored in shared memory (P, 8 round_up8(n) doubles: the area of the
+// Chebyshev tables, dead by now); then a warp takes four columns of the trailing
+// triangle at once, so that an element crosses L2 once per eight columns and a lane's
+// four loads are in flight together. Every element still receives its products one by
+// one, in k order. (One column at a time, each streamed the triangle through L2: 148
+// chains of N = 300 and 500, one step that falls back after 500 products, 170 and 712
+// ms; so 37 and 102. The block kernel's tile updates on the tensor cores in this
+// place: 32 and 70, but their registers made the kernel spill in the steps that do not
+// fall back, 3 to 10% of large chains' time.) False if not positive definite. Out of
 // line, with plain arguments: the chain's state stays in registers around the call.
-template <bool kBlocked>
-static __device__ __noinline__ int pair_cholesky(const RunArgs& a, const DevChain& ch, double* L, const double* ps,
-                                                 double* stage, int64_t room, const double* x, double* y) {
-    const int tid = threadIdx.x, TT = blockDim.x, wl = tid & 31, wi = tid >> 5, N = ch.N, n = 3 * N, ld = chol_ld(n);
+static __device__ __noinline__ bool pair_cholesky(double* L, double* P, const double* ps, int N, double hstar,
+                                                  const double* x, double* y) {
+    const int tid = threadIdx.x, TT = blockDim.x, wl = tid & 31, wi = tid >> 5, n = 3 * N, ld = (n + 7) & ~7;
     for (int mu = wi; mu < N; mu += TT / 32)
         for (int nu = mu + wl; nu < N; nu += 32) {
             double d[3], om1 = 1.0, om2 = 0.0;
             for (int k = 0; k < 3; ++k) d[k] = ps[pair_at(nu, k)] - ps[pair_at(mu, k)];
-            if (mu != nu) rpy_weights(ch.hstar, d[0] * d[0] + d[1] * d[1] + d[2] * d[2], om1, om2);
-            double* col = L + (int64_t)(3 * mu) * ld + 3 * nu;
+            if (mu != nu) rpy_weights(hstar, d[0] * d[0] + d[1] * d[1] + d[2] * d[2], om1, om2);
+            double* col = L + (int64_t)(3 * mu) * n + 3 * nu;
             for (int j = 0; j < 3; ++j)
-                for (int i = 0; i < 3; ++i) col[(int64_t)j * ld + i] = om2 * d[i] * d[j] + (i == j ? om1 : 0.0);
+                for (int i = 0; i < 3; ++i) col[(int64_t)j * n + i] = om2 * d[i] * d[j] + (i == j ? om1 : 0.0);
         }
     __syncthreads();
-    if (kBlocked && n >= kBlockedCholMin) {
-        Ctl& ctl = *reinterpret_cast<Ctl*>(stage);
-        constexpr int kCtl = (int)((sizeof(Ctl) + 63) / 64 * 8);
-        if (tid == 0) ctl.brk = 0;
+    constexpr int kPanel = 8, kCols = 4;
+    for (int k0 = 0; k0 < n; k0 += kPanel) {
+        const int kb = min(kPanel, n - k0), k1 = k0 + kb;
+        for (int u = 0; u < kb; ++u)
+            for (int i = k0 + u + tid; i < n; i += TT) P[u * ld + i] = L[(int64_t)(k0 + u) * n + i];
         __syncthreads();
-        Block<BDCU_FORM_PLAIN_FP64> B(a, ctl, ch);
-        B.N = N;
-        B.n = n;
-        B.Lt = L;
-        B.ldl = ld;
-        B.stage = stage + kCtl;
-        B.stage_cap = room - kCtl;
-        int nb = (int)((kLanczosWarm * round_up8(n) - kCtl) / (2 * kCholTileStride)) & ~7;
-        if (!B.cholesky_blocked(nb < kCholMaxBlock ? nb : kCholMaxBlock))
-            return ctl.brk == 2 ? BDCU_ST_TIMEOUT : BDCU_ST_NOT_PD;
-    } else {
-        for (int k = 0; k < n; ++k) {
-            const double s = L[(int64_t)k * ld + k];
-            if (!(s > 0.0)) return BDCU_ST_NOT_PD;
+        for (int u = 0; u < kb; ++u) {
+            const double s = P[u * ld + k0 + u];
+            if (!(s > 0.0)) return false;
             const double dk = sqrt(s);
             __syncthreads();
-            if (tid == 0) L[(int64_t)k * ld + k] = dk;
-            for (int i = k + 1 + tid; i < n; i += TT) L[(int64_t)k * ld + i] = L[(int64_t)k * ld + i] / dk;
+            if (tid == 0) P[u * ld + k0 + u] = dk;
+            for (int i = k0 + u + 1 + tid; i < n; i += TT) P[u * ld + i] = P[u * ld + i] / dk;
             __syncthreads();
-            const double* colk = L + (int64_t)k * ld;
-            for (int j = k + 1 + wi; j < n; j += TT / 32) {
-                const double ljk = colk[j];
-                for (int i = j + wl; i < n; i += 32) L[(int64_t)j * ld + i] -= colk[i] * ljk;
+            for (int v = u + 1; v < kb; ++v) {
+                const double l = P[u * ld + k0 + v];
+                for (int i = k0 + v + tid; i < n; i += TT) P[v * ld + i] -= P[u * ld + i] * l;
             }
             __syncthreads();
         }
+        for (int u = 0; u < kb; ++u)
+            for (int i = k0 + u + tid; i < n; i += TT) L[(int64_t)(k0 + u) * n + i] = P[u * ld + i];
+        for (int j = k1 + kCols * wi; j < n; j += kCols * (TT / 32)) {  // (kb = 8 where there is one)
+            double* col = L + (int64_t)j * n;
+#pragma unroll 1
+            for (int i = j + wl; i < n; i += 32) {
+                double v[kCols];
+#pragma unroll
+                for (int c = 0; c < kCols; ++c) v[c] = i >= j + c ? col[(int64_t)c * n + i] : 0.0;
+#pragma unroll
+                for (int u = 0; u < kPanel; ++u) {
+                    const double f = P[u * ld + i];
+#pragma unroll
+                    for (int c = 0; c < kCols; ++c) v[c] -= f * P[u * ld + min(j + c, n - 1)];
+                }
+#pragma unroll
+                for (int c = 0; c < kCols; ++c)
+                    if (i >= j + c) col[(int64_t)c * n + i] = v[c];
+            }
+        }
+        __syncthreads();
     }
     for (int i = tid; i < n; i += TT) {
         double s = 0.0;
-        for (int j = 0; j <= i; ++j) s += L[(int64_t)j * ld + i] * x[j];
+        for (int j = 0; j <= i; ++j) s += L[(int64_t)j * n + i] * x[j];
         y[i] = s;
     }
     __syncthreads();
-    return 0;
+    return true;
 }
 
 // Doubles of a chain's factor in shared memory: its 3x3 blocks of the lower
@@ -752,7 +764,7 @@ struct PairChain {
             }
             if (cold) {
                 __syncwarp();  // (the lanes of a bead read its basis entries back)
-                if (every || loss.project(j, al, bt, (ww * ib) * ib, 1.0e-15, 1.0e-9, 1.0e-10)) project(j + 1, u);
+                if (every || loss.project(j, al, bt, (ww * ib) * ib, 4.0e-16, 1.0e-8, 1.0e-10)) project(j + 1, u);
             }
         }
     }
@@ -766,7 +778,7 @@ struct PairChain {
             for (int d = 0; d < 3; ++d) ritz[d] = on ? 2.0 * V[3 * b + d] : 0.0;
             return;
         }
-        for (int e = wi; e < 2; e += T) {  // warp 0 the smallest eigenvalue, warp 1 (or 0 too) the largest
+        for (int e = wi; e < 2; ++e) {  // warp 0 the smallest eigenvalue, warp 1 (or the only one) the largest
             double lo = alpha[0], hi2 = alpha[0];
             for (int i = 0; i < k; ++i) {
                 const double rad = (i > 0 ? fabs(beta[i - 1]) : 0.0) + (i < k - 1 ? fabs(beta[i]) : 0.0);
@@ -797,6 +809,7 @@ struct PairChain {
                 if (wl == 0) wk_tridiag_vec(alpha, beta, k, r, y, s3 + 32 * e, s4 + 32 * e);
             }
             if (wl == 0) tot[e] = r;
+            if (T > 1) break;
         }
         __syncthreads();
         rmin = tot[0];
@@ -1105,14 +1118,10 @@ __global__ void __launch_bounds__(32 * T, pair_min_blocks(T, kHi)) integrate_pai
                     if (own)
                         for (int d = 0; d < 3; ++d) x[3 * b + d] = X0[d];
                     __syncthreads();
-                    // (staged in the tables' place, dead by now, and the cached weights')
-                    const int bad = pair_cholesky<(T > 4)>(a, ch, C.Lt, C.ps, C.area,
-                                                                                  lay.total - lay.area, x, y);
-                    if (bad) {
-                        C.status |= bad;
+                    if (!pair_cholesky(C.Lt, C.area, C.ps, N, ch.hstar, x, y)) {
+                        C.status |= BDCU_ST_NOT_PD;
                         break;
                     }
-                    C.build_weights();
 #pragma unroll
                     for (int d = 0; d < 3; ++d) bx[d] = on ? y[3 * b + d] : 0.0;
                 }

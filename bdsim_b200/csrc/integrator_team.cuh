@@ -257,9 +257,8 @@ static __device__ void wk_tridiag_vec(const double* a, const double* b, int m, d
     }
 }
 
-
 // Which vectors of a cold Lanczos run are projected on the whole basis (the reference
-// projects every one, src/hydrodynamics.cpp:171-186): a bound on their loss of
+// projects every one, src/hydrodynamics.cpp:146-264): a bound on their loss of
 // orthogonality, carried along by the recurrence that the loss follows (H. D. Simon,
 // "The Lanczos algorithm with partial reorthogonalization", Math. Comp. 42, 1984),
 //   |v_{j+1}.v_i| <= ((|a_i - a_j| + b_i + b_{i+1}) w_j + b_j w_{j-1} + eps |D|) / b_{j+1}
@@ -269,8 +268,8 @@ static __device__ void wk_tridiag_vec(const double* a, const double* b, int m, d
 // a margin. b_{j+1} comes from |D v_j|^2 by Pythagoras; where that cancels (below
 // `tiny` of it) the vectors are projected in any case. (Two of every six, whatever the
 // spectrum, lost all orthogonality within four steps on chains whose beads lie close
-// together: bounds off by up to 18x in FP64 and 1e4x on FP32 products. Projected in
-// FP64: 25% of the vectors on coils, 37% on collapsed chains.)
+// together: bounds off by up to 18x in FP64 and 1e4x on FP32 products. Projected:
+// 20% of the vectors on coils and 32% on collapsed chains, 39 and 56% on FP32 products.)
 struct BasisLoss {
     double w = 0.0, wp = 0.0, lo = 0.0, hi = 0.0, bmax = 0.0;
     bool again = false;

@@ -94,7 +94,7 @@ __host__ inline int64_t pair_cached(int n_max, int T, int blocks, int sm_count, 
 
 // Per-block global scratch (doubles): cold Lanczos basis, fallback factor.
 __host__ __device__ inline int64_t pair_scratch_doubles(int n_max) {
-    return (int64_t)kLanczosCold * round_up8(n_max) + (int64_t)n_max * chol_ld(n_max);
+    return (int64_t)kLanczosCold * round_up8(n_max) + (int64_t)n_max * n_max;
 }
 
 }  // namespace bdcu

@@ -91,7 +91,7 @@ class BasisLoss:
 
 def kernel_run(D, v, m, cold, mixed=False):
     n, V, al, be, u, vp = len(v), [], [], [], v, 0.0 * v
-    loss = BasisLoss(1e-7, 3e-4, 1e-5) if mixed else BasisLoss(1e-15, 1e-9, 1e-10)
+    loss = BasisLoss(1e-7, 3e-4, 1e-5) if mixed else BasisLoss(4e-16, 1e-8, 1e-10)
     m = min(n, m)
     for j in range(m):
         w = product(D, u, mixed)
