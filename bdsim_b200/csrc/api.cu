@@ -287,16 +287,14 @@ std::vector<Shape> block_shapes(const bdcu_ctx* ctx, const Bucket& b, int form) 
     std::vector<Shape> out;
     for (int blk : blocks)
         for (int v : v_opts) {
-            if ((size_t)smem_layout(b.n_max, 0, v, mixed).total * sizeof(double) > ctx->max_smem) continue;
+            if ((size_t)smem_layout(b.n_max, v, mixed).total * sizeof(double) > ctx->max_smem) continue;
             Shape s;
             s.block = blk;
             s.v_cap = v;
-            s.d_in_smem = 0;
             out.push_back(s);
         }
     return out;
 }
-
 
 // Fill the launch fields of a bucket for a shape (block or pair kernel) or for
 // the team kernel; 0 when the shape cannot run.
@@ -321,14 +319,13 @@ int fill_launch(bdcu_ctx* ctx, int form, Bucket& b, const Shape* s) {
         b.block = 32 * T * tpc;
         b.grid = std::max(1, std::min((b.count + tpc - 1) / tpc, per_sm * ctx->sm_count));
         b.v_cap = 0;
-        b.d_in_smem = 0;
         b.scratch_stride = b.need_d ? team_scratch_doubles(b.n_max) : 1;
         return BDCU_OK;
     }
     if (b.kernel == kKernelPair) {
         const int T = pair_warps(b.id, b.n_max, b.count, ctx->sm_count);
         b.block = 32 * T;
-        b.v_cap = b.d_in_smem = 0;
+        b.v_cap = 0;
         b.pair_hi = pair_hi(T, b.need_d, b.count, ctx->sm_count);
         b.w_pairs = pair_shared(b.id, T, b.n_max, b.need_lz, b.count, ctx->sm_count, ctx->max_smem);
         b.smem = (size_t)pair_layout(b.n_max, T, b.w_pairs).total * sizeof(double);
@@ -347,14 +344,13 @@ int fill_launch(bdcu_ctx* ctx, int form, Bucket& b, const Shape* s) {
     }
     b.block = s->block;
     b.v_cap = s->v_cap;
-    b.d_in_smem = s->d_in_smem;
-    b.smem = (size_t)smem_layout(b.n_max, b.d_in_smem, b.v_cap, mixed).total * sizeof(double);
+    b.smem = (size_t)smem_layout(b.n_max, b.v_cap, mixed).total * sizeof(double);
     if (b.smem > ctx->max_smem) return fail(ctx, BDCU_E_LIMIT, "chain too large for the shared-memory layout");
     e = mixed ? occupancy_mixed(b.block, b.smem, &per_sm) : occupancy_plain(b.block, b.smem, &per_sm);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
     if (per_sm < 1) return fail(ctx, BDCU_E_LIMIT, "block kernel shape cannot be resident");
     b.grid = std::max(1, std::min(b.count, per_sm * ctx->sm_count));
-    const ScratchLayout scl = scratch_layout(b.n_max, 0, b.v_cap, b.need_chol, mixed, 0, b.need_lz);
+    const ScratchLayout scl = scratch_layout(b.n_max, b.v_cap, b.need_chol, b.need_lz);
     b.scratch_stride = std::max<int64_t>(scl.total, 1);
     return BDCU_OK;
 }
@@ -447,8 +443,7 @@ int build_plan(bdcu_ctx* ctx, int form) {
             if (t.block > 0) {
                 // the tuned shape, or the nearest one that still fits this bucket
                 for (const Shape& s : shapes)
-                    if (s.block == std::min(t.block, shapes.front().block) && s.v_cap == t.v_cap &&
-                        s.d_in_smem == t.d_in_smem) {
+                    if (s.block == std::min(t.block, shapes.front().block) && s.v_cap == t.v_cap) {
                         pick = s;
                         b.tuned = 1;
                         break;
@@ -513,10 +508,8 @@ int launch_bucket(bdcu_ctx* ctx, int form, const Bucket& b, const State& st, int
     a.status = st.status;
     a.counters = st.counters;
     a.cache_mode = cache_mode;
-    a.d_in_smem = b.d_in_smem;
     a.v_cap = b.v_cap;
     a.need_chol = b.need_chol;
-    a.need_d = 0;  // (no dense D)
     a.need_lz = b.need_lz;
     a.work_counter = ctx->work_d + b.id;
     a.order = ctx->order_d + b.order_off;
@@ -784,7 +777,7 @@ int bdcu_describe_plan(bdcu_ctx* ctx, int form, bdcu_bucket_info* out, int cap, 
         o.block = b.block;
         o.grid = b.grid;
         o.v_cap = b.v_cap;
-        o.d_in_smem = b.d_in_smem;
+        o.d_in_smem = 0;
         o.tuned = b.tuned;
         o.smem_bytes = (int64_t)b.smem;
     }

@@ -64,10 +64,8 @@ struct RunArgs {
     int32_t* status;
     bdcu_counters* counters;
     int32_t cache_mode;
-    int32_t d_in_smem;      // shared memory holds room for a dense D (static-scratch layout only, unused)
     int32_t v_cap;          // Lanczos basis vectors that fit in shared memory
     int32_t need_chol;      // some chain may factor D (Cholesky or fallback)
-    int32_t need_d;         // scratch holds room for a dense D (static-scratch layout only, unused)
     int32_t need_lz;        // some chain uses the Chebyshev method (Lanczos)
     int32_t* work_counter;  // persistent-grid chain queue (zeroed before launch)
     const int32_t* order;   // the launch's work list: chain indices, largest first (null: 0..n_work-1)

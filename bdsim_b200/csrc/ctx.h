@@ -38,7 +38,6 @@ constexpr int kBucketOrder[kMaxBuckets] = {7, 6, 5, 4, 3, 2, 1, 8, 0};
 struct Shape {
     int block = 0;  // 0: not tuned
     int v_cap = -1;
-    int d_in_smem = -1;
     int team_warps = 0;
     int team_q = 0;
 };
@@ -52,7 +51,7 @@ struct Bucket {
     int n_max = 0;  // 3 * max_beads
     int need_chol = 0, need_d = 0, need_lz = 0;
     int64_t order_off = 0;  // first entry of this bucket's work list in order_d
-    int block = 0, grid = 0, v_cap = 0, d_in_smem = 0, tuned = 0;
+    int block = 0, grid = 0, v_cap = 0, tuned = 0;
     bool pair_hi = true;  // pair kernel: the build with HI
     int64_t w_pairs = 0;  // pair and team kernels: cached pair weights (per block, per team)
     size_t smem = 0;

@@ -6,8 +6,8 @@
 //   evaluated pair by pair from the positions, EV forces are accumulated per
 //   bead in the reference's pair order, Cholesky is right-looking (blocked from
 //   3N = 300, trailing updates on the FP64 tensor cores). It runs the chains the
-//   pair kernel does not take: the Cholesky method above N = 64, any chain above
-//   N = 512, and every chain of the static-scratch entry point.
+//   pair kernel does not take: the Cholesky method above N = 64 and any chain above
+//   N = 512.
 // FORM == BDCU_FORM_MIXED_FP32: D.x recomputed pairwise in FP32 from
 //   shared-memory bead coordinates (no stored D), FP32 excluded volume; FP64
 //   positions, connector solve, Lanczos bounds and Cholesky.
@@ -48,14 +48,14 @@ struct Ctl {
 enum { C_STEPS = 0, C_DX, C_CHEB, C_CORR, C_LZCOLD, C_LZWARM, C_FALLBACK, C_NONCONV };
 
 struct SmemLayout {
-    int64_t ctl, chain, red, alpha, beta, ymin, ymax, coef, sqx, slots, V, D, f32, total;  // in doubles
+    int64_t ctl, chain, red, alpha, beta, ymin, ymax, coef, sqx, slots, V, f32, total;  // in doubles
 };
 
 __host__ __device__ inline int64_t round_up8(int64_t x) { return (x + 7) / 8 * 8; }
 
 // Shared-memory layout (in doubles) for a launch whose largest chain has
 // 3N = n_max. Host and device compute it with the same function.
-__host__ __device__ inline SmemLayout smem_layout(int n_max, int d_in_smem, int v_cap, int mixed) {
+__host__ __device__ inline SmemLayout smem_layout(int n_max, int v_cap, int mixed) {
     SmemLayout s;
     int64_t o = 0;
     s.ctl = o;   o += round_up8((int64_t)(sizeof(Ctl) + 7) / 8);
@@ -70,7 +70,6 @@ __host__ __device__ inline SmemLayout smem_layout(int n_max, int d_in_smem, int 
     const int64_t nv = round_up8(n_max);
     s.slots = o; o += (int64_t)kSlots * nv;
     s.V = o;     o += (int64_t)v_cap * nv;
-    s.D = o;     if (d_in_smem) o += (int64_t)n_max * n_max;
     s.f32 = o;   if (mixed) o += 2 * nv;  // float4 bead coordinates + float4 staged vector (N <= n/3 each)
     s.total = o;
     return s;
@@ -83,19 +82,15 @@ __host__ __device__ inline SmemLayout smem_layout(int n_max, int d_in_smem, int 
 __host__ __device__ inline int chol_ld(int n) { return (n + 15) / 16 * 16; }
 
 // Global scratch per thread block (doubles): the Cholesky factor and the cold
-// Lanczos basis. The room for a dense D is kept where need_d asks for it: the
-// static-scratch entry point states its limit with it.
+// Lanczos basis.
 struct ScratchLayout {
-    int64_t D, Lt, V, total;
+    int64_t Lt, V, total;
 };
-__host__ __device__ inline ScratchLayout scratch_layout(int n_max, int d_in_smem, int v_cap, int need_chol,
-                                                        int mixed, int need_d, int need_lz) {
+__host__ __device__ inline ScratchLayout scratch_layout(int n_max, int v_cap, int need_chol, int need_lz) {
     // every region a whole number of 128-byte lines (16 doubles), so that a
-    // block's D and factor start on a line of their own (discard.global.L2)
+    // block's factor starts on a line of its own (discard.global.L2)
     ScratchLayout s;
     int64_t o = 0;
-    const int64_t nn = (int64_t)n_max * n_max, nn16 = (nn + 15) / 16 * 16;
-    s.D = o;  if (!mixed && need_d && !d_in_smem) o += nn16;
     s.Lt = o; if (need_chol) o += (int64_t)n_max * chol_ld(n_max);
     s.V = o;  if (need_lz && v_cap < kLanczosCold) o += ((int64_t)kLanczosCold * round_up8(n_max) + 15) / 16 * 16;
     s.total = o;
@@ -129,9 +124,8 @@ static __device__ double block_dot(const double* a, const double* b, int n, doub
     return red[0] + red[1];
 }
 
-// Drop the L2 lines of [p, p + doubles) without writing them back: the dense
-// D (and a factor) are rebuilt every step, so after a step's last read the
-// data is dead. p must start a 128-byte line and the range must end at the
+// Drop the L2 lines of [p, p + doubles) without writing them back: a factor is
+// rebuilt every step, so after a step's last read the data is dead. p must start a 128-byte line and the range must end at the
 // end of its allocation's last line (scratch_layout rounds every region to
 // whole lines); a misaligned p is left alone.
 __device__ __forceinline__ void discard_l2(const double* p, int64_t doubles) {
@@ -1305,8 +1299,8 @@ template <int FORM>
 __global__ void __launch_bounds__(512, 1) integrate_kernel(const RunArgs a) {
     extern __shared__ __align__(16) double sm[];
     constexpr bool kMixed = (FORM == BDCU_FORM_MIXED_FP32);
-    const SmemLayout lay = smem_layout(a.n_max, a.d_in_smem, a.v_cap, kMixed);
-    const ScratchLayout scl = scratch_layout(a.n_max, a.d_in_smem, a.v_cap, a.need_chol, kMixed, a.need_d, a.need_lz);
+    const SmemLayout lay = smem_layout(a.n_max, a.v_cap, kMixed);
+    const ScratchLayout scl = scratch_layout(a.n_max, a.v_cap, a.need_chol, a.need_lz);
     Ctl& ctl = *reinterpret_cast<Ctl*>(sm + lay.ctl);
     DevChain& ch = *reinterpret_cast<DevChain*>(sm + lay.chain);
     double* scr = a.scratch + (int64_t)blockIdx.x * a.scratch_stride;

@@ -145,7 +145,7 @@ extern "C" int bdcu_run_static(bdcu_ctx* ctx, int n_chains, const bdcu_phys* phy
     // buckets, as bdcu_run plans them (largest chains first within a bucket)
     const int mixed = (form == BDCU_FORM_MIXED_FP32);
     struct Launch {
-        int id, kernel, pair_hi, team_warps, team_q, block, grid, v_cap, d_in_smem, n_max, need_d, need_lz, count;
+        int id, kernel, pair_hi, team_warps, team_q, block, grid, v_cap, n_max, need_d, need_lz, count;
         size_t smem, per_block;
         int64_t stride, order_off, w_pairs;
     };
@@ -202,24 +202,18 @@ extern "C" int bdcu_run_static(bdcu_ctx* ctx, int n_chains, const bdcu_phys* phy
                 l.per_block = sizeof(double) * (size_t)l.stride;
                 l.grid = l.count;
             } else {
-                std::vector<int> d_opts = (!mixed && l.need_d) ? std::vector<int>{1, 0} : std::vector<int>{0};
-                std::vector<int> v_opts = l.need_lz ? std::vector<int>{kLanczosCold, kLanczosWarm, 0} : std::vector<int>{0};
-                l.d_in_smem = -1;
-                for (int d : d_opts) {
-                    for (int v : v_opts) {
-                        const size_t bytes = (size_t)smem_layout(l.n_max, d, v, mixed).total * sizeof(double);
-                        if (bytes <= ctx->max_smem) {
-                            l.d_in_smem = d;
-                            l.v_cap = v;
-                            l.smem = bytes;
-                            break;
-                        }
-                    }
-                    if (l.d_in_smem >= 0) break;
+                const std::vector<int> v_opts =
+                    l.need_lz ? std::vector<int>{kLanczosCold, kLanczosWarm, 0} : std::vector<int>{0};
+                l.v_cap = -1;
+                for (int v : v_opts) {
+                    l.smem = (size_t)smem_layout(l.n_max, v, mixed).total * sizeof(double);
+                    if (l.smem > ctx->max_smem) continue;
+                    l.v_cap = v;
+                    break;
                 }
-                if (l.d_in_smem < 0) return fail(ctx, BDCU_E_LIMIT, "bdcu_run_static: chain too large for the shared-memory layout");
+                if (l.v_cap < 0) return fail(ctx, BDCU_E_LIMIT, "bdcu_run_static: chain too large for the shared-memory layout");
                 l.block = widest_block(l.n_max);
-                const ScratchLayout scl = scratch_layout(l.n_max, l.d_in_smem, l.v_cap, l.need_d, mixed, l.need_d, l.need_lz);
+                const ScratchLayout scl = scratch_layout(l.n_max, l.v_cap, l.need_d, l.need_lz);
                 l.stride = std::max<int64_t>(scl.total, 1);
                 l.per_block = sizeof(double) * (size_t)l.stride;
                 e = mixed ? occupancy_mixed(l.block, l.smem, &per_sm) : occupancy_plain(l.block, l.smem, &per_sm);
@@ -320,10 +314,8 @@ extern "C" int bdcu_run_static(bdcu_ctx* ctx, int n_chains, const bdcu_phys* phy
         a.status = status;
         a.counters = counters;
         a.cache_mode = cache_mode;
-        a.d_in_smem = l.d_in_smem;
         a.v_cap = l.v_cap;
         a.need_chol = l.need_d;
-        a.need_d = l.need_d;
         a.need_lz = l.need_lz;
         a.w_pairs = l.w_pairs;
         a.work_counter = reinterpret_cast<int32_t*>(b + o_cnt) + l.id;

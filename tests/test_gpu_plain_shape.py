@@ -230,3 +230,36 @@ def test_mixed_fallback_costs_no_more_than_twice_the_cholesky_method():
 
     factor = ms(DelSMethod.Chebyshev, -1.0) - ms(DelSMethod.Chebyshev, 1.0)
     assert factor <= 2.0 * ms(DelSMethod.Cholesky, 1.0)
+
+
+@pytest.mark.parametrize("N,method", [(400, DelSMethod.Cholesky), (430, DelSMethod.Chebyshev)])
+def test_static_entry_point_asks_for_what_its_kernels_take(N, method):
+    """One block's factor (11.6 MB, 13.3 MB) fits the 16 MiB array; a dense tensor
+    beside it, which no kernel forms, did not."""
+    p, s = workloads.batched_cheb_phys(N)
+    p.hi_method = method
+    R0 = [B.gaussian_chain(N, bond_std=1.0, seed=1)]
+    ens = B.Ensemble([p], [s], R0, [(1, -1, 5)], form="plain")
+    ens.advance(0.0, 1, _abi.CACHE_RESET_PER_CALL)
+    rc, got = run_static([p], [s], R0, [(1, -1, 5)], 1, "plain")
+    assert rc == 0 and np.array_equal(got, ens.R.cpu().numpy())
+
+
+def test_static_entry_point_at_its_limit():
+    """A plain batch whose parameters leave room for the general kernel's scratch but
+    not for the pair kernel's still runs, to rounding."""
+    p, s = workloads.batched_cheb_phys(100)
+    R0 = [B.gaussian_chain(100, bond_std=1.0, seed=1)]
+    ens = B.Ensemble([p], [s], R0, [(1, -1, 5)], form="plain")
+    ens.advance(0.0, 1, _abi.CACHE_RESET_PER_CALL)
+    want = ens.R.cpu().numpy()
+    ran = {}
+    for kb in (0, 15600, 15630, 15700, 16300):
+        rc, got = run_static([p], [s], R0, [(1, -1, 5)], 1, "plain", pad=128 * kb)
+        ran[kb] = (rc, np.array_equal(got, want))
+        if rc == 0:
+            assert np.max(np.abs(got - want)) <= 1e-10 * max(1.0, np.max(np.abs(want)))
+        else:
+            assert rc == 5  # BDCU_E_LIMIT
+    assert ran[0] == (0, True) and ran[16300][0] == 5
+    assert any(rc == 0 and not same for rc, same in ran.values())
