@@ -764,7 +764,7 @@ struct PairChain {
             }
             if (cold) {
                 __syncwarp();  // (the lanes of a bead read its basis entries back)
-                if (every || loss.project(j, al, bt, (ww * ib) * ib, 4.0e-16, 1.0e-8, 1.0e-10)) project(j + 1, u);
+                if (every || loss.project(j, al, bt, (ww * ib) * ib, 4.0e-16f, 1.0e-8f, 1.0e-10f)) project(j + 1, u);
             }
         }
     }

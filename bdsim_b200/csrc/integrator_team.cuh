@@ -270,23 +270,24 @@ static __device__ void wk_tridiag_vec(const double* a, const double* b, int m, d
 // spectrum, lost all orthogonality within four steps on chains whose beads lie close
 // together: bounds off by up to 18x in FP64 and 1e4x on FP32 products. Projected:
 // 20% of the vectors on coils and 32% on collapsed chains, 39 and 56% on FP32 products.)
+// FP32 but for the cancelling difference: the bound's latency is on every step's path.
 struct BasisLoss {
-    double w = 0.0, wp = 0.0, lo = 0.0, hi = 0.0, bmax = 0.0;
+    float w = 0.f, wp = 0.f, lo = 0.f, hi = 0.f, bmax = 0.f;
     bool again = false;
     // After step j's alpha, beta (none at j = 0) and ww = |D v_j|^2: project the next vector?
-    __device__ __forceinline__ bool project(int j, double al, double bt, double ww, double eps, double tol, double tiny) {
+    __device__ __forceinline__ bool project(int j, double al, double bt, double ww, float eps, float tol, float tiny) {
         if (j == 0) {
-            lo = hi = al;
+            lo = hi = (float)al;
             bt = 0.0;
         }
-        lo = fmin(lo, al);
-        hi = fmax(hi, al);
-        bmax = fmax(bmax, bt);
-        const double bsq = ww - al * al - bt * bt;
-        const bool lost = !(bsq > tiny * ww);
-        const double ib = lost ? 1.0 : rsqrt_refined(bsq), bn = lost ? 1.0 : bsq * ib;
-        const double f = fmax(hi - al, al - lo) + 2.0 * fmax(bmax, bn);
-        double wn = (f * w + bt * wp + eps * (fabs(al) + bt + bn)) * ib;
+        const float a = (float)al, b = (float)bt, sq = (float)fma(-bt, bt, fma(-al, al, ww));
+        lo = fminf(lo, a);
+        hi = fmaxf(hi, a);
+        bmax = fmaxf(bmax, b);
+        const bool lost = !(sq > tiny * (float)ww);
+        const float ib = lost ? 1.f : rsqrtf(sq), bn = lost ? 1.f : sq * ib;
+        const float f = fmaxf(hi - a, a - lo) + 2.f * fmaxf(bmax, bn);
+        float wn = (f * w + b * wp + eps * (fabsf(a) + b + bn)) * ib;
         const bool hit = lost || !(wn <= tol), now = hit || again;
         again = lost || (hit && !again);
         if (now) wn = eps;
@@ -1049,7 +1050,7 @@ struct TeamChain {
                     if (j > 0) u[q][d] -= bt * vp[q][d];
                     vp[q][d] = v[q][d];
                 }
-            if (cold && (every || loss.project(j, al, bt, (ww * ib) * ib, 1.0e-7, 3.0e-4, 1.0e-5))) project(j + 1, u);
+            if (cold && (every || loss.project(j, al, bt, (ww * ib) * ib, 1.0e-7f, 3.0e-4f, 1.0e-5f))) project(j + 1, u);
         }
         sync();
         if (k == 1) {

@@ -66,22 +66,25 @@ def reference_run(D, v, m, mixed=False):
     return np.array(V), np.array(al), np.array(be[:len(al) - 1])
 
 
+F = np.float32
+
+
 class BasisLoss:
     def __init__(self, eps, tol, tiny):
-        self.eps, self.tol, self.tiny = eps, tol, tiny
-        self.w = self.wp = self.bmax = 0.0
+        self.eps, self.tol, self.tiny = F(eps), F(tol), F(tiny)
+        self.w = self.wp = self.bmax = F(0)
         self.again = False
 
     def project(self, j, al, bt, ww):
         if j == 0:
-            self.lo = self.hi = al
+            self.lo = self.hi = F(al)
             bt = 0.0
-        self.lo, self.hi, self.bmax = min(self.lo, al), max(self.hi, al), max(self.bmax, bt)
-        bsq = ww - al * al - bt * bt
-        lost = not bsq > self.tiny * ww
-        bn = 1.0 if lost else np.sqrt(bsq)
-        f = max(self.hi - al, al - self.lo) + 2.0 * max(self.bmax, bn)
-        wn = (f * self.w + bt * self.wp + self.eps * (abs(al) + bt + bn)) / bn
+        a, b, sq = F(al), F(bt), F(ww - al * al - bt * bt)
+        self.lo, self.hi, self.bmax = min(self.lo, a), max(self.hi, a), max(self.bmax, b)
+        lost = not sq > self.tiny * F(ww)
+        bn = F(1) if lost else np.sqrt(sq)
+        f = max(self.hi - a, a - self.lo) + F(2) * max(self.bmax, bn)
+        wn = (f * self.w + b * self.wp + self.eps * (abs(a) + b + bn)) / bn
         hit = lost or not wn <= self.tol
         now = hit or self.again
         self.again = lost or (hit and not self.again)
