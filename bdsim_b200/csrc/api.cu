@@ -1071,7 +1071,6 @@ int bdcu_integrate_host(bdcu_ctx* ctx, double* R_host, int32_t* rng_host, int32_
     const bool packed = o_valid <= kPinned;
     if (packed && !ctx->hpin) {
         CK(cudaHostAlloc(reinterpret_cast<void**>(&ctx->hpin), kPinned, cudaHostAllocDefault));
-        ctx->hpin_bytes = kPinned;
     }
     std::vector<double> t0(nc);
     std::vector<int32_t> steps(nc);

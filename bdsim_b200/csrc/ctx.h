@@ -126,5 +126,4 @@ struct bdcu_ctx {
     unsigned char* hblk = nullptr;
     size_t hblk_bytes = 0;
     unsigned char* hpin = nullptr;
-    size_t hpin_bytes = 0;
 };

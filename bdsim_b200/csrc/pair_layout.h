@@ -24,8 +24,11 @@ __host__ __device__ constexpr int pair_min_blocks(int T, bool hi) {
 }
 
 // Warps per chain of buckets 0..3 (N <= 64, 128, 256, 512; fewer in launches of the
-// shortest chains), and of the Cholesky method's.
-constexpr int kPairWarps[4] = {4, 8, 8, 16};
+// shortest chains), and of the Cholesky method's. One shape must serve any number of
+// chains (6 steps; 100 and 3000 chains): N = 130 on 8 warps 4.51 and 49.2 ms, on 16 3.31
+// and 43.9; N = 256 13.2 and 123, 9.2 and 121; N = 128 on 8 2.88 and 29.1, on 16 2.58 and
+// 33.2, on 4 4.07 and 32.7; N = 64 on 4 0.81 and 7.5, on 8 0.94 and 8.5.
+constexpr int kPairWarps[4] = {4, 8, 16, 16};
 constexpr int kPairCholWarps = 4;
 
 struct PairLayout {
