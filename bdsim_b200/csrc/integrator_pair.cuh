@@ -50,24 +50,23 @@ __device__ __forceinline__ void warp_multisect(const Count& count, int target, d
 // with 16-byte loads at fixed offsets from one pointer.
 __device__ __forceinline__ int pair_at(int j, int d) { return 6 * (j >> 1) + 2 * d + (j & 1); }
 
-// Cholesky fallback (src/mobility.cpp:69-81): the lower part of the dense D in
-// global scratch from the staged positions ps (element (i, k) at L[k n + i]), its
-// right-looking factor, y = L x (3N vectors in shared memory). Eight columns at a
-// time are factored in shared memory (P, 8 round_up8(n) doubles: the area of the
-// Chebyshev tables, dead by now); then a warp takes four columns of the trailing
-// triangle at once, so that an element crosses L2 once per eight columns and a lane's
-// four loads are in flight together. Every element still receives its products one by
-// one, in k order. (One column at a time, each streamed the triangle through L2: 148
-// chains of N = 300 and 500, one step that falls back after 500 products, 170 and 712
-// ms; so 37 and 102. The block kernel's tile updates on the tensor cores in this
-// place: 32 and 70, but their registers made the kernel spill in the steps that do not
-// fall back, 3 to 10% of large chains' time.) False if not positive definite. Out of
-// line, with plain arguments: the chain's state stays in registers around the call.
-static __device__ __noinline__ bool pair_cholesky(double* L, double* P, const double* ps, int N, double hstar,
-                                                  const double* x, double* y) {
-    const int tid = threadIdx.x, TT = blockDim.x, wl = tid & 31, wi = tid >> 5, n = 3 * N, ld = (n + 7) & ~7;
-    for (int mu = wi; mu < N; mu += TT / 32)
-        for (int nu = mu + wl; nu < N; nu += 32) {
+// Cholesky fallback (src/mobility.cpp:69-81), in four parts: the lower part of the
+// dense D in global scratch from the staged positions ps (element (i, k) at L[k n +
+// i]); its right-looking factor, eight columns at a time factored in shared memory
+// (P, 8 round_up8(n) doubles: the area of the Chebyshev tables, dead by now) and
+// taken off the trailing triangle, four of its columns per warp at once, so that an
+// element crosses L2 once per eight columns and a lane's four loads are in flight
+// together; y = L x (3N vectors in shared memory). Every element receives its
+// products one by one, in k order. 148 chains of N = 50, 300 and 500, one step that
+// falls back after 500 products: one column at a time 2.7, 170 and 712 ms, so 1.2, 39
+// and 108. (The block kernel's tile updates on the tensor cores in this place: 32 and
+// 70 ms for the long ones.) Each part out of line, with plain arguments and few
+// registers: as one function, or with the tensor cores, it made the kernel spill in
+// the steps that do not fall back (3 to 10% of long chains' time).
+static __device__ __noinline__ void pair_dense(double* L, const double* ps, int N, double hstar) {
+    const int n = 3 * N;
+    for (int mu = threadIdx.x >> 5; mu < N; mu += blockDim.x >> 5)
+        for (int nu = mu + (threadIdx.x & 31); nu < N; nu += 32) {
             double d[3], om1 = 1.0, om2 = 0.0;
             for (int k = 0; k < 3; ++k) d[k] = ps[pair_at(nu, k)] - ps[pair_at(mu, k)];
             if (mu != nu) rpy_weights(hstar, d[0] * d[0] + d[1] * d[1] + d[2] * d[2], om1, om2);
@@ -76,55 +75,64 @@ static __device__ __noinline__ bool pair_cholesky(double* L, double* P, const do
                 for (int i = 0; i < 3; ++i) col[(int64_t)j * n + i] = om2 * d[i] * d[j] + (i == j ? om1 : 0.0);
         }
     __syncthreads();
-    constexpr int kPanel = 8, kCols = 4;
-    for (int k0 = 0; k0 < n; k0 += kPanel) {
-        const int kb = min(kPanel, n - k0), k1 = k0 + kb;
-        for (int u = 0; u < kb; ++u)
-            for (int i = k0 + u + tid; i < n; i += TT) P[u * ld + i] = L[(int64_t)(k0 + u) * n + i];
+}
+constexpr int kPairPanel = 8;
+// Columns k0 .. k0 + 7 (fewer at the end) into P, factored, and back. False if not
+// positive definite.
+static __device__ __noinline__ bool pair_panel(double* L, double* P, int n, int k0) {
+    const int tid = threadIdx.x, TT = blockDim.x, ld = (n + 7) & ~7, kb = min(kPairPanel, n - k0);
+    for (int u = 0; u < kb; ++u)
+        for (int i = k0 + u + tid; i < n; i += TT) P[u * ld + i] = L[(int64_t)(k0 + u) * n + i];
+    __syncthreads();
+    for (int u = 0; u < kb; ++u) {
+        const double s = P[u * ld + k0 + u];
+        if (!(s > 0.0)) return false;
+        const double dk = sqrt(s);
         __syncthreads();
-        for (int u = 0; u < kb; ++u) {
-            const double s = P[u * ld + k0 + u];
-            if (!(s > 0.0)) return false;
-            const double dk = sqrt(s);
-            __syncthreads();
-            if (tid == 0) P[u * ld + k0 + u] = dk;
-            for (int i = k0 + u + 1 + tid; i < n; i += TT) P[u * ld + i] = P[u * ld + i] / dk;
-            __syncthreads();
-            for (int v = u + 1; v < kb; ++v) {
-                const double l = P[u * ld + k0 + v];
-                for (int i = k0 + v + tid; i < n; i += TT) P[v * ld + i] -= P[u * ld + i] * l;
-            }
-            __syncthreads();
-        }
-        for (int u = 0; u < kb; ++u)
-            for (int i = k0 + u + tid; i < n; i += TT) L[(int64_t)(k0 + u) * n + i] = P[u * ld + i];
-        for (int j = k1 + kCols * wi; j < n; j += kCols * (TT / 32)) {  // (kb = 8 where there is one)
-            double* col = L + (int64_t)j * n;
-#pragma unroll 1
-            for (int i = j + wl; i < n; i += 32) {
-                double v[kCols];
-#pragma unroll
-                for (int c = 0; c < kCols; ++c) v[c] = i >= j + c ? col[(int64_t)c * n + i] : 0.0;
-#pragma unroll
-                for (int u = 0; u < kPanel; ++u) {
-                    const double f = P[u * ld + i];
-#pragma unroll
-                    for (int c = 0; c < kCols; ++c) v[c] -= f * P[u * ld + min(j + c, n - 1)];
-                }
-#pragma unroll
-                for (int c = 0; c < kCols; ++c)
-                    if (i >= j + c) col[(int64_t)c * n + i] = v[c];
-            }
+        if (tid == 0) P[u * ld + k0 + u] = dk;
+        for (int i = k0 + u + 1 + tid; i < n; i += TT) P[u * ld + i] = P[u * ld + i] / dk;
+        __syncthreads();
+        for (int v = u + 1; v < kb; ++v) {
+            const double l = P[u * ld + k0 + v];
+            for (int i = k0 + v + tid; i < n; i += TT) P[v * ld + i] -= P[u * ld + i] * l;
         }
         __syncthreads();
     }
-    for (int i = tid; i < n; i += TT) {
+    for (int u = 0; u < kb; ++u)
+        for (int i = k0 + u + tid; i < n; i += TT) L[(int64_t)(k0 + u) * n + i] = P[u * ld + i];
+    return true;
+}
+// The panel P of the eight columns before k1 off the columns from k1 on.
+static __device__ __noinline__ void pair_trailing(double* L, const double* P, int n, int k1) {
+    constexpr int kCols = 4;
+    const int ld = (n + 7) & ~7;
+    for (int j = k1 + kCols * (threadIdx.x >> 5); j < n; j += kCols * (blockDim.x >> 5)) {
+        double* col = L + (int64_t)j * n;
+#pragma unroll 1
+        for (int i = j + (threadIdx.x & 31); i < n; i += 32) {
+            double v[kCols];
+#pragma unroll
+            for (int c = 0; c < kCols; ++c) v[c] = i >= j + c ? col[(int64_t)c * n + i] : 0.0;
+#pragma unroll 1
+            for (int u = 0; u < kPairPanel; ++u) {
+                const double f = P[u * ld + i];
+#pragma unroll
+                for (int c = 0; c < kCols; ++c) v[c] -= f * P[u * ld + min(j + c, n - 1)];
+            }
+#pragma unroll
+            for (int c = 0; c < kCols; ++c)
+                if (i >= j + c) col[(int64_t)c * n + i] = v[c];
+        }
+    }
+    __syncthreads();
+}
+static __device__ __noinline__ void pair_lower(const double* L, int n, const double* x, double* y) {
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
         double s = 0.0;
         for (int j = 0; j <= i; ++j) s += L[(int64_t)j * n + i] * x[j];
         y[i] = s;
     }
     __syncthreads();
-    return true;
 }
 
 // Doubles of a chain's factor in shared memory: its 3x3 blocks of the lower
@@ -1118,10 +1126,18 @@ __global__ void __launch_bounds__(32 * T, pair_min_blocks(T, kHi)) integrate_pai
                     if (own)
                         for (int d = 0; d < 3; ++d) x[3 * b + d] = X0[d];
                     __syncthreads();
-                    if (!pair_cholesky(C.Lt, C.area, C.ps, N, ch.hstar, x, y)) {
+                    bool pd = true;
+                    pair_dense(C.Lt, C.ps, N, ch.hstar);
+#pragma unroll 1
+                    for (int k0 = 0; pd && k0 < n; k0 += kPairPanel) {
+                        pd = pair_panel(C.Lt, C.area, n, k0);
+                        if (pd) pair_trailing(C.Lt, C.area, n, k0 + kPairPanel);
+                    }
+                    if (!pd) {
                         C.status |= BDCU_ST_NOT_PD;
                         break;
                     }
+                    pair_lower(C.Lt, n, x, y);
 #pragma unroll
                     for (int d = 0; d < 3; ++d) bx[d] = on ? y[3 * b + d] : 0.0;
                 }
