@@ -429,7 +429,8 @@ __device__ __forceinline__ void rpy_weights(double hstar, double sq, double& om1
 
 // 1/sqrt(s) for s in [1e-30, 3e38]: the single-precision estimate y (relative
 // error below 2^-21) refined by one third-order step of the Newton-Halley
-// family, y (1 + e/2 + 3 e^2/8) with e = 1 - s y^2, whose error is O(e^3).
+// family, y (1 + e/2 + 3 e^2/8) with e = 1 - s y^2, whose error is O(e^3). Within 2^-52
+// relative: half of e's own rounding (2^-53) and the last one (2^-53).
 __device__ __forceinline__ double rsqrt_refined(double s) {
     const double y = (double)rsqrtf((float)s);
     const double e = fma(-(s * y), y, 1.0);

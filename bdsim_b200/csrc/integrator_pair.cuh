@@ -725,8 +725,8 @@ struct PairChain {
     // 1e-12 relative (3e-10 for the smallest one of chains whose beads nearly
     // coincide). A cold run projects where BasisLoss says so (from 3N = 64; in
     // every step below, where the Krylov space is soon exhausted), which keeps the
-    // basis orthogonal to 1e-9, far below the square root of rounding that the
-    // tridiagonal's accuracy needs. (Projecting in every step read the basis from
+    // basis orthogonal to 1e-8, the square root of rounding that the tridiagonal's
+    // accuracy needs (3e-10 at most on rods, rings, coils and collapsed chains). (Projecting in every step read the basis from
     // L2 twice a step: 12.9 thousand cycles a step at N = 50, 2.7 of them the
     // product.) Returns its steps; the tridiagonal is left in alpha and beta.
     __device__ __forceinline__ int lanczos(double* V, bool cold, double (&v)[3], double (&w)[3], bool have_w) {
